@@ -243,7 +243,7 @@ void ipuma_gpu_destroy(ipuma_engine* e);
  *                 SMs proportional to its modelled work; 0 = one launch
  *                 after the other (always the case with time_launches)
  *   "latency_share" share of the batch's modelled time (per mille,
- *                 default 60) one pair's item may take in its class; a
+ *                 default 250) one pair's item may take in its class; a
  *                 pair over it takes a class that finishes it sooner
  *   "hybrid"      1 = pairs whose score can pass int16 run their strips
  *                 in biased 16-bit halves while a strip's values provably

@@ -97,7 +97,7 @@ struct ClassDef {
   int lanes, k, kind, width;
 };
 constexpr int kNumS16 = 21;     // s16x2 classes chosen by cost
-constexpr int kNumClasses = kNumS16 + 3;  // + the s32 class, the hybrid class, the strip-team class
+constexpr int kNumClasses = kNumS16 + 4;  // + the s32, hybrid, strip-team and long classes
 constexpr ClassDef kClasses[kNumClasses] = {
     {16, 4, IPUMA_KERNEL_S16_L16_K4, 64},    {16, 8, IPUMA_KERNEL_S16_L16_K8, 128},
     {16, 12, IPUMA_KERNEL_S16_L16_K12, 192}, {16, 16, IPUMA_KERNEL_S16_L16_K16, 256},
@@ -111,8 +111,9 @@ constexpr ClassDef kClasses[kNumClasses] = {
     {8, 12, IPUMA_KERNEL_S16_L8_K12, 96},    {8, 14, IPUMA_KERNEL_S16_L8_K14, 112},
     {8, 16, IPUMA_KERNEL_S16_L8_K16, 128},
     {32, 16, IPUMA_KERNEL_S32_K16, 512},     {32, 16, IPUMA_KERNEL_S16_HYBRID, 512},
-    {32, 16, IPUMA_KERNEL_S16_TEAM, 512},
+    {32, 16, IPUMA_KERNEL_S16_TEAM, 512},    {32, 16, IPUMA_KERNEL_S16_L32_K16, 512},
 };
+static_assert(kNumClasses <= NCLASS_MAX, "class tables");
 constexpr int kClsWidest = 5;  // widest wavefront class (very long |A|)
 constexpr int kMaxTimed = IPUMA_MAX_TIMED;  // launches timed per call (time_launches)
 constexpr int kClsThread = 6;  // per-thread class k_thread<16>
@@ -127,6 +128,9 @@ constexpr int kClsHi = kNumS16 + 1;
 // batch's strip count.
 constexpr int kClsTeam = kNumS16 + 2;
 constexpr int kTeamWarpsDefault = 8;
+// Long class: the widest strips with one tag bit, for pairs whose score may
+// pass what class kClsWidest holds (BinParams::fit).
+constexpr int kClsLong = kNumS16 + 3;
 // Per-thread class: rows it accepts (its boundary scratch is rows x threads)
 // and the share of the batch's time one of its pairs may take.
 constexpr int kThrMaxRows = 2048;
@@ -136,7 +140,9 @@ constexpr float kThrLatencyShare = 0.5f;
 // / packing efficiency).  In small batches that sends pairs to the class
 // that finishes them soonest: there one long pair, not throughput, sets the
 // batch's time.
-constexpr float kLatencyShare = 0.06f;  // measured best of 0.03-0.25 on the protein workloads
+// (B200, 300,000 DNA pairs with start coordinates: 7.07 ms at 0.06, 4.93 at
+// 0.25, 4.90 at 0.5; 200,000 protein pairs 11.0, 11.7 and 11.9 ms.)
+constexpr float kLatencyShare = 0.25f;
 constexpr float kPackingEfficiency = 0.85f;
 constexpr float kLatencyMinBatchPs = 0.f;
 // Option "concurrent" = 3 (default) picks the launch mode by batch size:
@@ -149,6 +155,11 @@ constexpr int kShareModeMaxPairs = 48000;
 // (K = 4, 8, 12, 16), since every class launch costs a few microseconds
 // even when empty.
 constexpr int kFineClassMinPairs = 150000;
+// 8-lane groups of linear-gap strips (strip_ref) from this many pairs: an
+// item holds eight pairs instead of four, which leaves warps without work
+// in smaller batches (10,000 pairs of 150 x 150-300 on B200: 329 us with 8
+// lanes, 290 with 16).
+constexpr int kEightLaneMinPairs = 48000;
 constexpr unsigned kCoarseClasses = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 5);
 // 8-lane groups for the five narrowest strip widths (64 to 128 columns):
 // twice the columns per lane over a wavefront half as deep, so the per-step
@@ -213,7 +224,9 @@ struct ipuma_engine {
   SwConst sc{};
   bool fast_ok = false;  // wavefront kernels valid for this scoring
   bool s16_ok = false;   // s16x2 lanes valid for this scoring
-  int s16_max_len = 0;
+  // Which lanes the 16-bit classes run (kernel_of), fixed by the scoring.
+  enum Cells { kLinear, kAffine, kAnyScore } cells = kAnyScore;
+  int typical = 1;       // score of a typical identical residue (BinParams::fit)
 
   // options
   int scheduler = 0;
@@ -341,7 +354,9 @@ int occupancy_grid(ipuma_engine* e, K kernel, int smem, int threads = kThreads) 
 // Letters of the query profile for codes of `bits` bits: 2-bit codes are
 // A/C/G/T (codes 1..4), so their profile needs four rows, not one per
 // letter of the alphabet -- less shared memory, more resident blocks.
-int prof_letters(const ipuma_engine* e, int bits) { return (bits == 2 && e->M >= 5) ? 4 : e->M; }
+int prof_letters(const ipuma_engine* e, int bits) {
+  return (bits == 2 && e->sw.datatype == IPUMA_DT_NUCLEIC_ACID && e->M >= 5) ? 4 : e->M;
+}
 
 // Shared memory of a wavefront launch whose profile has P letters (P < 0:
 // one per letter of the alphabet).
@@ -350,16 +365,119 @@ int smem_for(const ipuma_engine* e, int P = -1) {
   return SmemLayout<T, K, LANES>::total(e->M, P < 0 ? e->M : P, kWarpsPerBlock);
 }
 
-// Grid of a k_batched<T, K, LANES, HYB> launch (the instantiation for the
-// engine's forwardOnly, which is fixed at creation) with a P-letter profile.
+// The k_batched instantiation a class launches (all share one signature).
+using BatchedKernel = decltype(&k_batched<LaneS32, 16, 32>);
+struct KernelRef {
+  BatchedKernel fn = nullptr;  // null: the class has no kernel for this scoring
+  int lanes = 0, k = 0, smem = 0;
+  int buffers = 2;             // strip-boundary columns per lane group
+  int shift = 0;               // bits the lanes hold scores shifted by
+  int limit = 0;               // largest score the lanes may hold
+};
+
 template <class T, int K, int LANES, bool HYB = false>
-int batched_grid(ipuma_engine* e, int P) {
-  return e->sc.forwardOnly ? occupancy_grid(e, k_batched<T, K, LANES, HYB, true>, smem_for<T, K, LANES>(e, P))
-                           : occupancy_grid(e, k_batched<T, K, LANES, HYB, false>, smem_for<T, K, LANES>(e, P));
+KernelRef kernel_ref(const ipuma_engine* e, int P) {
+  KernelRef r;
+  r.fn = e->sc.forwardOnly ? k_batched<T, K, LANES, HYB, true> : k_batched<T, K, LANES, HYB, false>;
+  r.lanes = LANES;
+  r.k = K;
+  r.smem = smem_for<T, K, LANES>(e, P);
+  r.buffers = HYB ? 3 : 2;
+  r.shift = kProfShift<T>;
+  r.limit = Cell<T>::limit(e->sc);
+  return r;
+}
+
+// Lanes of the 16-bit classes.  Linear gaps keep four tag bits (2,047
+// points), which fit every pair their strips are meant for; affine scorings,
+// proteins mostly, keep two (8,191 points) so that only very long or
+// near-identical pairs need the long class, whose lanes hold 16 bits.
+// Matrices whose scaled values pass a profile byte run unscaled.
+using LaneLin = LaneTag<4, true, true>;
+using LaneAff = LaneTag<2, false, true>;
+using LaneAny = LaneTag<2, false, false>;
+using LaneLinLong = LaneTag<1, true, false>;
+using LaneAffLong = LaneTag<1, false, false>;
+
+// Strips of 16 * K columns: 16 lanes of K, or 8 lanes of 2 K with the
+// four-row profile, whose shared memory then allows it (measured on B200,
+// 60,000 pairs of 240 x 320, linear gaps: 16 lanes 6488, 8 lanes 7061
+// GCUPS -- a lane's work per step covers twice the cells).  Affine lanes of
+// more than 24 columns spill; they stay at 16.
+template <int K>
+KernelRef strip_ref(const ipuma_engine* e, int P, bool eight) {
+  if (e->cells == ipuma_engine::kLinear)
+    return P < e->M && eight ? kernel_ref<LaneLin, 2 * K, 8>(e, P) : kernel_ref<LaneLin, K, 16>(e, P);
+  if (e->cells == ipuma_engine::kAffine) return kernel_ref<LaneAff, K, 16>(e, P);
+  if constexpr (K % 4 == 0) return kernel_ref<LaneAny, K, 16>(e, P);
+  return KernelRef{};
+}
+template <int K>
+KernelRef narrow_ref(const ipuma_engine* e, int P) {
+  if (e->cells == ipuma_engine::kLinear) return kernel_ref<LaneLin, K, 8>(e, P);
+  if (e->cells == ipuma_engine::kAffine) return kernel_ref<LaneAff, K, 8>(e, P);
+  return KernelRef{};
+}
+template <int K>
+KernelRef wide_ref(const ipuma_engine* e, int P) {
+  if (e->cells == ipuma_engine::kLinear) return kernel_ref<LaneLin, K, 32>(e, P);
+  if (e->cells == ipuma_engine::kAffine) return kernel_ref<LaneAff, K, 32>(e, P);
+  return kernel_ref<LaneAny, K, 32>(e, P);
+}
+
+// Kernel of a wavefront class for a P-letter profile (not the per-thread
+// and the team class); eight: the batch fills 8-lane groups.
+KernelRef kernel_of(const ipuma_engine* e, int cls, int P, bool eight) {
+  switch (cls) {
+    case 0: return strip_ref<4>(e, P, eight);
+    case 10: return strip_ref<5>(e, P, eight);
+    case 7: return strip_ref<6>(e, P, eight);
+    case 11: return strip_ref<7>(e, P, eight);
+    case 1: return strip_ref<8>(e, P, eight);
+    case 12: return strip_ref<9>(e, P, eight);
+    case 8: return strip_ref<10>(e, P, eight);
+    case 13: return strip_ref<11>(e, P, eight);
+    case 2: return strip_ref<12>(e, P, eight);
+    case 14: return strip_ref<13>(e, P, eight);
+    case 9: return strip_ref<14>(e, P, eight);
+    case 15: return strip_ref<15>(e, P, eight);
+    case 3: return strip_ref<16>(e, P, eight);
+    case 16: return narrow_ref<8>(e, P);
+    case 17: return narrow_ref<10>(e, P);
+    case 18: return narrow_ref<12>(e, P);
+    case 19: return narrow_ref<14>(e, P);
+    case 20: return narrow_ref<16>(e, P);
+    case 4: return wide_ref<12>(e, P);
+    case 5: return wide_ref<16>(e, P);
+    case kClsLong:
+      return e->cells == ipuma_engine::kLinear ? kernel_ref<LaneLinLong, 16, 32>(e, P)
+                                               : kernel_ref<LaneAffLong, 16, 32>(e, P);
+    case kClsHi: return kernel_ref<LaneHi, 16, 32, true>(e, P);
+    case kClsS32: return kernel_ref<LaneS32, 16, 32>(e, P);
+    default: return KernelRef{};
+  }
+}
+
+int kernel_grid(ipuma_engine* e, const KernelRef& r) { return r.fn ? occupancy_grid(e, r.fn, r.smem) : 0; }
+
+// Kernel of the strip-team class (linear gaps or affine, one tag bit).
+using TeamKernel = decltype(&k_strips<LaneAffLong, 16>);
+TeamKernel team_kernel(const ipuma_engine* e) {
+  return e->cells == ipuma_engine::kLinear ? k_strips<LaneLinLong, 16> : k_strips<LaneAffLong, 16>;
+}
+
+// Constants of a launch whose lanes hold scores shifted by `shift` bits.
+SwConst lane_const(SwConst sc, int shift) {
+  const auto splat = [&](int x) { return (uint32_t)((x << shift) & 0xffff) * 0x00010001u; };
+  sc.one = 1;
+  sc.gE2 = splat(sc.gE);
+  sc.gIgE2 = splat(sc.gIgE);
+  sc.gEp2 = splat(std::max(sc.gE, sc.gIgE));
+  return sc;
 }
 
 int team_smem(const ipuma_engine* e, int P, int warps) {
-  return SmemLayout<Lane16, 16, 32>::total(e->M, P, warps);
+  return SmemLayout<LaneAffLong, 16, 32>::total(e->M, P, warps);
 }
 
 // Static shared memory of k_strips (progress words, merge slots) plus slack.
@@ -379,7 +497,7 @@ int team_warps_for(const ipuma_engine* e, int P, int maxA) {
 
 // Grid of a k_strips<16> launch with `warps` warps per block.
 int team_grid(ipuma_engine* e, int P, int warps) {
-  return occupancy_grid(e, k_strips<16>, team_smem(e, P, warps), 32 * warps);
+  return occupancy_grid(e, team_kernel(e), team_smem(e, P, warps), 32 * warps);
 }
 
 template <int K>
@@ -393,38 +511,16 @@ long thread_threads(ipuma_engine* e) {
   return (long)occupancy_grid(e, k_thread<K>, thread_smem<K>(e)) * kThreads;
 }
 
-// Lane groups (one scratch slice each) of the widest batched launch (either
-// profile size).
-int max_batched_groups(ipuma_engine* e) {
-  int g = 0;
+// Fills the grid cache (no occupancy query or attribute change happens
+// later, during a capture): every wavefront class and team size, for either
+// profile size.
+void warm_grids(ipuma_engine* e) {
   for (int P : {e->M, prof_letters(e, 2)}) {
-    g = std::max(g, batched_grid<Lane16, 4, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 8, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 12, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 16, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 6, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 10, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 14, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 5, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 7, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 9, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 11, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 13, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 15, 16>(e, P) * 2);
-    g = std::max(g, batched_grid<Lane16, 8, 8>(e, P) * 4);
-    g = std::max(g, batched_grid<Lane16, 10, 8>(e, P) * 4);
-    g = std::max(g, batched_grid<Lane16, 12, 8>(e, P) * 4);
-    g = std::max(g, batched_grid<Lane16, 14, 8>(e, P) * 4);
-    g = std::max(g, batched_grid<Lane16, 16, 8>(e, P) * 4);
-    g = std::max(g, batched_grid<Lane16, 12, 32>(e, P));
-    g = std::max(g, batched_grid<Lane16, 16, 32>(e, P));
-    g = std::max(g, batched_grid<LaneS32, 16, 32>(e, P));
-    g = std::max(g, batched_grid<LaneHi, 16, 32, true>(e, P));
-    // Warm the cache of the team grids (no occupancy query during a capture).
+    for (int c = 0; c < kNumClasses; ++c)
+      for (bool eight : {false, true}) kernel_grid(e, kernel_of(e, c, P, eight));
     for (int w = 2; w <= std::min(e->team_warps, kTeamMaxWarps); ++w)
       if (team_smem(e, P, w) + kTeamStaticSmem <= e->smem_optin) team_grid(e, P, w);
   }
-  return g * kWarpsPerBlock;
 }
 
 // Device buffers of one run of the batched pipeline: the control block and
@@ -470,19 +566,16 @@ int timed_end(ipuma_engine* e, cudaStream_t s) {
 
 // allot_idx = entry of the control block's ClassAllot table (the class, or
 // NCLASS_MAX for the s32 rerun).
-template <class T, int K, int LANES, bool HYB = false>
-int launch_batched(ipuma_engine* e, const SwConst& sc, const RunBufs& rb, cudaStream_t s, const uint8_t* codes,
-                   const PairDesc* pairs, const int* list, const int* range, int* head, long rowsCap,
-                   int* score, int* arange, int* brange, int kind, int cls, int allot_idx) {
-  const int smem = smem_for<T, K, LANES>(e, sc.P);
-  const int grid = batched_grid<T, K, LANES, HYB>(e, sc.P);
+int launch_batched(ipuma_engine* e, const KernelRef& kr, const SwConst& sc, const RunBufs& rb, cudaStream_t s,
+                   const uint8_t* codes, const PairDesc* pairs, const int* list, const int* range, int* head,
+                   long rowsCap, int* score, int* arange, int* brange, int kind, int cls, int allot_idx) {
+  const int grid = kernel_grid(e, kr);
   int* ctl = rb.ctl;
   auto* cells = reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS);
   int rc;
   if ((rc = timed_begin(e, s, kind, cls))) return rc;
-  auto* kern = e->sc.forwardOnly ? k_batched<T, K, LANES, HYB, true> : k_batched<T, K, LANES, HYB, false>;
-  kern<<<grid, kThreads, smem, s>>>(
-      sc, e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(),
+  kr.fn<<<grid, kThreads, kr.smem, s>>>(
+      lane_const(sc, kr.shift), e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(),
       rowsCap, score, arange, brange, rb.ovf->as<int>(), cells + CELLS_RERUN,
       reinterpret_cast<DevStatus*>(ctl + CTL_STATUS),
       reinterpret_cast<const ClassAllot*>(ctl + CTL_ALLOT) + allot_idx,
@@ -501,8 +594,8 @@ int launch_team(ipuma_engine* e, const SwConst& sc, const RunBufs& rb, cudaStrea
   auto* cells = reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS);
   int rc;
   if ((rc = timed_begin(e, s, kClasses[kClsTeam].kind, kClsTeam))) return rc;
-  k_strips<16><<<grid, 32 * warps, smem, s>>>(
-      sc, e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(), rowsCap, score, arange,
+  team_kernel(e)<<<grid, 32 * warps, smem, s>>>(
+      lane_const(sc, 0), e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(), rowsCap, score, arange,
       brange, rb.ovf->as<int>(), cells + CELLS_RERUN, reinterpret_cast<DevStatus*>(ctl + CTL_STATUS),
       reinterpret_cast<const ClassAllot*>(ctl + CTL_ALLOT) + kClsTeam,
       e->trace ? reinterpret_cast<unsigned long long*>(ctl + CTL_TRACE) + 2 * kClsTeam : nullptr);
@@ -546,44 +639,21 @@ long thread_rows(const ipuma_engine* e, int maxA, int maxB) {
 // thread_rows per thread.
 // Full-occupancy grid and strip scratch (int2) per block of every class,
 // for a P-letter profile.
-void class_grids(ipuma_engine* e, int P, int maxA, int maxB, int* grid, long long* spb) {
+void class_grids(ipuma_engine* e, int P, bool eight, int maxA, int maxB, int* grid, long long* spb) {
   const long long rowsCap = std::max(1, maxB);
   for (int c = 0; c < kNumClasses; ++c) {
-    switch (c) {
-      case kClsHi: grid[c] = batched_grid<LaneHi, 16, 32, true>(e, P); break;
-      case 0: grid[c] = batched_grid<Lane16, 4, 16>(e, P); break;
-      case 1: grid[c] = batched_grid<Lane16, 8, 16>(e, P); break;
-      case 2: grid[c] = batched_grid<Lane16, 12, 16>(e, P); break;
-      case 3: grid[c] = batched_grid<Lane16, 16, 16>(e, P); break;
-      case 4: grid[c] = batched_grid<Lane16, 12, 32>(e, P); break;
-      case 5: grid[c] = batched_grid<Lane16, 16, 32>(e, P); break;
-      case kClsThread: grid[c] = (int)(thread_threads<16>(e) / kThreads); break;
-      case 7: grid[c] = batched_grid<Lane16, 6, 16>(e, P); break;
-      case 8: grid[c] = batched_grid<Lane16, 10, 16>(e, P); break;
-      case 9: grid[c] = batched_grid<Lane16, 14, 16>(e, P); break;
-      case 10: grid[c] = batched_grid<Lane16, 5, 16>(e, P); break;
-      case 11: grid[c] = batched_grid<Lane16, 7, 16>(e, P); break;
-      case 12: grid[c] = batched_grid<Lane16, 9, 16>(e, P); break;
-      case 13: grid[c] = batched_grid<Lane16, 11, 16>(e, P); break;
-      case 14: grid[c] = batched_grid<Lane16, 13, 16>(e, P); break;
-      case 15: grid[c] = batched_grid<Lane16, 15, 16>(e, P); break;
-      case 16: grid[c] = batched_grid<Lane16, 8, 8>(e, P); break;
-      case 17: grid[c] = batched_grid<Lane16, 10, 8>(e, P); break;
-      case 18: grid[c] = batched_grid<Lane16, 12, 8>(e, P); break;
-      case 19: grid[c] = batched_grid<Lane16, 14, 8>(e, P); break;
-      case 20: grid[c] = batched_grid<Lane16, 16, 8>(e, P); break;
-      case kClsTeam: {
-        const int w = team_warps_for(e, P, maxA);
-        grid[c] = w ? team_grid(e, P, w) : 0;
-        spb[c] = (long long)w * rowsCap;  // one boundary column per warp of a team
-        continue;
-      }
-      default: grid[c] = batched_grid<LaneS32, 16, 32>(e, P); break;
-    }
-    if (c == kClsThread)
+    if (c == kClsTeam) {
+      const int w = team_warps_for(e, P, maxA);
+      grid[c] = w ? team_grid(e, P, w) : 0;
+      spb[c] = (long long)w * rowsCap;  // one boundary column per warp of a team
+    } else if (c == kClsThread) {
+      grid[c] = (int)(thread_threads<16>(e) / kThreads);
       spb[c] = (long long)kThreads * thread_rows(e, maxA, maxB);
-    else
-      spb[c] = (long long)kWarpsPerBlock * (32 / kClasses[c].lanes) * (c == kClsHi ? 3 : 2) * rowsCap;
+    } else {
+      const KernelRef kr = kernel_of(e, c, P, eight);
+      grid[c] = kernel_grid(e, kr);
+      spb[c] = kr.fn ? (long long)kWarpsPerBlock * (32 / kr.lanes) * kr.buffers * rowsCap : 0;
+    }
   }
 }
 
@@ -595,15 +665,16 @@ size_t scratch_int2(ipuma_engine* e, int maxA, int maxB) {
   int grid[NCLASS_MAX + 1];
   long long spb[NCLASS_MAX + 1];
   long long full = 0, round = 0;
-  for (int P : {e->M, prof_letters(e, 2)}) {  // the smaller profile may fit more blocks
-    class_grids(e, P, maxA, maxB, grid, spb);
-    long long r = 0;
-    for (int c = 0; c < kNumClasses; ++c) {
-      full = std::max(full, (long long)grid[c] * spb[c]);
-      r += spb[c];
+  for (int P : {e->M, prof_letters(e, 2)})  // the smaller profile may fit more blocks
+    for (bool eight : {false, true}) {
+      class_grids(e, P, eight, maxA, maxB, grid, spb);
+      long long r = 0;
+      for (int c = 0; c < kNumClasses; ++c) {
+        full = std::max(full, (long long)grid[c] * spb[c]);
+        r += spb[c];
+      }
+      round = std::max(round, r);
     }
-    round = std::max(round, r);
-  }
   return (size_t)std::max(full + round, 2 * full);
 }
 
@@ -612,7 +683,7 @@ size_t scratch_int2(ipuma_engine* e, int maxA, int maxB) {
 // The hybrid class and the widest class (the long pairs of a heavy-tailed
 // batch) come first and land on different streams, so the widest class's
 // blocks start on the SMs the hybrid class frees during its tail.
-constexpr int kLaunchOrder[kNumClasses] = {23, 22, 5, 21, 4, 6, 3, 15, 9, 14, 2, 13, 8, 12, 1, 20, 11, 19, 7, 18, 10, 17, 0, 16};
+constexpr int kLaunchOrder[kNumClasses] = {23, 22, 24, 5, 21, 4, 6, 3, 15, 9, 14, 2, 13, 8, 12, 1, 20, 11, 19, 7, 18, 10, 17, 0, 16};
 
 int reserve_bufs(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, int n, int maxA, int maxB) {
   int rc;
@@ -672,15 +743,20 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.cls_s32 = kClsS32;
   bp.cls_hi = e->hybrid ? kClsHi : kClsS32;
   bp.nclass = kNumClasses;
-  bp.s16_max_len = e->s16_max_len;
   bp.force_s32 = e->s16_ok ? 0 : 1;
+  const bool eight = n >= kEightLaneMinPairs;
+  KernelRef kr[kNumClasses];
   for (int c = 0; c < kNumClasses; ++c) {
-    bp.lanes[c] = kClasses[c].lanes;
+    kr[c] = kernel_of(e, c, sc.P, eight);
+    bp.lanes[c] = kr[c].fn ? kr[c].lanes : kClasses[c].lanes;
     bp.width[c] = kClasses[c].width;
     bp.slot_ps[c] = e->slot_ps[c];
     bp.strip_ps[c] = e->strip_ps[c];
+    bp.fit[c] = (kr[c].fn ? kr[c].limit : e->sc.s16Limit) / e->typical;
   }
   bp.widest = kClsWidest;
+  bp.cls_long = kClsLong;
+  bp.s16_max_len = e->maxSub > 0 ? kr[kClsLong].limit / e->maxSub : (1 << 30);
   const long thrThreads = thread_threads<16>(e);
   bp.thr_cls = kClsThread;
   bp.thr_on = e->thread_class && bits == 8;
@@ -698,8 +774,10 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   unsigned enabled = kCoarseClasses | (1u << kClsS32);
   if (e->hybrid) enabled |= 1u << kClsHi;
   if (n >= kFineClassMinPairs) enabled |= kFineClasses;
+  // The long class, when the batch may hold a pair past the widest's scores.
+  if (std::min(maxA, maxB) > bp.fit[kClsWidest]) enabled |= 1u << kClsLong;
   if (e->thread_class && bits == 8) enabled |= 1u << kClsThread;  // k_thread reads bytes only
-  if (sc.P < e->M) {
+  if (sc.P < e->M && (eight || e->cells != ipuma_engine::kLinear)) {
     // Four-row profiles: the narrow widths in 8-lane groups.
     for (const auto& w : kNarrowPairs)
       if ((enabled >> w[0]) & 1u) enabled = (enabled & ~(1u << w[0])) | (1u << w[1]);
@@ -713,18 +791,26 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
                 kClsTeam + 1);
   if (teamW >= 2 && maxA > kClasses[kClsTeam].width && e->tile_k == 0) enabled |= 1u << kClsTeam;
   if (e->tile_k > 0) enabled |= 1u << (e->tile_k - 1);
+  for (int c = 0; c < kNumClasses; ++c)
+    if (c != kClsThread && c != kClsTeam && !kr[c].fn) {
+      if (e->tile_k == c + 1) return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d has no kernel for this scoring", e->tile_k);
+      enabled &= ~(1u << c);
+    }
   bp.enabled = enabled;
   bp.team_cls = ((enabled >> kClsTeam) & 1u) ? kClsTeam : -1;
   bp.team_warps = std::max(teamW, 1);
-  class_grids(e, sc.P, maxA, maxB, bp.grid, bp.scr_per_block);
+  class_grids(e, sc.P, eight, maxA, maxB, bp.grid, bp.scr_per_block);
   bp.scr_cap = (long long)(rb.scratch->cap / sizeof(int2));
   float slot_min = 1e30f;
   for (int c = 0; c < kNumS16; ++c) {
     // cell slots one warp step covers: 32 lanes x k columns x 2 pairs
     // (the per-thread class: 32 threads x 16 columns x 2 pairs per row)
-    bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * kWarpsPerBlock);
-    if (c != kClsThread) slot_min = std::min(slot_min, e->slot_ps[c]);
+    const int k = kr[c].fn ? kr[c].k : kClasses[c].k;
+    bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)k * (float)(bp.grid[c] * kWarpsPerBlock);
+    if (kr[c].fn) slot_min = std::min(slot_min, e->slot_ps[c]);
   }
+  bp.step_ps[kClsLong] =
+      e->slot_ps[kClsLong] * 64.f * (float)kClasses[kClsLong].k * (float)(bp.grid[kClsLong] * kWarpsPerBlock);
   // A warp of a team steps like one of the widest class's warps.
   bp.step_ps[kClsTeam] =
       e->slot_ps[kClsTeam] * 64.f * (float)kClasses[kClsTeam].k * (float)(bp.grid[kClsTeam] * bp.team_warps);
@@ -749,7 +835,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.n_codes = (long long)n_codes;
   bp.bits = bits;
   bp.M = e->M;
-  bp.s16_limit = e->sc.s16Limit;
+  bp.s16_limit = kr[kClsLong].limit;
   if ((rc = rb.flag->ensure((size_t)n + 64, s))) return rc;
   const int nkeys = bp.nclass * NBUCKET;
   const int tb = 256;
@@ -796,67 +882,26 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     return IPUMA_OK;
   };
   const int* R = ctl + CTL_RANGES;
-#define IPUMA_LAUNCH(T, K, L, cls)                                                                     \
-  if ((enabled >> (cls)) & 1u) {                                                                       \
-    cudaStream_t cs = on(cls);                                                                         \
-    if ((rc = launch_batched<T, K, L>(e, sc, rb, cs, codes, pairs, list, R + 2 * (cls), heads + (cls), \
-                                      rowsCap, score, arange, brange, kClasses[cls].kind, cls, cls)))  \
-      return rc;                                                                                       \
-    if ((rc = done(cls))) return rc;                                                                   \
-    ++*launches;                                                                                       \
-  }
-  if ((enabled >> kClsTeam) & 1u) {
-    cudaStream_t cs = on(kClsTeam);
-    if ((rc = launch_team(e, sc, rb, cs, codes, pairs, list, R + 2 * kClsTeam, heads + kClsTeam, rowsCap, score,
-                          arange, brange, teamW)))
-      return rc;
-    if ((rc = done(kClsTeam))) return rc;
+  for (const int c : kLaunchOrder) {
+    if (!((enabled >> c) & 1u)) continue;
+    cudaStream_t cs = on(c);
+    if (c == kClsTeam)
+      rc = launch_team(e, sc, rb, cs, codes, pairs, list, R + 2 * c, heads + c, rowsCap, score, arange, brange,
+                       teamW);
+    else if (c == kClsThread)
+      rc = launch_thread<16>(e, rb, cs, codes, pairs, list, R + 2 * c, heads + c, thread_rows(e, maxA, maxB), score,
+                             arange, brange, c);
+    else
+      rc = launch_batched(e, kr[c], sc, rb, cs, codes, pairs, list, R + 2 * c, heads + c, rowsCap, score, arange,
+                          brange, kClasses[c].kind, c, c);
+    if (rc || (rc = done(c))) return rc;
     ++*launches;
   }
-  if ((enabled >> kClsHi) & 1u) {
-    cudaStream_t cs = on(kClsHi);
-    if ((rc = launch_batched<LaneHi, 16, 32, true>(e, sc, rb, cs, codes, pairs, list, R + 2 * kClsHi,
-                                                      heads + kClsHi, rowsCap, score, arange, brange,
-                                                      kClasses[kClsHi].kind, kClsHi, kClsHi)))
-      return rc;
-    if ((rc = done(kClsHi))) return rc;
-    ++*launches;
-  }
-  IPUMA_LAUNCH(LaneS32, 16, 32, kClsS32)
-  IPUMA_LAUNCH(Lane16, 16, 32, 5)
-  IPUMA_LAUNCH(Lane16, 12, 32, 4)
-  if ((enabled >> kClsThread) & 1u) {
-    cudaStream_t cs = on(kClsThread);
-    if ((rc = launch_thread<16>(e, rb, cs, codes, pairs, list, R + 2 * kClsThread, heads + kClsThread,
-                                thread_rows(e, maxA, maxB), score, arange, brange, kClsThread)))
-      return rc;
-    if ((rc = done(kClsThread))) return rc;
-    ++*launches;
-  }
-  IPUMA_LAUNCH(Lane16, 16, 16, 3)
-  IPUMA_LAUNCH(Lane16, 15, 16, 15)
-  IPUMA_LAUNCH(Lane16, 14, 16, 9)
-  IPUMA_LAUNCH(Lane16, 13, 16, 14)
-  IPUMA_LAUNCH(Lane16, 12, 16, 2)
-  IPUMA_LAUNCH(Lane16, 11, 16, 13)
-  IPUMA_LAUNCH(Lane16, 10, 16, 8)
-  IPUMA_LAUNCH(Lane16, 9, 16, 12)
-  IPUMA_LAUNCH(Lane16, 8, 16, 1)
-  IPUMA_LAUNCH(Lane16, 16, 8, 20)
-  IPUMA_LAUNCH(Lane16, 7, 16, 11)
-  IPUMA_LAUNCH(Lane16, 14, 8, 19)
-  IPUMA_LAUNCH(Lane16, 6, 16, 7)
-  IPUMA_LAUNCH(Lane16, 12, 8, 18)
-  IPUMA_LAUNCH(Lane16, 5, 16, 10)
-  IPUMA_LAUNCH(Lane16, 10, 8, 17)
-  IPUMA_LAUNCH(Lane16, 4, 16, 0)
-  IPUMA_LAUNCH(Lane16, 8, 8, 16)
-#undef IPUMA_LAUNCH
   // Exact 32-bit rerun of the s16x2 pairs whose score may have overflowed
   // (after every class: it reads their overflow list).
-  if ((rc = launch_batched<LaneS32, 16, 32>(e, sc, rb, s, codes, pairs, rb.ovf->as<int>(), ctl + CTL_STATUS + 1,
-                                            heads + NCLASS_MAX, rowsCap, score, arange, brange,
-                                            IPUMA_KERNEL_S32_RERUN, CELLS_RERUN, NCLASS_MAX)))
+  if ((rc = launch_batched(e, kr[kClsS32], sc, rb, s, codes, pairs, rb.ovf->as<int>(), ctl + CTL_STATUS + 1,
+                           heads + NCLASS_MAX, rowsCap, score, arange, brange, IPUMA_KERNEL_S32_RERUN, CELLS_RERUN,
+                           NCLASS_MAX)))
     return rc;
   *launches += 1;
   return IPUMA_OK;
@@ -1026,6 +1071,8 @@ void set_s32_rates(ipuma_engine* e) {
   // pipeline that fills and drains once per item: modelled in pair_key).
   e->slot_ps[kClsTeam] = e->slot_ps[kClsWidest];
   e->strip_ps[kClsTeam] = e->strip_ps[kClsWidest];
+  e->slot_ps[kClsLong] = e->slot_ps[kClsWidest];
+  e->strip_ps[kClsLong] = e->strip_ps[kClsWidest];
 }
 
 void set_default_rates(ipuma_engine* e) {
@@ -1050,8 +1097,8 @@ std::string tune_key(const ipuma_engine* e) {
   char buf[512];
   // The rates are those of the engine's kernels, which differ by mode: a
   // full alignment (forward + reverse pass) takes longer per cell.
-  snprintf(buf, sizeof(buf), "%s|sm%d%d|M=%d|sim=%d|gI=%d|gE=%d|fwd=%d|v7", prop.name, prop.major, prop.minor, e->M,
-           e->sw.similarity, e->sw.gap_init, e->sw.gap_extend, e->sc.forwardOnly);
+  snprintf(buf, sizeof(buf), "%s|sm%d%d|M=%d|sim=%d|gI=%d|gE=%d|fwd=%d|cells=%d|v8", prop.name, prop.major, prop.minor, e->M,
+           e->sw.similarity, e->sw.gap_init, e->sw.gap_extend, e->sc.forwardOnly, (int)e->cells);
   for (char* c = buf; *c; ++c)
     if (*c == '\t' || *c == '\n') *c = ' ';
   return buf;
@@ -1181,30 +1228,9 @@ int run_autotune(ipuma_engine* e, const char* cache_path) {
     // far more pairs resident, so two rounds of items suffice there.
     const int perItem = L > 0 ? (32 / L) * 2 : 64;
     const int rounds = L > 0 ? 6 : 2;
-    int grid = 1;
-    switch (c) {
-      case 0: grid = batched_grid<Lane16, 4, 16>(e, e->M); break;
-      case 1: grid = batched_grid<Lane16, 8, 16>(e, e->M); break;
-      case 2: grid = batched_grid<Lane16, 12, 16>(e, e->M); break;
-      case 3: grid = batched_grid<Lane16, 16, 16>(e, e->M); break;
-      case 4: grid = batched_grid<Lane16, 12, 32>(e, e->M); break;
-      case 5: grid = batched_grid<Lane16, 16, 32>(e, e->M); break;
-      case 7: grid = batched_grid<Lane16, 6, 16>(e, e->M); break;
-      case 8: grid = batched_grid<Lane16, 10, 16>(e, e->M); break;
-      case 9: grid = batched_grid<Lane16, 14, 16>(e, e->M); break;
-      case 10: grid = batched_grid<Lane16, 5, 16>(e, e->M); break;
-      case 11: grid = batched_grid<Lane16, 7, 16>(e, e->M); break;
-      case 12: grid = batched_grid<Lane16, 9, 16>(e, e->M); break;
-      case 13: grid = batched_grid<Lane16, 11, 16>(e, e->M); break;
-      case 14: grid = batched_grid<Lane16, 13, 16>(e, e->M); break;
-      case 15: grid = batched_grid<Lane16, 15, 16>(e, e->M); break;
-      case 16: grid = batched_grid<Lane16, 8, 8>(e, e->M); break;
-      case 17: grid = batched_grid<Lane16, 10, 8>(e, e->M); break;
-      case 18: grid = batched_grid<Lane16, 12, 8>(e, e->M); break;
-      case 19: grid = batched_grid<Lane16, 14, 8>(e, e->M); break;
-      case 20: grid = batched_grid<Lane16, 16, 8>(e, e->M); break;
-      default: grid = (int)(thread_threads<16>(e) / kThreads); break;
-    }
+    const KernelRef kr = kernel_of(e, c, e->M, true);
+    if (c != kClsThread && !kr.fn) continue;  // no kernel of this class for this scoring
+    const int grid = c == kClsThread ? (int)(thread_threads<16>(e) / kThreads) : kernel_grid(e, kr);
     const int minPairs = grid * kWarpsPerBlock * perItem * rounds;
     // (strips, rows) of the two calibration batches.  The per-thread class
     // passes a boundary column through global memory at every strip, so
@@ -1659,9 +1685,23 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   e->sc.P = m;
   e->sc.pshift = 0;
   e->s16_ok = e->fast_ok;
-  e->s16_max_len = e->maxSub > 0 ? (e->sc.s16Limit / e->maxSub) : (1 << 30);
+  // Lanes of the 16-bit classes: linear gaps, affine with every scaled
+  // value in a profile byte, or any.
+  const auto scaled = [&](int bias, int bits) {
+    return (minSub + bias) * (1 << bits) >= -128 && (e->maxSub + bias) * (1 << bits) <= 127;
+  };
+  e->cells = gI == 0 && scaled(-gE, kProfShift<LaneLin>) ? ipuma_engine::kLinear
+             : scaled(0, kProfShift<LaneAff>)            ? ipuma_engine::kAffine
+                                                         : ipuma_engine::kAnyScore;
+  int diag = 0, letters = 0;
+  for (int x = 0; x < m; ++x)
+    if (e->sim[x * m + x] > 0) {
+      diag += e->sim[x * m + x];
+      ++letters;
+    }
+  e->typical = letters > 0 ? std::max(1, (diag + letters - 1) / letters) : 1;
   set_default_rates(e.get());
-  max_batched_groups(e.get());  // warm the grid cache
+  warm_grids(e.get());
   thread_threads<16>(e.get());
   *out = e.release();
   return IPUMA_OK;

@@ -68,14 +68,10 @@ __global__ void __launch_bounds__(64) k_noalloc(SwConst sc, SimParam sim, const 
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int8_t* s_simp = reinterpret_cast<int8_t*>(smem);
-  uint8_t* wbase = smem + L::simp_bytes(sc.M) + wib * L::warp_bytes(sc.P);
+  uint8_t* wbase = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P);
   uint8_t* s_prof = wbase;
   uint16_t* s_bring = reinterpret_cast<uint16_t*>(wbase + L::prof_bytes(sc.P));
-  const int M = sc.M;
-  for (int k = threadIdx.x; k < M * (M + 1); k += blockDim.x) {
-    const int a = k / (M + 1), x = k % (M + 1);
-    s_simp[k] = (x < M) ? sim.v[a * M + x] : (int8_t)SUB_PAD;
-  }
+  load_table(s_simp, sim.v, sc);
   __syncthreads();
   const long gw = (long)blockIdx.x * kWarps + wib;
   const long nw = (long)gridDim.x * kWarps;

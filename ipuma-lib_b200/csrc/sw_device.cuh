@@ -30,7 +30,8 @@
 // __shfl_up_sync.  A longer than one strip is processed strip by strip; the
 // last column of a strip is handed to the next one through per-warp global
 // scratch (a strip team, StripTeam, spreads one couple's strips over the
-// warps of a block instead).  Substitution scores come from a per-strip
+// warps of a block instead).  The 16-bit classes run tag_pass
+// (sw_tagged.cuh), the same layout with fewer ALU instructions per cell.  Substitution scores come from a per-strip
 // query profile in shared memory (int8, one row per B letter plus a
 // padding row).
 //
@@ -69,6 +70,8 @@ struct SwConst {
   int bits;     // bits per residue of the code array (8, or packed 2/4/5: code_at)
   int P;        // letters of the query profile (M, or 4 for 2-bit A/C/G/T codes)
   int pshift;   // profile row of a code: code - pshift (1 for 2-bit codes, else 0)
+  int one;      // 1, unknown to the compiler (tag_pass's multiplier)
+  unsigned gE2, gIgE2, gEp2;  // gE and gI + gE in both halfwords (tag_pass: operands from the parameter bank)
 };
 
 // Control of a hybrid pass (sw_pass with HYB): an s16x2 pass that stops
@@ -85,7 +88,7 @@ struct PassCtl {
   int stoppedAt = -1;      // out (s16x2 pass): strip it stopped before, -1: none
 };
 
-// Early stop of a reverse pass (sw_pass with EARLY): the reverse maximum of
+// Early stop of a reverse pass (tag_pass with EARLY): the reverse maximum of
 // a pair equals its forward score, so a strip may end once every pair's
 // group has reached its target and all lanes have passed that row, and a
 // later strip (larger columns) can only win with a smaller row, so it runs
@@ -139,6 +142,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 struct LaneS32 {
   using V = int;
   static constexpr int NP = 1;
+  static constexpr bool LINEAR = false;
   __device__ __forceinline__ static V splat(int x) { return x; }
   __device__ __forceinline__ static V add(V a, V b) { return a + b; }
   // max(a + b, c)
@@ -163,6 +167,7 @@ struct LaneS32 {
 struct LaneS16x2 {
   using V = uint32_t;
   static constexpr int NP = 2;
+  static constexpr bool LINEAR = false;
   __device__ __forceinline__ static V splat(int x) {
     return (uint32_t)(x & 0xffff) | ((uint32_t)(x & 0xffff) << 16);
   }
@@ -208,6 +213,7 @@ struct LaneS16x2 {
 struct LaneB16x2 {
   using V = uint32_t;
   static constexpr int NP = 2;
+  static constexpr bool LINEAR = false;
   static constexpr int BIAS = 1024;
   static constexpr int OFFSET = BIAS - 32768;  // score -> stored halfword
   __device__ __forceinline__ static V splat(int x) {  // a score
@@ -266,7 +272,7 @@ struct Cell {
     return T::addmax_relu(d, s, f);
   }
   __device__ __forceinline__ static typename T::V delta(int x) { return T::splat(x); }
-  __device__ __forceinline__ static int limit(const SwConst& sc) { return sc.s16Limit; }
+  __host__ __device__ __forceinline__ static int limit(const SwConst& sc) { return sc.s16Limit; }
 };
 template <>
 struct Cell<LaneB16x2> {
@@ -276,7 +282,7 @@ struct Cell<LaneB16x2> {
   }
   __device__ __forceinline__ static V ymax(V d, V s, V f) { return LaneB16x2::addmax(d, s, f); }
   __device__ __forceinline__ static V delta(int x) { return LaneB16x2::delta(x); }
-  __device__ __forceinline__ static int limit(const SwConst& sc) { return sc.u16Limit; }
+  __host__ __device__ __forceinline__ static int limit(const SwConst& sc) { return sc.u16Limit; }
 };
 
 // -------------------------------------------------------------------------
@@ -350,70 +356,137 @@ __device__ __forceinline__ bool better(int s1, int i1, int j1, int s2, int i2, i
 }
 
 // -------------------------------------------------------------------------
-// Query profile of one group's strip: lane l's K columns of letter x at
-// prof[x * LANES * KP + l * KP + c] = sim[A[col0 + l * K + c]][x] as int8,
-// KP = K rounded up to whole 32-bit words (bytes c >= K are unused).  The
-// profile has P + 1 rows: row x < P is letter x + pshift (2-bit A/C/G/T
-// codes need only the rows of codes 1..4), row P (the padding letter) and
-// columns past |A| hold SUB_PAD.
+// Query profile of one group's strip: K int8 values sim[A[col0 + l * K + c]][x]
+// per lane l and letter x, padded to KP = K rounded up to whole 32-bit words.
+// The profile has P + 1 rows of LANES * KP bytes: row x < P is letter x +
+// pshift (2-bit A/C/G/T codes need only the rows of codes 1..4), row P (the
+// padding letter) and columns past |A| hold SUB_PAD.
+//
+// A row is laid out in planes, so that every load of a warp is as wide as
+// the remaining bytes allow and free of bank conflicts (a lane's bytes side
+// by side would put 8 lanes of a 16-byte load 2 x on the same banks for
+// K > 16, and K = 12, 20, 28 would load 4 bytes at a time): planes of 16
+// bytes per lane, then one of 8 and one of 4.
 // -------------------------------------------------------------------------
 template <int K>
 struct ProfileWords {
   static constexpr int KP = ((K + 3) / 4) * 4;  // profile bytes per lane
   static constexpr int W = KP / 4;              // 32-bit words per lane
+  static constexpr int N16 = KP / 16;           // 16-byte planes
+  static constexpr bool HAS8 = KP % 16 >= 8, HAS4 = KP % 8 == 4;
 };
 
+// This lane's bytes of row 0 in the 16-, 8- and 4-byte planes.
 template <int K, int LANES>
-__device__ __forceinline__ void build_profile(uint8_t* prof, const int8_t* s_simp, const SwConst& sc,
-                                              const PassSeq& ps, int col0, int lane) {
-  // s_simp[a * (M + 1) + x] = sim[a][x] and SUB_PAD for x == M.
-  const int M = sc.M, P = sc.P, bits = sc.bits;
-  constexpr int KP = ProfileWords<K>::KP;
-  constexpr int SWP = LANES * KP;
-  int acode[KP];
-#pragma unroll
-  for (int c = 0; c < KP; ++c) {
-    const int col = col0 + lane * K + c;
-    acode[c] = (c < K && col < ps.alen) ? code_at(ps.base, ps.a + (long long)col * ps.da, bits) : -1;
+struct ProfilePtr {
+  using W = ProfileWords<K>;
+  static constexpr int OFF8 = W::N16 * LANES * 16, OFF4 = OFF8 + (W::HAS8 ? LANES * 8 : 0);
+  uint32_t lane;
+  // Byte offset of word w of the lane within a row.
+  __device__ __forceinline__ uint32_t word(int w) const {
+    if (w < 4 * W::N16) return (w / 4) * LANES * 16 + lane * 16 + (w % 4) * 4;
+    const int r = w - 4 * W::N16;
+    if (W::HAS8 && r < 2) return OFF8 + lane * 8 + r * 4;
+    return OFF4 + lane * 4;
   }
-  for (int x = 0; x <= P; ++x) {
-    const int xs = x < P ? x + sc.pshift : M;  // column of s_simp
+  // Loads the lane's words of the row at `row`.
+  __device__ __forceinline__ void load(uint32_t (&v)[W::W], const uint8_t* row) const {
+    if constexpr (W::N16 > 0) {
+      const uint8_t* p = row + lane * 16;
 #pragma unroll
-    for (int w = 0; w < KP / 4; ++w) {
-      uint32_t word = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int a = acode[4 * w + q];
-        const int v = (a >= 0) ? (int)s_simp[a * (M + 1) + xs] : SUB_PAD;
-        word |= ((uint32_t)(uint8_t)(int8_t)v) << (8 * q);
+      for (int q = 0; q < W::N16; ++q) {
+        const uint4 x = *reinterpret_cast<const uint4*>(p + q * LANES * 16);
+        v[4 * q + 0] = x.x;
+        v[4 * q + 1] = x.y;
+        v[4 * q + 2] = x.z;
+        v[4 * q + 3] = x.w;
       }
-      *reinterpret_cast<uint32_t*>(prof + x * SWP + lane * KP + 4 * w) = word;
+    }
+    if constexpr (W::HAS8) {
+      const uint2 x = *reinterpret_cast<const uint2*>(row + lane * 8 + OFF8);
+      v[4 * W::N16 + 0] = x.x;
+      v[4 * W::N16 + 1] = x.y;
+    }
+    if constexpr (W::HAS4) v[W::W - 1] = *reinterpret_cast<const uint32_t*>(row + lane * 4 + OFF4);
+  }
+};
+
+// Substitution table of a block in shared memory: row a (A code; row M =
+// padding column) holds the values of profile rows 0 .. P, (sim + bias) *
+// 2^shift, padded to whole words.
+struct SubTable {
+  __host__ __device__ static int stride(int P) { return (P + 1 + 3) & ~3; }
+  __host__ __device__ static int bytes(int M, int P) { return ((M + 1) * stride(P) + 15) & ~15; }
+};
+
+__device__ __forceinline__ void load_table(int8_t* s_simp, const int8_t* sim, const SwConst& sc, int bias = 0,
+                                           int shift = 0) {
+  const int st = SubTable::stride(sc.P);
+  for (int k = threadIdx.x; k < (sc.M + 1) * st; k += blockDim.x) {
+    const int a = k / st, x = k % st;
+    s_simp[k] = (a < sc.M && x < sc.P) ? (int8_t)((sim[a * sc.M + x + sc.pshift] + bias) * (1 << shift))
+                                       : (int8_t)SUB_PAD;
+  }
+}
+
+// A codes of columns col .. col + 3 of a pass (M past `end`).
+__device__ __forceinline__ void column_codes(const SwConst& sc, const PassSeq& ps, int col, int end, int (&a)[4]) {
+  const int pad = sc.M;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) a[q] = pad;
+  if (col >= end) return;
+  if (sc.bits == 8) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (col + q < end) a[q] = min((int)ps.base[ps.a + (long long)(col + q) * ps.da], pad);
+  } else {
+    // The four fields lie in the two words from the lowest one's word on
+    // (20 bits at most); a reversed pass has no field below residue 0.
+    const long long p = ps.a + (long long)col * ps.da;
+    const long long lo = ps.da > 0 ? p : (p > 3 ? p - 3 : 0);
+    const int s = (int)(p - lo);
+    const long long bit = lo * sc.bits;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(ps.base) + (bit >> 5);
+    const uint32_t v = __funnelshift_r(__ldg(w), __ldg(w + 1), (uint32_t)bit & 31u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int at = ps.da > 0 ? q : s - q;
+      if (col + q < end) {
+        const int x = (int)((v >> (at * sc.bits)) & ((1u << sc.bits) - 1u));
+        a[q] = min(sc.bits == 2 ? x + 1 : x, pad);
+      }
     }
   }
 }
 
-// Loads KB bytes (a multiple of 4) of a profile row into words.
-template <int K>
-__device__ __forceinline__ void load_profile_row(uint32_t (&w)[K / 4], const uint8_t* p) {
-  if constexpr (K % 16 == 0) {
+// Builds the profile of the strip starting at col0: four columns by four
+// letters at a time, each a byte transpose of four table words.
+template <int K, int LANES>
+__device__ __forceinline__ void build_profile(uint8_t* prof, const int8_t* s_simp, const SwConst& sc,
+                                              const PassSeq& ps, int col0, int lane) {
+  constexpr int KP = ProfileWords<K>::KP;
+  constexpr int SWP = LANES * KP;
+  const int P = sc.P, st = SubTable::stride(P);
+  const ProfilePtr<K, LANES> pp{(uint32_t)lane};
+  const int first = col0 + lane * K, end = min(ps.alen, first + K);
 #pragma unroll
-    for (int q = 0; q < K / 16; ++q) {
-      uint4 v = reinterpret_cast<const uint4*>(p)[q];
-      w[4 * q + 0] = v.x;
-      w[4 * q + 1] = v.y;
-      w[4 * q + 2] = v.z;
-      w[4 * q + 3] = v.w;
+  for (int w = 0; w < KP / 4; ++w) {
+    int a[4];
+    column_codes(sc, ps, first + 4 * w, end, a);
+    const int8_t *t0 = s_simp + a[0] * st, *t1 = s_simp + a[1] * st, *t2 = s_simp + a[2] * st,
+                 *t3 = s_simp + a[3] * st;
+    uint8_t* dst = prof + pp.word(w);
+    for (int x = 0; x <= P; x += 4) {
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(t0 + x), w1 = *reinterpret_cast<const uint32_t*>(t1 + x);
+      const uint32_t w2 = *reinterpret_cast<const uint32_t*>(t2 + x), w3 = *reinterpret_cast<const uint32_t*>(t3 + x);
+      const uint32_t u0 = prmt(w0, w1, 0x5140), u1 = prmt(w2, w3, 0x5140);
+      const uint32_t u2 = prmt(w0, w1, 0x7362), u3 = prmt(w2, w3, 0x7362);
+      uint8_t* d = dst + x * SWP;
+      *reinterpret_cast<uint32_t*>(d) = prmt(u0, u1, 0x5410);
+      if (x + 1 <= P) *reinterpret_cast<uint32_t*>(d + SWP) = prmt(u0, u1, 0x7632);
+      if (x + 2 <= P) *reinterpret_cast<uint32_t*>(d + 2 * SWP) = prmt(u2, u3, 0x5410);
+      if (x + 3 <= P) *reinterpret_cast<uint32_t*>(d + 3 * SWP) = prmt(u2, u3, 0x7632);
     }
-  } else if constexpr (K % 8 == 0) {
-#pragma unroll
-    for (int q = 0; q < K / 8; ++q) {
-      uint2 v = reinterpret_cast<const uint2*>(p)[q];
-      w[2 * q + 0] = v.x;
-      w[2 * q + 1] = v.y;
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < K / 4; ++q) w[q] = reinterpret_cast<const uint32_t*>(p)[q];
   }
 }
 
@@ -493,7 +566,7 @@ __device__ __forceinline__ typename T::V raise_to_group(typename T::V best) {
 // the warp's pairs in s32 lanes.
 //
 //   s_prof   : this group's profile area, NP * (P + 1) * LANES * KP bytes
-//   s_simp   : substitution table with the padding column (build_profile)
+//   s_simp   : substitution table (load_table)
 //   s_bring  : this group's rings of B letters, 64 entries per pair stored
 //              twice (pair h at s_bring + 128 h, entry e also at e + 64, so
 //              a block of steps reads base + k without wrapping), each the
@@ -507,12 +580,10 @@ __device__ __forceinline__ typename T::V raise_to_group(typename T::V best) {
 // it; an s32 pass with ctl->strip0 > 0 starts there from the packed
 // boundary half ctl->bndHalf in buffer ctl->scrBase, keeping `out` (the
 // best of the strips before) and using the two other buffers.
-template <class T, int K, int LANES, bool HYB = false, bool EARLY = false, bool TEAM = false>
+template <class T, int K, int LANES, bool HYB = false>
 __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, const int8_t* s_simp,
                                         uint16_t* s_bring, const PassSeq (&ps)[T::NP], int2* scr,
-                                        long rowsCap, Best (&out)[T::NP], PassCtl* ctl = nullptr,
-                                        PassStop stop = PassStop{}, StripTeam team = StripTeam{}) {
-  static_assert(!TEAM || (LANES == 32 && !HYB && !EARLY), "strip teams run whole-warp passes without an early stop");
+                                        long rowsCap, Best (&out)[T::NP], PassCtl* ctl = nullptr) {
   using V = typename T::V;
   constexpr int SW = LANES * K;          // columns per strip
   constexpr int KP = ProfileWords<K>::KP;
@@ -521,8 +592,8 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
   const int lane = threadIdx.x & (LANES - 1);
   const int P = sc.P;
   const int profStride = (P + 1) * SWP;
-  const uint8_t* profP = s_prof + lane * KP;  // this lane's columns of pair P's profile
-  const uint8_t* profQ = profP + profStride;  // ... and of pair Q's
+  const ProfilePtr<K, LANES> prof{(uint32_t)lane};
+  const uint8_t* profQ = s_prof + profStride;  // pair Q's profile
 
   const int strip0 = HYB ? ctl->strip0 : 0;
   int rowsG = 0, amax = 0;
@@ -539,12 +610,6 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
   int rowsW = __reduce_max_sync(FULL, rowsG);
   int rowsMin = __reduce_min_sync(FULL, rowsG);
   const int nstrips = (__reduce_max_sync(FULL, amax) + SW - 1) / SW;
-  // EARLY: rows each pair still needs (its best row once it reached its
-  // target), and this lane's group in the warp.
-  int capRows[NP];
-#pragma unroll
-  for (int h = 0; h < NP; ++h) capRows[h] = ps[h].blen;
-  const unsigned gmask = (LANES == 32) ? FULL : (((1u << LANES) - 1u) << (threadIdx.x & (32 - LANES)));
   using C = Cell<T>;
   const V vgE = C::delta(sc.gE);
   const V vgEp = C::delta(max(sc.gE, sc.gIgE));
@@ -565,7 +630,6 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
   // Scratch buffer written by strip s: 0/1 alternating, or for an s32
   // continuation the two buffers other than the one holding its input.
   auto wbuf = [&](int sidx) -> int {
-    if constexpr (TEAM) return sidx % team.warps;
     if (!HYB || strip0 == 0) return sidx & 1;
     return (ctl->scrBase + 1 + ((sidx - strip0) & 1)) % 3;
   };
@@ -573,58 +637,7 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
   // the bound of the next strip.
   V bmax = vZero;
 
-  // TEAM: marks the team as given up (overflow, or a wait that ran out).
-  auto team_fail = [&]() {
-    if constexpr (TEAM) {
-      if (lane == 0) *(volatile int*)team.abort = 1;
-    }
-  };
-  // TEAM: waits until the previous warp published `need` rows of strip
-  // s's boundary.  Warp-uniform result; false once the team gave up.
-  auto team_wait = [&](int s, int need) -> bool {
-    bool ok = true;
-    if constexpr (TEAM) {
-      const int target = (s << 16) | need;
-      const volatile int* pr = team.prog + (team.warp + team.warps - 1) % team.warps;
-      const volatile int* ab = team.abort;
-      unsigned long long t_start = 0;
-      for (int it = 0; *pr < target; ++it) {
-        if (*ab != 0) {
-          ok = false;
-          break;
-        }
-        if ((it & 255) == 0) {
-          const unsigned long long now = global_ns();
-          if (it == 0) t_start = now;
-          if (now - t_start > kTeamWaitNs || it >= (1 << 26)) {
-            atomicCAS(team.err, 0, team.errCode);
-            *(volatile int*)team.abort = 1;
-            ok = false;
-            break;
-          }
-        }
-        __nanosleep(64);
-      }
-      __threadfence_block();  // the boundary rows are read after the flag
-      ok = __all_sync(FULL, ok);
-    }
-    return ok;
-  };
-  bool teamGaveUp = false;
-
-  const int stripFirst = strip0 + (TEAM ? team.warp : 0);
-  const int stripStep = TEAM ? team.warps : 1;
-  for (int strip = stripFirst; strip < nstrips; strip += stripStep) {
-    if constexpr (EARLY) {
-      if (stop.on && strip > strip0) {
-        rowsG = 0;
-#pragma unroll
-        for (int h = 0; h < NP; ++h) rowsG = max(rowsG, min(ps[h].blen, capRows[h]));
-        rowsW = __reduce_max_sync(FULL, rowsG);
-        rowsMin = __reduce_min_sync(FULL, rowsG);
-        if (rowsW == 0) break;  // caps only shrink: no later strip can win
-      }
-    }
+  for (int strip = strip0; strip < nstrips; ++strip) {
     const int col0 = strip * SW;
     const bool hasIn = strip > 0;
     const bool hasOut = strip + 1 < nstrips;
@@ -677,12 +690,6 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
     // Boundary (Y, Ê) of the previous strip's last column: lane k of the
     // group's chunk registers holds row (chunkBase + k).
     int2 chunk = make_int2(0, 0), chunkNext = make_int2(0, 0);
-    if constexpr (TEAM) {
-      if (hasIn && !team_wait(strip - 1, min(2 * LANES, rowsG))) {
-        teamGaveUp = true;
-        break;
-      }
-    }
     if (hasIn) {
       if (lane < rowsG) chunk = bnd(lane);
       if (LANES + lane < rowsG) chunkNext = bnd(LANES + lane);
@@ -729,9 +736,9 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
       if (!decltype(check)::value || (i >= 0 && i < rowsG)) {
         uint32_t wp[KP / 4], wq[KP / 4];
         const int slot = ringBase + k;  // (i mod 64), < 64 + LANES
-        load_profile_row<KP>(wp, profP + s_bring[slot]);
+        prof.load(wp, s_prof + s_bring[slot]);
         if constexpr (NP == 2) {
-          load_profile_row<KP>(wq, profQ + s_bring[128 + slot]);
+          prof.load(wq, profQ + s_bring[128 + slot]);
         } else {
 #pragma unroll
           for (int q = 0; q < KP / 4; ++q) wq[q] = 0;
@@ -792,23 +799,7 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
 
     const int nsteps = rowsW + LANES - 1;
     bool gaveUp = false;
-    int stopAt = nsteps;  // EARLY: end of the block after every pair is done
     for (int t0 = 0; t0 < nsteps; t0 += LANES) {
-      if constexpr (EARLY) {
-        if (t0 >= stopAt) break;
-        if (stop.on && stopAt == nsteps) {
-          // A pair is done once its group reached the target (before t0, so
-          // the slowest lane passes that row within this block) or all
-          // lanes are past its rows.  Warp-uniform.
-          bool done = true;
-#pragma unroll
-          for (int h = 0; h < NP; ++h) {
-            const bool found = (__ballot_sync(FULL, T::half(best, h) >= stop.target[h]) & gmask) != 0;
-            done = done && (found || t0 - (LANES - 1) >= min(ps[h].blen, capRows[h]));
-          }
-          if (__all_sync(FULL, done)) stopAt = t0 + LANES;
-        }
-      }
       if constexpr (NP == 2) {
         if ((t0 & 31) == 0) {
           // A cell above s16Limit could overflow the next additions.
@@ -817,13 +808,6 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
             gaveUp = true;
             break;
           }
-        }
-      }
-      if constexpr (TEAM) {
-        // Another warp gave up: this pass's results are not used.
-        if (__any_sync(FULL, *(volatile int*)team.abort != 0)) {
-          teamGaveUp = true;
-          break;
         }
       }
       if (t0 > 0) best = raise_to_group<T, LANES>(best);
@@ -836,12 +820,6 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
       bnext = fetch_letters(t0 + LANES + lane);
       __syncwarp();
       if (hasIn && t0 > 0) {
-        if constexpr (TEAM) {
-          if (!team_wait(strip - 1, min(t0 + 2 * LANES, rowsG))) {
-            teamGaveUp = true;
-            break;
-          }
-        }
         chunk = chunkNext;
         const int r = t0 + LANES + lane;
         chunkNext = (r < rowsG) ? bnd(r) : make_int2(0, 0);
@@ -853,25 +831,11 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
 #pragma unroll 1
         for (int k = 0; k < LANES; ++k) step(t0 + k, k, std::true_type{});
       }
-      if constexpr (TEAM) {
-        // Lane LANES - 1 wrote the boundary rows up to t0 (those below
-        // rowsG): release them to the next strip's warp.
-        if (hasOut && lane == LANES - 1) {
-          __threadfence_block();
-          *(volatile int*)(team.prog + team.warp) = (strip << 16) | min(t0 + 1, rowsG);
-        }
-      }
-    }
-    if constexpr (TEAM) {
-      if (teamGaveUp) break;
     }
 
     if constexpr (NP == 2) {
       if (!gaveUp) gaveUp = __any_sync(FULL, T::half(best, 0) > lim || T::half(best, 1) > lim);
-      if (gaveUp) {
-        team_fail();
-        return false;
-      }
+      if (gaveUp) return false;
     }
     // Strip result: first column of the lane's snapshot that holds its best.
 #pragma unroll
@@ -895,17 +859,11 @@ __device__ __forceinline__ bool sw_pass(const SwConst& sc, uint8_t* s_prof, cons
         out[h].i = ii;
         out[h].j = j;
       }
-      if constexpr (EARLY) {
-        if (stop.on && out[h].s >= stop.target[h]) capRows[h] = min(capRows[h], out[h].i);
-      }
     }
     if (hasOut) {
       __threadfence_block();
       __syncwarp();
     }
-  }
-  if constexpr (TEAM) {
-    if (teamGaveUp) return false;
   }
   return true;
 }

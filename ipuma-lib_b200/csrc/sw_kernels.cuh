@@ -28,6 +28,7 @@
 //                     offsets and class shares), k_bin_scatter (the list).
 #pragma once
 #include "sw_device.cuh"
+#include "sw_tagged.cuh"
 
 namespace ipuma_dev {
 
@@ -98,22 +99,36 @@ struct SmemLayout {
   static constexpr int SW = LANES * K;
   static constexpr int GROUPS = 32 / LANES;
   // M = alphabet size (substitution table), P = letters of the profile.
-  __host__ __device__ static int simp_bytes(int M) { return ((M * (M + 1)) + 15) & ~15; }
+  __host__ __device__ static int simp_bytes(int M, int P) { return SubTable::bytes(M, P); }
   __host__ __device__ static int prof_bytes(int P) { return T::NP * (P + 1) * LANES * ProfileWords<K>::KP; }
   __host__ __device__ static int ring_bytes() { return 128 * 2 * T::NP; }  // a doubled uint16 ring per pair
   __host__ __device__ static int group_bytes(int P) { return (prof_bytes(P) + ring_bytes() + 15) & ~15; }
   __host__ __device__ static int warp_bytes(int P) { return GROUPS * group_bytes(P); }
-  __host__ __device__ static int total(int M, int P, int warps) { return simp_bytes(M) + warps * warp_bytes(P); }
+  __host__ __device__ static int total(int M, int P, int warps) { return simp_bytes(M, P) + warps * warp_bytes(P); }
 };
 
-// Loads the substitution table with its padding column: simp[a][x] =
-// sim[a][x] for x < M, SUB_PAD for x == M.
-__device__ __forceinline__ void load_simp(int8_t* s_simp, const int8_t* sim, const SwConst& sc) {
-  const int M = sc.M;
-  for (int k = threadIdx.x; k < M * (M + 1); k += blockDim.x) {
-    const int a = k / (M + 1), x = k % (M + 1);
-    s_simp[k] = (x < M) ? sim[a * M + x] : (int8_t)SUB_PAD;
-  }
+// One pass of a lane type: tagged 16-bit lanes or sw_pass's lanes.
+template <class T>
+constexpr bool kTagged = false;
+template <int TB, bool LIN, bool SCALED>
+constexpr bool kTagged<LaneTag<TB, LIN, SCALED>> = true;
+template <>
+constexpr bool kTagged<LaneBig> = true;
+// Bias (-gE for linear gaps) and scale of a lane type's profile values.
+template <class T>
+constexpr bool kProfBias = T::LINEAR;
+template <class T>
+constexpr int kProfShift = 0;
+template <int TB, bool LIN, bool SCALED>
+constexpr int kProfShift<LaneTag<TB, LIN, SCALED>> = SCALED ? TB : 0;
+template <class T, int K, int LANES, bool EARLY = false>
+__device__ __forceinline__ bool one_pass(const SwConst& sc, uint8_t* s_prof, const int8_t* s_simp, uint16_t* s_bring,
+                                         const PassSeq (&ps)[T::NP], int2* scr, long rowsCap, Best (&out)[T::NP],
+                                         PassStop stop = PassStop{}) {
+  if constexpr (kTagged<T>)
+    return tag_pass<T, K, LANES, EARLY>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, out, stop);
+  else
+    return sw_pass<T, K, LANES>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, out);
 }
 
 // Forward pass (+ reverse pass unless forwardOnly) for the NP pairs held
@@ -141,7 +156,7 @@ __device__ __forceinline__ void align_pairs(const SwConst& sc, uint8_t* s_prof,
   for (int h = 0; h < NP; ++h) rv[h] = Best{0, 0, 0};
   if (MODE == 1 || (MODE == 0 && sc.forwardOnly)) {
     if constexpr (MODE != 2) {
-      const bool done = sw_pass<T, K, LANES>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, fw);
+      const bool done = one_pass<T, K, LANES>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, fw);
 #pragma unroll
       for (int h = 0; h < NP; ++h) ovf[h] = (NP == 2) && (!done || fw[h].s > Cell<T>::limit(sc));
     }
@@ -158,8 +173,7 @@ __device__ __forceinline__ void align_pairs(const SwConst& sc, uint8_t* s_prof,
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     Best res[NP];
-    const bool done = sw_pass<T, K, LANES, false, MODE == 2>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, res,
-                                                              nullptr, stop);
+    const bool done = one_pass<T, K, LANES, MODE == 2>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, res, stop);
     if (pass == 1) {
 #pragma unroll
       for (int h = 0; h < NP; ++h) rv[h] = res[h];
@@ -303,10 +317,10 @@ __global__ void __launch_bounds__(128, (FWD && !HYB) ? 4 : 3) k_batched(SwConst 
   const int group = lane32 / LANES;
   const int glane = lane32 & (LANES - 1);
   int8_t* s_simp = reinterpret_cast<int8_t*>(smem);
-  uint8_t* gbase = smem + L::simp_bytes(sc.M) + wib * L::warp_bytes(sc.P) + group * L::group_bytes(sc.P);
+  uint8_t* gbase = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P) + group * L::group_bytes(sc.P);
   uint8_t* s_prof = gbase;
   uint16_t* s_bring = reinterpret_cast<uint16_t*>(gbase + L::prof_bytes(sc.P));
-  load_simp(s_simp, sim, sc);
+  load_table(s_simp, sim, sc, kProfBias<T> ? -sc.gE : 0, kProfShift<T>);
   __syncthreads();
 
   // range = {first list entry, number of entries}, written by the binning
@@ -377,7 +391,7 @@ __global__ void __launch_bounds__(128, (FWD && !HYB) ? 4 : 3) k_batched(SwConst 
 
 // Strip-team kernel: the blockDim.x / 32 warps of a block align one item
 // (the two pairs of a 32-lane s16x2 group), taking its 32 * K wide strips
-// round robin (sw_pass with TEAM), so a long pair finishes up to `warps`
+// round robin (tag_pass with TEAM), so a long pair finishes up to `warps`
 // times sooner than on one warp.  Each warp keeps the best cell of its own
 // strips; the block merges them with the first-strict-maximum order
 // (better), the order-independent total order the one-warp pass applies
@@ -386,7 +400,7 @@ __global__ void __launch_bounds__(128, (FWD && !HYB) ? 4 : 3) k_batched(SwConst 
 // past kTeamWaitNs, which also sets ERR_WAIT) sends both pairs to the s32
 // rerun.  Block scratch: `warps` boundary columns of rowsCap rows.
 constexpr int kTeamMaxWarps = 8;
-template <int K>
+template <class T, int K>
 __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __restrict__ sim,
                                                    const uint8_t* __restrict__ codes,
                                                    const PairDesc* __restrict__ pairs,
@@ -399,7 +413,6 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
   if ((int)blockIdx.x >= allot->blocks) return;
   scratch += allot->base;
   if (trace && threadIdx.x == 0) atomicMax(&trace[0], ~global_ns());
-  using T = LaneS16x2;
   using L = SmemLayout<T, K, 32>;
   constexpr int NP = 2;
   extern __shared__ __align__(16) uint8_t smem[];
@@ -412,9 +425,9 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int8_t* s_simp = reinterpret_cast<int8_t*>(smem);
-  uint8_t* s_prof = smem + L::simp_bytes(sc.M) + wib * L::warp_bytes(sc.P);
+  uint8_t* s_prof = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P);
   uint16_t* s_bring = reinterpret_cast<uint16_t*>(s_prof + L::prof_bytes(sc.P));
-  load_simp(s_simp, sim, sc);
+  load_table(s_simp, sim, sc, kProfBias<T> ? -sc.gE : 0, kProfShift<T>);
 
   const int n = range[1];
   list += range[0];
@@ -459,8 +472,7 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
       Best out[NP];
-      sw_pass<T, K, 32, false, false, true>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, out, nullptr,
-                                            PassStop{}, team);
+      tag_pass<T, K, 32, false, true>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, out, PassStop{}, team);
       if (lane == 0) {
 #pragma unroll
         for (int h = 0; h < NP; ++h) s_res[wib][h] = out[h];
@@ -534,10 +546,10 @@ __global__ void __launch_bounds__(128) k_plain(SwConst sc, const int8_t* __restr
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int8_t* s_simp = reinterpret_cast<int8_t*>(smem);
-  uint8_t* wbase = smem + L::simp_bytes(sc.M) + wib * L::warp_bytes(sc.P);
+  uint8_t* wbase = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P);
   uint8_t* s_prof = wbase;
   uint16_t* s_bring = reinterpret_cast<uint16_t*>(wbase + L::prof_bytes(sc.P));
-  load_simp(s_simp, sim, sc);
+  load_table(s_simp, sim, sc);
   __syncthreads();
   const long gw = (long)blockIdx.x * warps + wib;
   const long nw = (long)gridDim.x * warps;
@@ -583,10 +595,10 @@ __global__ void __launch_bounds__(128) k_plain16(SwConst sc, const int8_t* __res
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int8_t* s_simp = reinterpret_cast<int8_t*>(smem);
-  uint8_t* wbase = smem + L::simp_bytes(sc.M) + wib * L::warp_bytes(sc.P);
+  uint8_t* wbase = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P);
   uint8_t* s_prof = wbase;  // the s32 redo uses the first half of it
   uint16_t* s_bring = reinterpret_cast<uint16_t*>(wbase + L::prof_bytes(sc.P));
-  load_simp(s_simp, sim, sc);
+  load_table(s_simp, sim, sc);
   __syncthreads();
   const long gw = (long)blockIdx.x * warps + wib;
   const long nw = (long)gridDim.x * warps;
@@ -711,7 +723,7 @@ static __global__ void k_exact(SwConst sc, const int8_t* __restrict__ sim, const
 constexpr int NROWB = 256;    // row buckets (16 per power of two)
 constexpr int NSTRIPB = 16;   // strip-count buckets
 constexpr int NBUCKET = NROWB * NSTRIPB;
-constexpr int NCLASS_MAX = 24;
+constexpr int NCLASS_MAX = 25;
 
 // Log-linear bucket of |B| (16 sub-buckets per power of two): pairs that
 // share a bucket differ by at most 1/16 in rows, so the groups of a warp
@@ -727,8 +739,12 @@ struct BinParams {
   int cls_s32;             // class index of the exact-32-bit kernel
   int cls_hi;              // class of pairs the diagonal bound sends to 32 bits:
                            // the hybrid class (or cls_s32 when it is off)
-  int s16_max_len;         // min(|A|,|B|) above which s16x2 could overflow
-  int s16_limit;           // scores above this need s32 lanes
+  int s16_max_len;         // min(|A|,|B|) above which the 16-bit lanes could overflow
+  int s16_limit;           // scores above this need more than the long class's 16 bits
+  // Longest min(|A|,|B|) a class is chosen for by cost: a typical identical
+  // pair of that length still fits the scores its lanes hold (a pair that
+  // does not is rerun in s32 lanes).
+  int fit[NCLASS_MAX];
   int lanes[NCLASS_MAX];   // lanes per group of each class
   int width[NCLASS_MAX];   // strip width (lanes * K) of each class
   float slot_ps[NCLASS_MAX];   // time per cell slot of a strip (autotuned)
@@ -743,8 +759,9 @@ struct BinParams {
   float batch_ps_per_cell;
   float lat_share;
   float lat_min_ps;
-  int long_a;                  // |A| above which the widest class is used
-  int widest;                  // that class
+  int long_a;                  // |A| above which the widest strips are used
+  int widest;                  // class of the widest strips
+  int cls_long;                // the same strips with room for the longest scores (past fit[widest])
   int forced_class;        // >= 0: every s16x2 pair goes to this class
   int team_cls;            // strip-team class (-1: none in this batch)
   int team_warps;          // warps per team
@@ -840,9 +857,10 @@ static __device__ int warp_diagonal_bound(const uint8_t* codes, int bits, long l
   return __shfl_sync(FULL, r.best, 0);
 }
 
-// Steps a team warp starts behind the warp before it: it reads boundary
-// rows two blocks of 32 ahead, which that warp publishes a block later.
-constexpr float kTeamLagSteps = 96.f;
+// Steps a team warp starts behind the warp before it: it reads the boundary
+// rows of a block of 32 when it starts the block, and that warp publishes
+// them a block later.
+constexpr float kTeamLagSteps = 64.f;
 // Share of the batch's modelled time above which a pair's one-warp latency
 // sends it to a strip team (measured on B200: a 500,000-pair heavy-tailed
 // protein batch, whose 8,000-residue pairs take about a third of its time
@@ -868,22 +886,24 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
   } else {
     const float batch_ps = bp.total_cells ? (float)(*bp.total_cells) * bp.batch_ps_per_cell : 0.f;
     float bestLat = -1.f;  // one-warp latency of the class picked below
+    const int fit = min(alen, blen);
+    const int wide = fit <= bp.fit[bp.widest] ? bp.widest : bp.cls_long;
     if (alen > bp.long_a) {
       // Very long pairs are few and each keeps one warp busy for long: their
       // latency, not throughput, sets the end of the launch, and the widest
       // strips finish a pair in the fewest steps.
-      cls = bp.widest;
+      cls = wide;
       bestLat = (float)((alen + bp.width[cls] - 1) / bp.width[cls]) * (float)(blen + bp.lanes[cls]) *
                 bp.step_ps[cls];
     } else {
-      cls = 0;
+      cls = wide;
       float bestCost = -1.f;
-      int latCls = 0;
+      int latCls = wide;
       const bool thr_ok = bp.thr_on && blen <= bp.thr_max_rows && (float)alen * (float)blen <= thr_cap;
       const float lat_cap = batch_ps >= bp.lat_min_ps ? bp.lat_share * batch_ps : 3.0e38f;
       for (int c = 0; c < bp.n_s16_classes; ++c) {
         if (!((bp.enabled >> c) & 1u)) continue;
-        if (c == bp.thr_cls && !thr_ok) continue;
+        if ((c == bp.thr_cls && !thr_ok) || fit > bp.fit[c]) continue;
         const int strips = (alen + bp.width[c] - 1) / bp.width[c];
         const float lat = (float)strips * (float)(blen + bp.lanes[c]) * bp.step_ps[c];
         if (bestLat < 0.f || lat < bestLat) {
@@ -898,7 +918,10 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
           cls = c;
         }
       }
-      if (bestCost < 0.f) {
+      if (bestLat < 0.f) {  // no class holds its scores but the long one
+        bestLat = (float)((alen + bp.width[cls] - 1) / bp.width[cls]) * (float)(blen + bp.lanes[cls]) *
+                  bp.step_ps[cls];
+      } else if (bestCost < 0.f) {
         cls = latCls;  // every class is too slow: the fastest
       } else {
         bestLat = 0.f;  // a class keeps the pair under the latency cap

@@ -42,6 +42,41 @@ struct ThreadSmem {
   __host__ __device__ static int total(int M, int warps) { return simp_bytes(M) + warps * warp_bytes(M); }
 };
 
+// Loads the substitution table with its padding column: simp[a][x] =
+// sim[a][x] for x < M, SUB_PAD for x == M.
+__device__ __forceinline__ void load_simp(int8_t* s_simp, const int8_t* sim, const SwConst& sc) {
+  const int M = sc.M;
+  for (int k = threadIdx.x; k < M * (M + 1); k += blockDim.x) {
+    const int a = k / (M + 1), x = k % (M + 1);
+    s_simp[k] = (x < M) ? sim[a * M + x] : (int8_t)SUB_PAD;
+  }
+}
+
+// Loads KB bytes (a multiple of 4) of a profile row into words.
+template <int K>
+__device__ __forceinline__ void load_profile_row(uint32_t (&w)[K / 4], const uint8_t* p) {
+  if constexpr (K % 16 == 0) {
+#pragma unroll
+    for (int q = 0; q < K / 16; ++q) {
+      uint4 v = reinterpret_cast<const uint4*>(p)[q];
+      w[4 * q + 0] = v.x;
+      w[4 * q + 1] = v.y;
+      w[4 * q + 2] = v.z;
+      w[4 * q + 3] = v.w;
+    }
+  } else if constexpr (K % 8 == 0) {
+#pragma unroll
+    for (int q = 0; q < K / 8; ++q) {
+      uint2 v = reinterpret_cast<const uint2*>(p)[q];
+      w[2 * q + 0] = v.x;
+      w[2 * q + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) w[q] = reinterpret_cast<const uint32_t*>(p)[q];
+  }
+}
+
 // Builds this thread's profile slice for the strip starting at col0.
 template <int K>
 __device__ __forceinline__ void thread_profile(uint8_t* s_warp, const int8_t* s_simp, int M,
