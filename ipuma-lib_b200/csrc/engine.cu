@@ -97,7 +97,7 @@ struct ClassDef {
   int lanes, k, kind, width;
 };
 constexpr int kNumS16 = 21;     // s16x2 classes chosen by cost
-constexpr int kNumClasses = kNumS16 + 4;  // + the s32, hybrid, strip-team and long classes
+constexpr int kNumClasses = kNumS16 + 6;  // + the s32, hybrid, strip-team, long, big and big strip-team classes
 constexpr ClassDef kClasses[kNumClasses] = {
     {16, 4, IPUMA_KERNEL_S16_L16_K4, 64},    {16, 8, IPUMA_KERNEL_S16_L16_K8, 128},
     {16, 12, IPUMA_KERNEL_S16_L16_K12, 192}, {16, 16, IPUMA_KERNEL_S16_L16_K16, 256},
@@ -112,14 +112,16 @@ constexpr ClassDef kClasses[kNumClasses] = {
     {8, 16, IPUMA_KERNEL_S16_L8_K16, 128},
     {32, 16, IPUMA_KERNEL_S32_K16, 512},     {32, 16, IPUMA_KERNEL_S16_HYBRID, 512},
     {32, 16, IPUMA_KERNEL_S16_TEAM, 512},    {32, 16, IPUMA_KERNEL_S16_L32_K16, 512},
+    {32, 16, IPUMA_KERNEL_S16_HYBRID, 512},  {32, 16, IPUMA_KERNEL_S16_TEAM, 512},
 };
 static_assert(kNumClasses <= NCLASS_MAX, "class tables");
 constexpr int kClsWidest = 5;  // widest wavefront class (very long |A|)
 constexpr int kMaxTimed = IPUMA_MAX_TIMED;  // launches timed per call (time_launches)
 constexpr int kClsThread = 6;  // per-thread class k_thread<16>
 constexpr int kClsS32 = kNumS16;
-// Hybrid class: pairs whose score can pass int16 (main-diagonal bound) run
-// their safe strips in s16x2 and the rest in s32 (option "hybrid").
+// Hybrid class: pairs whose score passes the big class's (main-diagonal
+// bound) run their safe strips in biased halves and the rest in s32 (option
+// "hybrid", which also turns the big class on).
 constexpr int kClsHi = kNumS16 + 1;
 // Strip-team class (k_strips<16>): the warps of a block share one item's
 // 512-column strips, so a long pair finishes up to `warps` times sooner.
@@ -131,6 +133,11 @@ constexpr int kTeamWarpsDefault = 8;
 // Long class: the widest strips with one tag bit, for pairs whose score may
 // pass what class kClsWidest holds (BinParams::fit).
 constexpr int kClsLong = kNumS16 + 3;
+// Big class: pairs whose main diagonal passes the long class's scores, in
+// biased halves (LaneBig, scores up to 64,000); and its strip teams.  Pairs
+// whose diagonal passes even that go to the hybrid class.
+constexpr int kClsBig = kNumS16 + 4;
+constexpr int kClsBigTeam = kNumS16 + 5;
 // Per-thread class: rows it accepts (its boundary scratch is rows x threads)
 // and the share of the batch's time one of its pairs may take.
 constexpr int kThrMaxRows = 2048;
@@ -158,8 +165,8 @@ constexpr int kFineClassMinPairs = 150000;
 // 8-lane groups of linear-gap strips (strip_ref) from this many pairs: an
 // item holds eight pairs instead of four, which leaves warps without work
 // in smaller batches (10,000 pairs of 150 x 150-300 on B200: 329 us with 8
-// lanes, 290 with 16).
-constexpr int kEightLaneMinPairs = 48000;
+// lanes, 250 with 16; 69,000 of 100-200 x 100-200: 1.07 against 0.91 ms).
+constexpr int kEightLaneMinPairs = 150000;
 constexpr unsigned kCoarseClasses = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 5);
 // 8-lane groups for the five narrowest strip widths (64 to 128 columns):
 // twice the columns per lane over a wavefront half as deep, so the per-step
@@ -251,6 +258,7 @@ struct ipuma_engine {
   std::string tune_source = "defaults";
 
   // per-launch timing of the current call (time_launches)
+  int* h_ctl = nullptr;  // pinned copy of the control blocks' cleared parts (check_status)
   cudaEvent_t tev[2 * kMaxTimed] = {};
   int n_timed = 0;
   int timed_kind[kMaxTimed] = {};
@@ -303,19 +311,24 @@ constexpr int CTL_STATUS = 0;                       // DevStatus (4 ints)
 constexpr int CTL_RANGES = 4;                       // 2 * NCLASS_MAX
 constexpr int CTL_HEADS = CTL_RANGES + 2 * NCLASS_MAX;  // NCLASS_MAX + 1
 constexpr int CTL_INFO = CTL_HEADS + NCLASS_MAX + 1;    // wire check {maxA, maxB, bad} (+1 pad)
-constexpr int CTL_CELLS = ((CTL_INFO + 4) + 1) & ~1;    // 8-byte aligned: NCELLS uint64
-constexpr int NCELLS = NCLASS_MAX + 3;              // per class, rerun, wire check, batch total
-constexpr int CTL_COST = CTL_CELLS + 2 * NCELLS;    // modelled cost per class (uint64, ps)
-constexpr int CTL_ALLOT = CTL_COST + 2 * NCLASS_MAX;  // ClassAllot per class + rerun (4 ints each)
-static_assert(CTL_COST % 2 == 0 && CTL_ALLOT % 2 == 0, "8-byte aligned control block fields");
+constexpr int CTL_SUMS = ((CTL_INFO + 4) + 1) & ~1;     // ClassSums per class (8-byte aligned)
+constexpr int kSumInts = sizeof(ClassSums) / sizeof(int);
+constexpr int CTL_CELLS = CTL_SUMS + kSumInts * NCLASS_MAX;  // cells of the rerun, wire check, batch (uint64)
+constexpr int CELLS_RERUN = 0;                      // index of the rerun cells
+constexpr int CELLS_WIRE = 1;                       // cells found by the wire check
+constexpr int CELLS_TOTAL = 2;                      // cells of the batch (k_bin_total)
+constexpr int NCELLS = 3;
+constexpr int CTL_ALLOT = CTL_CELLS + 2 * NCELLS;   // ClassAllot per class + rerun (4 ints each)
 constexpr int CTL_TRACE = CTL_ALLOT + 4 * (NCLASS_MAX + 1);  // {~start, end} ns per class + rerun (uint64)
-static_assert(CTL_TRACE % 2 == 0, "8-byte aligned trace");
-constexpr int CTL_HIST = CTL_TRACE + 4 * (NCLASS_MAX + 1);  // NCLASS_MAX * NBUCKET
+static_assert(CTL_CELLS % 2 == 0 && CTL_ALLOT % 2 == 0 && CTL_TRACE % 2 == 0, "8-byte aligned control block fields");
+constexpr int CTL_CLEAR = CTL_TRACE + 4 * (NCLASS_MAX + 1);  // cleared before every run, up to here
+constexpr int CTL_HIST = (CTL_CLEAR + 3) & ~3;      // NCLASS_MAX * NBUCKET (cleared by k_bin_total)
 constexpr int CTL_OFFS = CTL_HIST + NCLASS_MAX * NBUCKET;
 constexpr int CTL_INTS = CTL_OFFS + NCLASS_MAX * NBUCKET;
-constexpr int CELLS_RERUN = NCLASS_MAX;             // index of the rerun cells
-constexpr int CELLS_WIRE = NCLASS_MAX + 1;          // cells found by the wire check
-constexpr int CELLS_TOTAL = NCLASS_MAX + 2;         // cells of the batch (k_bin_total)
+static_assert(CTL_HIST % 4 == 0 && CTL_INTS % 4 == 0, "16-byte aligned histogram");
+// Index of a launch's cells in the engine's timing tables: its class, or
+// past the classes a field of CTL_CELLS.
+constexpr int kTimedRerun = NCLASS_MAX + CELLS_RERUN, kTimedWire = NCLASS_MAX + CELLS_WIRE;
 
 // A kernel's dynamic shared memory limit is one process-wide attribute per
 // device, shared by every engine: engines with different alphabets need
@@ -452,6 +465,7 @@ KernelRef kernel_of(const ipuma_engine* e, int cls, int P, bool eight) {
     case kClsLong:
       return e->cells == ipuma_engine::kLinear ? kernel_ref<LaneLinLong, 16, 32>(e, P)
                                                : kernel_ref<LaneAffLong, 16, 32>(e, P);
+    case kClsBig: return kernel_ref<LaneBig, 16, 32>(e, P);
     case kClsHi: return kernel_ref<LaneHi, 16, 32, true>(e, P);
     case kClsS32: return kernel_ref<LaneS32, 16, 32>(e, P);
     default: return KernelRef{};
@@ -460,9 +474,11 @@ KernelRef kernel_of(const ipuma_engine* e, int cls, int P, bool eight) {
 
 int kernel_grid(ipuma_engine* e, const KernelRef& r) { return r.fn ? occupancy_grid(e, r.fn, r.smem) : 0; }
 
-// Kernel of the strip-team class (linear gaps or affine, one tag bit).
+// Kernel of a strip-team class: linear gaps or affine with one tag bit, or
+// the big class's lanes.
 using TeamKernel = decltype(&k_strips<LaneAffLong, 16>);
-TeamKernel team_kernel(const ipuma_engine* e) {
+TeamKernel team_kernel(const ipuma_engine* e, bool big) {
+  if (big) return k_strips<LaneBig, 16>;
   return e->cells == ipuma_engine::kLinear ? k_strips<LaneLinLong, 16> : k_strips<LaneAffLong, 16>;
 }
 
@@ -496,8 +512,8 @@ int team_warps_for(const ipuma_engine* e, int P, int maxA) {
 }
 
 // Grid of a k_strips<16> launch with `warps` warps per block.
-int team_grid(ipuma_engine* e, int P, int warps) {
-  return occupancy_grid(e, team_kernel(e), team_smem(e, P, warps), 32 * warps);
+int team_grid(ipuma_engine* e, int P, int warps, bool big) {
+  return occupancy_grid(e, team_kernel(e, big), team_smem(e, P, warps), 32 * warps);
 }
 
 template <int K>
@@ -519,7 +535,8 @@ void warm_grids(ipuma_engine* e) {
     for (int c = 0; c < kNumClasses; ++c)
       for (bool eight : {false, true}) kernel_grid(e, kernel_of(e, c, P, eight));
     for (int w = 2; w <= std::min(e->team_warps, kTeamMaxWarps); ++w)
-      if (team_smem(e, P, w) + kTeamStaticSmem <= e->smem_optin) team_grid(e, P, w);
+      if (team_smem(e, P, w) + kTeamStaticSmem <= e->smem_optin)
+        for (bool big : {false, true}) team_grid(e, P, w, big);
   }
 }
 
@@ -527,7 +544,7 @@ void warm_grids(ipuma_engine* e) {
 // the per-run work lists and strip scratch.  Two runs may execute at once
 // (on two streams) only with disjoint sets.
 struct RunBufs {
-  int* ctl;  // CTL_INTS ints, cleared before the run
+  int* ctl;  // CTL_INTS ints, the first CTL_CLEAR cleared before the run
   DevBuf* scratch;
   DevBuf* list;
   DevBuf* ovf;
@@ -584,21 +601,21 @@ int launch_batched(ipuma_engine* e, const KernelRef& kr, const SwConst& sc, cons
   return timed_end(e, s);
 }
 
-// Launches the strip-team class (`warps` warps per block) over its list range.
+// Launches a strip-team class (`warps` warps per block) over its list range.
 int launch_team(ipuma_engine* e, const SwConst& sc, const RunBufs& rb, cudaStream_t s, const uint8_t* codes,
                 const PairDesc* pairs, const int* list, const int* range, int* head, long rowsCap, int* score,
-                int* arange, int* brange, int warps) {
+                int* arange, int* brange, int warps, int cls) {
   const int smem = team_smem(e, sc.P, warps);
-  const int grid = team_grid(e, sc.P, warps);
+  const int grid = team_grid(e, sc.P, warps, cls == kClsBigTeam);
   int* ctl = rb.ctl;
   auto* cells = reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS);
   int rc;
-  if ((rc = timed_begin(e, s, kClasses[kClsTeam].kind, kClsTeam))) return rc;
-  team_kernel(e)<<<grid, 32 * warps, smem, s>>>(
+  if ((rc = timed_begin(e, s, kClasses[cls].kind, cls))) return rc;
+  team_kernel(e, cls == kClsBigTeam)<<<grid, 32 * warps, smem, s>>>(
       lane_const(sc, 0), e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(), rowsCap, score, arange,
       brange, rb.ovf->as<int>(), cells + CELLS_RERUN, reinterpret_cast<DevStatus*>(ctl + CTL_STATUS),
-      reinterpret_cast<const ClassAllot*>(ctl + CTL_ALLOT) + kClsTeam,
-      e->trace ? reinterpret_cast<unsigned long long*>(ctl + CTL_TRACE) + 2 * kClsTeam : nullptr);
+      reinterpret_cast<const ClassAllot*>(ctl + CTL_ALLOT) + cls,
+      e->trace ? reinterpret_cast<unsigned long long*>(ctl + CTL_TRACE) + 2 * cls : nullptr);
   CUDA_TRY(cudaGetLastError());
   return timed_end(e, s);
 }
@@ -642,9 +659,9 @@ long thread_rows(const ipuma_engine* e, int maxA, int maxB) {
 void class_grids(ipuma_engine* e, int P, bool eight, int maxA, int maxB, int* grid, long long* spb) {
   const long long rowsCap = std::max(1, maxB);
   for (int c = 0; c < kNumClasses; ++c) {
-    if (c == kClsTeam) {
+    if (c == kClsTeam || c == kClsBigTeam) {
       const int w = team_warps_for(e, P, maxA);
-      grid[c] = w ? team_grid(e, P, w) : 0;
+      grid[c] = w ? team_grid(e, P, w, c == kClsBigTeam) : 0;
       spb[c] = (long long)w * rowsCap;  // one boundary column per warp of a team
     } else if (c == kClsThread) {
       grid[c] = (int)(thread_threads<16>(e) / kThreads);
@@ -683,7 +700,7 @@ size_t scratch_int2(ipuma_engine* e, int maxA, int maxB) {
 // The hybrid class and the widest class (the long pairs of a heavy-tailed
 // batch) come first and land on different streams, so the widest class's
 // blocks start on the SMs the hybrid class frees during its tail.
-constexpr int kLaunchOrder[kNumClasses] = {23, 22, 24, 5, 21, 4, 6, 3, 15, 9, 14, 2, 13, 8, 12, 1, 20, 11, 19, 7, 18, 10, 17, 0, 16};
+constexpr int kLaunchOrder[kNumClasses] = {26, 23, 25, 22, 24, 5, 21, 4, 6, 3, 15, 9, 14, 2, 13, 8, 12, 1, 20, 11, 19, 7, 18, 10, 17, 0, 16};
 
 int reserve_bufs(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, int n, int maxA, int maxB) {
   int rc;
@@ -742,6 +759,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.n_s16_classes = kNumS16;
   bp.cls_s32 = kClsS32;
   bp.cls_hi = e->hybrid ? kClsHi : kClsS32;
+  bp.cls_big = e->hybrid ? kClsBig : kClsS32;
   bp.nclass = kNumClasses;
   bp.force_s32 = e->s16_ok ? 0 : 1;
   const bool eight = n >= kEightLaneMinPairs;
@@ -750,6 +768,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     kr[c] = kernel_of(e, c, sc.P, eight);
     bp.lanes[c] = kr[c].fn ? kr[c].lanes : kClasses[c].lanes;
     bp.width[c] = kClasses[c].width;
+    bp.inv_width[c] = (unsigned)(((1ull << 32) + kClasses[c].width - 1) / kClasses[c].width);
     bp.slot_ps[c] = e->slot_ps[c];
     bp.strip_ps[c] = e->strip_ps[c];
     bp.fit[c] = (kr[c].fn ? kr[c].limit : e->sc.s16Limit) / e->typical;
@@ -771,8 +790,11 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   const bool conc = mode != 0;
   bp.concurrent = mode;
   // Classes this batch may use (the others are not launched).
-  unsigned enabled = kCoarseClasses | (1u << kClsS32);
-  if (e->hybrid) enabled |= 1u << kClsHi;
+  unsigned enabled = kCoarseClasses;
+  // Pairs that may pass 16 bits need both sequences longer than s16_max_len.
+  const bool highScores = std::min(maxA, maxB) > bp.s16_max_len;
+  if (!e->s16_ok || (highScores && !e->hybrid)) enabled |= 1u << kClsS32;
+  if (highScores && e->hybrid) enabled |= (1u << kClsHi) | (1u << kClsBig);
   if (n >= kFineClassMinPairs) enabled |= kFineClasses;
   // The long class, when the batch may hold a pair past the widest's scores.
   if (std::min(maxA, maxB) > bp.fit[kClsWidest]) enabled |= 1u << kClsLong;
@@ -791,13 +813,15 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
                 kClsTeam + 1);
   if (teamW >= 2 && maxA > kClasses[kClsTeam].width && e->tile_k == 0) enabled |= 1u << kClsTeam;
   if (e->tile_k > 0) enabled |= 1u << (e->tile_k - 1);
+  if (((enabled >> kClsTeam) & 1u) && ((enabled >> kClsBig) & 1u)) enabled |= 1u << kClsBigTeam;
   for (int c = 0; c < kNumClasses; ++c)
-    if (c != kClsThread && c != kClsTeam && !kr[c].fn) {
+    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].fn) {
       if (e->tile_k == c + 1) return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d has no kernel for this scoring", e->tile_k);
       enabled &= ~(1u << c);
     }
   bp.enabled = enabled;
   bp.team_cls = ((enabled >> kClsTeam) & 1u) ? kClsTeam : -1;
+  bp.team_big = ((enabled >> kClsBigTeam) & 1u) ? kClsBigTeam : -1;
   bp.team_warps = std::max(teamW, 1);
   class_grids(e, sc.P, eight, maxA, maxB, bp.grid, bp.scr_per_block);
   bp.scr_cap = (long long)(rb.scratch->cap / sizeof(int2));
@@ -809,11 +833,11 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)k * (float)(bp.grid[c] * kWarpsPerBlock);
     if (kr[c].fn) slot_min = std::min(slot_min, e->slot_ps[c]);
   }
-  bp.step_ps[kClsLong] =
-      e->slot_ps[kClsLong] * 64.f * (float)kClasses[kClsLong].k * (float)(bp.grid[kClsLong] * kWarpsPerBlock);
+  for (int c : {kClsLong, kClsBig})
+    bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * kWarpsPerBlock);
   // A warp of a team steps like one of the widest class's warps.
-  bp.step_ps[kClsTeam] =
-      e->slot_ps[kClsTeam] * 64.f * (float)kClasses[kClsTeam].k * (float)(bp.grid[kClsTeam] * bp.team_warps);
+  for (int c : {kClsTeam, kClsBigTeam})
+    bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * bp.team_warps);
   bp.batch_ps_per_cell = slot_min / kPackingEfficiency;
   bp.lat_share = e->latency_share;
   bp.lat_min_ps = kLatencyMinBatchPs;
@@ -836,25 +860,31 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.bits = bits;
   bp.M = e->M;
   bp.s16_limit = kr[kClsLong].limit;
+  bp.big_limit = kr[kClsBig].limit;
   if ((rc = rb.flag->ensure((size_t)n + 64, s))) return rc;
   const int nkeys = bp.nclass * NBUCKET;
   const int tb = 256;
   const int gb = std::min<int>((n + tb - 1) / tb, e->nsm * 8);
-  k_bin_total<<<gb, tb, 0, s>>>(bp, pairs, n,
-                                reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS) + CELLS_TOTAL);
-  k_bin_bound<<<gb, tb, 0, s>>>(bp, codes, e->d_sim.as<int8_t>(), pairs, n, rb.flag->as<uint8_t>());
-  k_bin_count<<<gb, tb, 0, s>>>(bp, codes, e->d_sim.as<int8_t>(), pairs, n, ctl + CTL_HIST,
-                                rb.flag->as<uint8_t>(),
-                                reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS),
-                                reinterpret_cast<unsigned long long*>(ctl + CTL_COST), st, score,
-                                arange, brange);
-  k_bin_scan<<<1, 1024, 0, s>>>(bp, nkeys, ctl + CTL_HIST, ctl + CTL_OFFS, ctl + CTL_RANGES,
-                                reinterpret_cast<const unsigned long long*>(ctl + CTL_COST),
-                                reinterpret_cast<ClassAllot*>(ctl + CTL_ALLOT), st);
-  k_bin_scatter<<<gb, tb, 0, s>>>(bp, pairs, n, rb.flag->as<uint8_t>(), ctl + CTL_OFFS,
-                                  rb.list->as<int>());
+  auto* total = reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS) + CELLS_TOTAL;
+  auto* sums = reinterpret_cast<ClassSums*>(ctl + CTL_SUMS);
+  auto* allot = reinterpret_cast<ClassAllot*>(ctl + CTL_ALLOT);
+  uint8_t* flags = rb.flag->as<uint8_t>();
+  if (highScores) {  // without long pairs no flag is read
+    k_bin_bound<<<gb, tb, 0, s>>>(bp, codes, e->d_sim.as<int8_t>(), pairs, n, flags);
+    *launches += 1;
+  }
+  if (n <= kSmallBin) {
+    k_bin_small<<<1, 1024, 0, s>>>(bp, pairs, n, flags, total, sums, ctl + CTL_RANGES, allot, st, rb.list->as<int>(),
+                                   score, arange, brange);
+    *launches += 1;
+  } else {
+    k_bin_total<<<gb, tb, 0, s>>>(bp, pairs, n, total, ctl + CTL_HIST, nkeys);
+    k_bin_count<<<gb, tb, 0, s>>>(bp, pairs, n, ctl + CTL_HIST, flags, sums, st, score, arange, brange);
+    k_bin_scan<<<bp.nclass, 1024, 0, s>>>(bp, ctl + CTL_HIST, ctl + CTL_OFFS, sums, ctl + CTL_RANGES, allot, st);
+    k_bin_scatter<<<gb, tb, 0, s>>>(bp, pairs, n, flags, ctl + CTL_OFFS, rb.list->as<int>());
+    *launches += 4;
+  }
   CUDA_TRY(cudaGetLastError());
-  *launches += 5;
 
   int* list = rb.list->as<int>();
   int* heads = ctl + CTL_HEADS;
@@ -885,9 +915,9 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   for (const int c : kLaunchOrder) {
     if (!((enabled >> c) & 1u)) continue;
     cudaStream_t cs = on(c);
-    if (c == kClsTeam)
+    if (c == kClsTeam || c == kClsBigTeam)
       rc = launch_team(e, sc, rb, cs, codes, pairs, list, R + 2 * c, heads + c, rowsCap, score, arange, brange,
-                       teamW);
+                       teamW, c);
     else if (c == kClsThread)
       rc = launch_thread<16>(e, rb, cs, codes, pairs, list, R + 2 * c, heads + c, thread_rows(e, maxA, maxB), score,
                              arange, brange, c);
@@ -897,10 +927,17 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     if (rc || (rc = done(c))) return rc;
     ++*launches;
   }
+  // No pair of this batch can leave the range of the lanes it ran in?
+  const long long maxScore = (long long)std::min(maxA, maxB) * std::max(0, e->maxSub);
+  bool overflow = e->thread_class || e->tile_k == kClsThread + 1;
+  for (int c = 0; c < kNumClasses; ++c)
+    if (((enabled >> c) & 1u) && c != kClsS32)
+      overflow |= maxScore > (kr[c].fn ? kr[c].limit : kr[kClsLong].limit);
+  if (!overflow) return IPUMA_OK;
   // Exact 32-bit rerun of the s16x2 pairs whose score may have overflowed
   // (after every class: it reads their overflow list).
   if ((rc = launch_batched(e, kr[kClsS32], sc, rb, s, codes, pairs, rb.ovf->as<int>(), ctl + CTL_STATUS + 1,
-                           heads + NCLASS_MAX, rowsCap, score, arange, brange, IPUMA_KERNEL_S32_RERUN, CELLS_RERUN,
+                           heads + NCLASS_MAX, rowsCap, score, arange, brange, IPUMA_KERNEL_S32_RERUN, kTimedRerun,
                            NCLASS_MAX)))
     return rc;
   *launches += 1;
@@ -911,39 +948,42 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
 int reset_ctl(ipuma_engine* e, cudaStream_t s) {
   int rc;
   if ((rc = e->d_ctl.ensure(sizeof(int) * CTL_INTS, s))) return rc;
-  CUDA_TRY(cudaMemsetAsync(e->d_ctl.p, 0, sizeof(int) * CTL_INTS, s));
+  CUDA_TRY(cudaMemsetAsync(e->d_ctl.p, 0, sizeof(int) * CTL_CLEAR, s));
   e->n_timed = 0;
   return IPUMA_OK;
 }
 
-// Forward-pass cells counted for class c (or the rerun) over `nblk` runs.
-template <size_t N>
-unsigned long long cells_of(const unsigned long long (*cells)[N], int nblk, int c) {
-  unsigned long long v = 0;
-  for (int k = 0; k < nblk; ++k) v += cells[k][c];
-  return v;
-}
-
 // Waits for the stream and reads the status of the call's runs: `nblk`
 // consecutive control blocks at the start of d_ctl (one per run; errors,
-// overflow reruns and per-class cells are summed).
+// overflow reruns and per-class cells are summed).  The cleared part of a
+// block holds all of it: one copy per run, into pinned memory (three
+// pageable copies cost a small call 30 us).
 int check_status(ipuma_engine* e, cudaStream_t s, int nblk = 1) {
-  DevStatus st{};
-  unsigned long long cells[NCELLS] = {};
-  DevStatus stk[kMaxChunks];
-  unsigned long long cellsk[kMaxChunks][NCELLS];
-  unsigned long long tracek[kMaxChunks][2 * (NCLASS_MAX + 1)];
-  int rangesk[kMaxChunks][2 * NCLASS_MAX];
   nblk = std::max(1, std::min(nblk, kMaxChunks));
-  for (int k = 0; k < nblk; ++k) {
-    const int* ctl = e->d_ctl.as<int>() + (size_t)k * CTL_INTS;
-    CUDA_TRY(cudaMemcpyAsync(&stk[k], ctl + CTL_STATUS, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaMemcpyAsync(cellsk[k], ctl + CTL_CELLS, sizeof(cellsk[k]), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaMemcpyAsync(rangesk[k], ctl + CTL_RANGES, sizeof(rangesk[k]), cudaMemcpyDeviceToHost, s));
-    if (e->trace)
-      CUDA_TRY(cudaMemcpyAsync(tracek[k], ctl + CTL_TRACE, sizeof(tracek[k]), cudaMemcpyDeviceToHost, s));
-  }
+  if (!e->h_ctl) CUDA_TRY(cudaHostAlloc(&e->h_ctl, sizeof(int) * CTL_CLEAR * kMaxChunks, cudaHostAllocPortable));
+  for (int k = 0; k < nblk; ++k)
+    CUDA_TRY(cudaMemcpyAsync(e->h_ctl + (size_t)k * CTL_CLEAR, e->d_ctl.as<int>() + (size_t)k * CTL_INTS,
+                             sizeof(int) * CTL_CLEAR, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
+  DevStatus st{};
+  // Cells per class, then those of CTL_CELLS (kTimedRerun, kTimedWire).
+  unsigned long long cells[NCLASS_MAX + NCELLS] = {};
+  const auto block = [&](int k) { return e->h_ctl + (size_t)k * CTL_CLEAR; };
+  e->stats.s32_pairs = 0;
+  for (int k = 0; k < nblk; ++k) {
+    DevStatus stk;
+    memcpy(&stk, block(k) + CTL_STATUS, sizeof(stk));
+    if (!st.error) st.error = stk.error;
+    st.overflow_count += stk.overflow_count;
+    ClassSums sums[NCLASS_MAX];
+    memcpy(sums, block(k) + CTL_SUMS, sizeof(sums));
+    unsigned long long more[NCELLS];
+    memcpy(more, block(k) + CTL_CELLS, sizeof(more));
+    for (int c = 0; c < NCLASS_MAX; ++c) cells[c] += sums[c].cells;
+    for (int c = 0; c < NCELLS; ++c) cells[NCLASS_MAX + c] += more[c];
+    // Pairs the binning sent to the s32, hybrid and big classes.
+    for (int c : {kClsS32, kClsHi, kClsBig, kClsBigTeam}) e->stats.s32_pairs += sums[c].count;
+  }
   e->stats.n_trace = 0;
   if (e->trace) {
     // Per class (and the rerun): earliest block start and latest warp end
@@ -954,9 +994,11 @@ int check_status(ipuma_engine* e, cudaStream_t s, int nblk = 1) {
       st0[c] = ~0ull;
       en[c] = 0;
       for (int k = 0; k < nblk; ++k) {
-        if (!tracek[k][2 * c + 1]) continue;
-        st0[c] = std::min(st0[c], ~tracek[k][2 * c]);
-        en[c] = std::max(en[c], tracek[k][2 * c + 1]);
+        unsigned long long t[2];
+        memcpy(t, block(k) + CTL_TRACE + 4 * c, sizeof(t));
+        if (!t[1]) continue;
+        st0[c] = std::min(st0[c], ~t[0]);
+        en[c] = std::max(en[c], t[1]);
       }
       if (en[c]) t0 = std::min(t0, st0[c]);
     }
@@ -966,20 +1008,10 @@ int check_status(ipuma_engine* e, cudaStream_t s, int nblk = 1) {
       e->stats.trace_kind[i] = c < kNumClasses ? kClasses[c].kind : IPUMA_KERNEL_S32_RERUN;
       e->stats.trace_start_ms[i] = (double)(st0[c] - t0) * 1e-6;
       e->stats.trace_end_ms[i] = (double)(en[c] - t0) * 1e-6;
-      e->stats.trace_cells[i] = (int64_t)cells_of(cellsk, nblk, c < kNumClasses ? c : CELLS_RERUN);
+      e->stats.trace_cells[i] = (int64_t)cells[c < kNumClasses ? c : kTimedRerun];
     }
   }
-  for (int k = 0; k < nblk; ++k) {
-    if (!st.error) st.error = stk[k].error;
-    st.overflow_count += stk[k].overflow_count;
-    for (int c = 0; c < NCELLS; ++c) cells[c] += cellsk[k][c];
-  }
   e->stats.overflow_reruns = st.overflow_count;
-  // Pairs the binning sent to the s32 and hybrid classes ({start, count}
-  // list ranges per class).
-  e->stats.s32_pairs = 0;
-  for (int k = 0; k < nblk; ++k)
-    e->stats.s32_pairs += (int64_t)rangesk[k][2 * kClsS32 + 1] + (int64_t)rangesk[k][2 * kClsHi + 1];
   e->stats.n_timed = e->n_timed;
   for (int k = 0; k < e->n_timed; ++k) {
     float ms = 0;
@@ -987,7 +1019,7 @@ int check_status(ipuma_engine* e, cudaStream_t s, int nblk = 1) {
     e->stats.timed_kind[k] = e->timed_kind[k];
     e->stats.timed_ms[k] = ms;
     const int c = e->timed_cls[k];
-    e->stats.timed_cells[k] = (c >= 0 && c < NCELLS) ? (int64_t)cells[c] : 0;
+    e->stats.timed_cells[k] = c >= 0 ? (int64_t)cells[c] : 0;
   }
   e->n_timed = 0;
   if (st.error == ERR_LENGTH) return fail(IPUMA_ERR_TOO_LONG, "a pair exceeds the stated maximum length");
@@ -1018,7 +1050,7 @@ int run_plain_wire(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const int
     const long warps = (long)grid * kWarpsPerBlock;
     int r;
     if ((r = rb.scratch->ensure(sizeof(int2) * 2 * rowsCap * warps, s))) return r;
-    if ((r = timed_begin(e, s, s16 ? IPUMA_KERNEL_PLAIN_S16 : IPUMA_KERNEL_PLAIN, CELLS_WIRE))) return r;
+    if ((r = timed_begin(e, s, s16 ? IPUMA_KERNEL_PLAIN_S16 : IPUMA_KERNEL_PLAIN, kTimedWire))) return r;
     kern<<<grid, kThreads, smem, s>>>(e->sc, e->d_sim.as<int8_t>(), d_inputs, seqWordsPerTile,
                                       metaOffset, maxBatches, totalSlots, rb.scratch->as<int2>(),
                                       rowsCap, d_results, st);
@@ -1073,6 +1105,10 @@ void set_s32_rates(ipuma_engine* e) {
   e->strip_ps[kClsTeam] = e->strip_ps[kClsWidest];
   e->slot_ps[kClsLong] = e->slot_ps[kClsWidest];
   e->strip_ps[kClsLong] = e->strip_ps[kClsWidest];
+  for (int c : {kClsBig, kClsBigTeam}) {  // their whole best row costs a seventh more per cell
+    e->slot_ps[c] = 1.15f * e->slot_ps[kClsWidest];
+    e->strip_ps[c] = e->strip_ps[kClsWidest];
+  }
 }
 
 void set_default_rates(ipuma_engine* e) {
@@ -1723,6 +1759,7 @@ void ipuma_gpu_destroy(ipuma_engine* e) {
                   &e->x_ovf, &e->x_flag, &e->w1.inputs, &e->w1.results, &e->w1.pairs, &e->w1.ctl, &e->w1.list,
                   &e->w1.scratch, &e->w1.ovf, &e->w1.flag})
     b->release();
+  if (e->h_ctl) cudaFreeHost(e->h_ctl);
   for (auto& ev : e->cev)
     if (ev) cudaEventDestroy(ev);
   for (int c = 0; c < NCLASS_MAX; ++c) {
@@ -2052,7 +2089,7 @@ static int compare_host(ipuma_engine* e, const uint8_t* codes, size_t n_codes, i
     const bool pinned_out = is_pinned(score) && is_pinned(arange) && is_pinned(brange);
     cudaStream_t run_s[2] = {s, e->stream2};
     CUDA_TRY(cudaEventRecord(e->ev[0], s));
-    CUDA_TRY(cudaMemsetAsync(e->d_ctl.p, 0, sizeof(int) * CTL_INTS * (size_t)nch, s));
+    CUDA_TRY(cudaMemset2DAsync(e->d_ctl.p, sizeof(int) * CTL_INTS, 0, sizeof(int) * CTL_CLEAR, nch, s));
     e->n_timed = 0;
     CUDA_TRY(cudaEventRecord(e->ev[1], s));
     CUDA_TRY(cudaStreamWaitEvent(e->stream2, e->ev[1], 0));
@@ -2215,7 +2252,7 @@ static int enqueue_buffer(ipuma_engine* e, const int32_t* inputs, size_t n_input
     return rc;
 
   CUDA_TRY(cudaEventRecord(j.ev[0], s));
-  CUDA_TRY(cudaMemsetAsync(w.rb.ctl, 0, sizeof(int) * CTL_INTS, s));
+  CUDA_TRY(cudaMemsetAsync(w.rb.ctl, 0, sizeof(int) * CTL_CLEAR, s));
   e->n_timed = 0;
   int32_t* d_in = w.inputs->as<int32_t>();
   const long usedTiles = m.last < 0 ? 0 : m.last / std::max(1, a.max_batches) + 1;

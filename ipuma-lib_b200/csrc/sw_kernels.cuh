@@ -25,7 +25,8 @@
 //                     k_bin_total (batch cells), k_bin_bound (main-diagonal
 //                     bounds of the long pairs, a warp per pair), k_bin_count
 //                     (class and bucket of every pair), k_bin_scan (list
-//                     offsets and class shares), k_bin_scatter (the list).
+//                     offsets and class shares), k_bin_scatter (the list);
+//                     k_bin_small does all of it for a few thousand pairs.
 #pragma once
 #include "sw_device.cuh"
 #include "sw_tagged.cuh"
@@ -389,17 +390,48 @@ __global__ void __launch_bounds__(128, (FWD && !HYB) ? 4 : 3) k_batched(SwConst 
   if (trace && lane32 == 0) atomicMax(&trace[1], global_ns());
 }
 
-// Strip-team kernel: the blockDim.x / 32 warps of a block align one item
-// (the two pairs of a 32-lane s16x2 group), taking its 32 * K wide strips
-// round robin (tag_pass with TEAM), so a long pair finishes up to `warps`
-// times sooner than on one warp.  Each warp keeps the best cell of its own
-// strips; the block merges them with the first-strict-maximum order
+// Strip-team kernel: teams of warps of a block align one item each (two
+// pairs in 16-bit halves), taking its 32 * K wide strips round robin
+// (tag_pass with TEAM), so a long pair finishes up to `team size` times
+// sooner than on one warp.  Each warp keeps the best cell of its own
+// strips; the team merges them with the first-strict-maximum order
 // (better), the order-independent total order the one-warp pass applies
 // strip by strip.  With start coordinates the team then runs the reverse
 // pass the same way.  A team that gave up (a 16-bit overflow, or a wait
 // past kTeamWaitNs, which also sets ERR_WAIT) sends both pairs to the s32
-// rerun.  Block scratch: `warps` boundary columns of rowsCap rows.
+// rerun.  Block scratch: one boundary column of rowsCap rows per warp.
+//
+// A block's warps form one team, two or four (team_size): with fewer items
+// than blocks only the largest team uses the SM's warps at all; with more,
+// a smaller one wastes less on the strips' rounding (9 strips keep 8 warps
+// busy 9 of 16 turns, two warps 9 of 10) and on the lag between warps.
 constexpr int kTeamMaxWarps = 8;
+
+// Steps a team warp starts behind the warp before it: it reads the boundary
+// rows of a block of 32 when it starts the block, and that warp publishes
+// them a block later.
+constexpr float kTeamLagSteps = 64.f;
+
+// Warps per team: the divisor of the block's warps (down to a quarter, two
+// at least) that finishes `items` items like the list's first, its longest,
+// soonest -- rounds of items times the steps of one item.
+__device__ __forceinline__ int team_size(int warps, long blocks, int items, int strips, int rows) {
+  int best = warps;
+  float bestCost = 3.0e38f;
+  for (int t = warps; t >= 2 && 4 * t >= warps; t /= 2) {
+    const long slots = blocks * (warps / t);
+    const float cost = (float)((items + slots - 1) / slots) *
+                       ((float)((strips + t - 1) / t) * (float)(rows + 32) +
+                        kTeamLagSteps * (float)(min(strips, t) - 1));
+    if (cost < bestCost) {
+      bestCost = cost;
+      best = t;
+    }
+    if (t & 1) break;
+  }
+  return best;
+}
+
 template <class T, int K>
 __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __restrict__ sim,
                                                    const uint8_t* __restrict__ codes,
@@ -416,11 +448,12 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
   using L = SmemLayout<T, K, 32>;
   constexpr int NP = 2;
   extern __shared__ __align__(16) uint8_t smem[];
+  constexpr int MAXT = kTeamMaxWarps / 2;  // teams of a block
   __shared__ int s_prog[kTeamMaxWarps];
-  __shared__ int s_abort, s_item;
+  __shared__ int s_abort[MAXT], s_item[MAXT];
   __shared__ Best s_res[kTeamMaxWarps][NP];
-  __shared__ Best s_best[2][NP];  // merged best of the forward / reverse pass
-  __shared__ bool s_ovf[NP];
+  __shared__ Best s_bestT[MAXT][2][NP];  // merged best of the forward / reverse pass
+  __shared__ bool s_ovfT[MAXT][NP];
   const int warps = blockDim.x >> 5;
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -429,20 +462,35 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
   uint16_t* s_bring = reinterpret_cast<uint16_t*>(s_prof + L::prof_bytes(sc.P));
   load_table(s_simp, sim, sc, kProfBias<T> ? -sc.gE : 0, kProfShift<T>);
 
+  __syncthreads();  // s_simp is loaded
+
   const int n = range[1];
   list += range[0];
   const int items = (n + NP - 1) / NP;
-  int2* scr = scratch + (long)blockIdx.x * warps * rowsCap;
-  const StripTeam team{s_prog, &s_abort, &st->error, ERR_WAIT, wib, warps};
+  if (n <= 0) return;
+  const PairDesc longest = pairs[list[0]];
+  const int tsize = team_size(warps, min((long)gridDim.x, (long)allot->blocks), items,
+                              (longest.a_len + 32 * K - 1) / (32 * K), longest.b_len);
+  const int q = wib / tsize, tw = wib % tsize;  // this warp's team, and its place there
+  if (q >= warps / tsize) return;               // warps past the last whole team
+  const int tid = tw * 32 + lane;
+  // A barrier of the team's warps (barrier 0 is the block's).
+  const auto team_sync = [&]() {
+    asm volatile("bar.sync %0, %1;" ::"r"(q + 1), "r"(32 * tsize) : "memory");
+  };
+  Best(&s_best)[2][NP] = s_bestT[q];
+  bool(&s_ovf)[NP] = s_ovfT[q];
+  int2* scr = scratch + ((long)blockIdx.x * warps + q * tsize) * rowsCap;
+  const StripTeam team{s_prog + q * tsize, &s_abort[q], &st->error, ERR_WAIT, tw, tsize};
   while (true) {
-    __syncthreads();  // the previous item's merge is done; s_simp is loaded
-    if (threadIdx.x == 0) {
-      s_item = atomicAdd(queue_head, 1);
-      s_abort = 0;
+    team_sync();  // the previous item's merge is done
+    if (tid == 0) {
+      s_item[q] = atomicAdd(queue_head, 1);
+      s_abort[q] = 0;
     }
-    if (threadIdx.x < warps) s_prog[threadIdx.x] = -1;
-    __syncthreads();
-    const int item = s_item;
+    if (lane == 0) s_prog[wib] = -1;
+    team_sync();
+    const int item = s_item[q];
     if (item >= items) break;
     int pid[NP];
     PairDesc d[NP];
@@ -456,7 +504,7 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
     }
     if (tooLong) {
       // The host sizes the scratch for the longest B; report, never trap.
-      if (threadIdx.x == 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
+      if (tid == 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
       continue;
     }
     PassSeq ps[NP];
@@ -477,23 +525,23 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
 #pragma unroll
         for (int h = 0; h < NP; ++h) s_res[wib][h] = out[h];
       }
-      __syncthreads();
-      if (threadIdx.x < NP) {
-        const int h = threadIdx.x;
-        Best b = s_res[0][h];
-        for (int w = 1; w < warps; ++w) {
-          const Best c = s_res[w][h];
+      team_sync();
+      if (tid < NP) {
+        const int h = tid;
+        Best b = s_res[q * tsize][h];
+        for (int w = 1; w < tsize; ++w) {
+          const Best c = s_res[q * tsize + w][h];
           if (better(c.s, c.i, c.j, b.s, b.i, b.j)) b = c;
         }
         s_best[pass][h] = b;
         // A team that gave up (in either pass) sends the pair to the rerun.
         if (pass == 0) {
-          s_ovf[h] = s_abort != 0 || b.s > Cell<T>::limit(sc);
+          s_ovf[h] = s_abort[q] != 0 || b.s > Cell<T>::limit(sc);
           s_best[1][h] = Best{0, 0, 0};  // the start of a pair without a reverse pass
         }
-        if (pass == 1 && s_abort != 0) s_ovf[h] = true;
+        if (pass == 1 && s_abort[q] != 0) s_ovf[h] = true;
       }
-      __syncthreads();
+      team_sync();
       if (pass == 1 || sc.forwardOnly) break;
       bool any = false;
 #pragma unroll
@@ -506,13 +554,13 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
       }
       if (!any) break;  // block-uniform: every thread read the same words
       // A fresh team for the reverse pass (after every warp read s_ovf).
-      __syncthreads();
-      if (threadIdx.x == 0) s_abort = 0;
-      if (threadIdx.x < warps) s_prog[threadIdx.x] = -1;
-      __syncthreads();
+      team_sync();
+      if (tid == 0) s_abort[q] = 0;
+      if (lane == 0) s_prog[wib] = -1;
+      team_sync();
     }
-    if (threadIdx.x < NP) {
-      const int h = threadIdx.x;
+    if (tid < NP) {
+      const int h = tid;
       if (pid[h] >= 0) {
         if (s_ovf[h]) {
           const int slot = atomicAdd(&st->overflow_count, 1);
@@ -723,7 +771,7 @@ static __global__ void k_exact(SwConst sc, const int8_t* __restrict__ sim, const
 constexpr int NROWB = 256;    // row buckets (16 per power of two)
 constexpr int NSTRIPB = 16;   // strip-count buckets
 constexpr int NBUCKET = NROWB * NSTRIPB;
-constexpr int NCLASS_MAX = 25;
+constexpr int NCLASS_MAX = 27;
 
 // Log-linear bucket of |B| (16 sub-buckets per power of two): pairs that
 // share a bucket differ by at most 1/16 in rows, so the groups of a warp
@@ -737,8 +785,12 @@ __device__ __forceinline__ int rows_bucket(int b) {
 struct BinParams {
   int nclass;
   int cls_s32;             // class index of the exact-32-bit kernel
-  int cls_hi;              // class of pairs the diagonal bound sends to 32 bits:
+  int cls_hi;              // class of pairs whose diagonal bound passes big_limit:
                            // the hybrid class (or cls_s32 when it is off)
+  int cls_big;             // class of the other pairs past s16_limit (cls_s32 when
+                           // the hybrid class is off), and its strip-team class (-1: none)
+  int team_big;
+  int big_limit;           // scores above this need more than 16 biased bits
   int s16_max_len;         // min(|A|,|B|) above which the 16-bit lanes could overflow
   int s16_limit;           // scores above this need more than the long class's 16 bits
   // Longest min(|A|,|B|) a class is chosen for by cost: a typical identical
@@ -747,6 +799,7 @@ struct BinParams {
   int fit[NCLASS_MAX];
   int lanes[NCLASS_MAX];   // lanes per group of each class
   int width[NCLASS_MAX];   // strip width (lanes * K) of each class
+  unsigned inv_width[NCLASS_MAX];  // ceil(2^32 / width): strips_of
   float slot_ps[NCLASS_MAX];   // time per cell slot of a strip (autotuned)
   float strip_ps[NCLASS_MAX];  // fixed time per strip (autotuned)
   // Latency bound: one warp item of class c advances one step (row) every
@@ -857,10 +910,6 @@ static __device__ int warp_diagonal_bound(const uint8_t* codes, int bits, long l
   return __shfl_sync(FULL, r.best, 0);
 }
 
-// Steps a team warp starts behind the warp before it: it reads the boundary
-// rows of a block of 32 when it starts the block, and that warp publishes
-// them a block later.
-constexpr float kTeamLagSteps = 64.f;
 // Share of the batch's modelled time above which a pair's one-warp latency
 // sends it to a strip team (measured on B200: a 500,000-pair heavy-tailed
 // protein batch, whose 8,000-residue pairs take about a third of its time
@@ -874,13 +923,45 @@ constexpr float kTeamLatencyShare = 0.5f;
 // each strip's wavefront, and slot_ps / strip_ps are the per-class rates
 // the autotuner measured.  Key = class, then strip count (descending), then
 // rows (descending).
-__device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen, bool s32, float thr_cap,
+// Strips of class c that cover alen columns: (alen + width - 1) / width by
+// multiplication (exact: the numerator times width stays below 2^32).
+__device__ __forceinline__ int strips_of(const BinParams& bp, int c, int alen) {
+  return (int)__umulhi((unsigned)(alen + bp.width[c] - 1), bp.inv_width[c]);
+}
+
+// A strip team's class `tc` for a pair whose one-warp latency is `lat`, or
+// cls: taken when even the fastest warp would take a large share of the
+// whole batch's modelled time (kTeamLatencyShare: below it the other pairs'
+// work hides the pair, and a team's fill and idle warps only cost
+// throughput) and the team finishes the pair sooner.  Its warps take the
+// strips round robin, each starting about kTeamLagSteps behind the warp
+// before it.
+__device__ __forceinline__ int team_class(const BinParams& bp, int cls, int tc, int alen, int blen, float lat,
+                                          float batch_ps) {
+  if (tc < 0 || lat <= kTeamLatencyShare * batch_ps) return cls;
+  const int strips = strips_of(bp, tc, alen);
+  if (strips < 2) return cls;
+  const int rounds = (strips + bp.team_warps - 1) / bp.team_warps;
+  const float tl = ((float)rounds * (float)(blen + bp.lanes[tc]) +
+                    kTeamLagSteps * (float)(min(strips, bp.team_warps) - 1)) *
+                   bp.step_ps[tc];
+  return tl < lat ? tc : cls;
+}
+
+// `flag`: 0, 1 (the diagonal bound passes s16_limit) or 2 (big_limit).
+__device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen, int flag, float thr_cap,
                                         float* cost_out = nullptr) {
   int cls;
   if (bp.force_s32) {
     cls = bp.cls_s32;
-  } else if (s32) {
+  } else if (flag == 2) {
     cls = bp.cls_hi;
+  } else if (flag == 1) {
+    cls = bp.cls_big;
+    const float batch_ps = bp.total_cells ? (float)(*bp.total_cells) * bp.batch_ps_per_cell : 0.f;
+    const float lat = (float)strips_of(bp, cls, alen) * (float)(blen + bp.lanes[cls]) *
+                      bp.step_ps[cls];
+    cls = team_class(bp, cls, bp.team_big, alen, blen, lat, batch_ps);
   } else if (bp.forced_class >= 0) {
     cls = bp.forced_class;
   } else {
@@ -893,7 +974,7 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
       // latency, not throughput, sets the end of the launch, and the widest
       // strips finish a pair in the fewest steps.
       cls = wide;
-      bestLat = (float)((alen + bp.width[cls] - 1) / bp.width[cls]) * (float)(blen + bp.lanes[cls]) *
+      bestLat = (float)strips_of(bp, cls, alen) * (float)(blen + bp.lanes[cls]) *
                 bp.step_ps[cls];
     } else {
       cls = wide;
@@ -904,7 +985,7 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
       for (int c = 0; c < bp.n_s16_classes; ++c) {
         if (!((bp.enabled >> c) & 1u)) continue;
         if ((c == bp.thr_cls && !thr_ok) || fit > bp.fit[c]) continue;
-        const int strips = (alen + bp.width[c] - 1) / bp.width[c];
+        const int strips = strips_of(bp, c, alen);
         const float lat = (float)strips * (float)(blen + bp.lanes[c]) * bp.step_ps[c];
         if (bestLat < 0.f || lat < bestLat) {
           bestLat = lat;
@@ -919,7 +1000,7 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
         }
       }
       if (bestLat < 0.f) {  // no class holds its scores but the long one
-        bestLat = (float)((alen + bp.width[cls] - 1) / bp.width[cls]) * (float)(blen + bp.lanes[cls]) *
+        bestLat = (float)strips_of(bp, cls, alen) * (float)(blen + bp.lanes[cls]) *
                   bp.step_ps[cls];
       } else if (bestCost < 0.f) {
         cls = latCls;  // every class is too slow: the fastest
@@ -927,25 +1008,9 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
         bestLat = 0.f;  // a class keeps the pair under the latency cap
       }
     }
-    // A strip team, when even the fastest warp would take a large share of
-    // the whole batch's modelled time (kTeamLatencyShare: below it the
-    // other pairs' work hides the pair, and a team's fill and idle warps
-    // only cost throughput) and the team finishes the pair sooner.  Its
-    // warps take the strips round robin, each starting about kTeamLagSteps
-    // behind the warp before it.
-    const int tc = bp.team_cls;
-    if (tc >= 0 && bestLat > kTeamLatencyShare * batch_ps) {
-      const int strips = (alen + bp.width[tc] - 1) / bp.width[tc];
-      if (strips >= 2) {
-        const int rounds = (strips + bp.team_warps - 1) / bp.team_warps;
-        const float lat = ((float)rounds * (float)(blen + bp.lanes[tc]) +
-                           kTeamLagSteps * (float)(min(strips, bp.team_warps) - 1)) *
-                          bp.step_ps[tc];
-        if (lat < bestLat) cls = tc;
-      }
-    }
+    cls = team_class(bp, cls, bp.team_cls, alen, blen, bestLat, batch_ps);
   }
-  const int strips = (alen + bp.width[cls] - 1) / bp.width[cls];
+  const int strips = strips_of(bp, cls, alen);
   if (cost_out)
     *cost_out = (float)strips *
                 ((float)(blen + bp.lanes[cls]) * (float)bp.width[cls] * bp.slot_ps[cls] + bp.strip_ps[cls]);
@@ -965,7 +1030,9 @@ __device__ __forceinline__ float thread_cap(const BinParams& bp) {
 // Sum of |A| * |B| over the pairs the pipeline will align (the batch size
 // the per-thread class's latency cap is measured against).
 static __global__ void k_bin_total(BinParams bp, const PairDesc* __restrict__ pairs, int n,
-                                   unsigned long long* total) {
+                                   unsigned long long* total, int* hist, int nkeys) {
+  // The key histogram of the launches after this one starts at zero.
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nkeys; k += gridDim.x * blockDim.x) hist[k] = 0;
   unsigned long long local = 0;
   for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
     const PairDesc d = pairs[p];
@@ -1007,140 +1074,223 @@ static __global__ void k_bin_bound(BinParams bp, const uint8_t* __restrict__ cod
       const PairDesc d = pairs[q];
       const int bound =
           warp_diagonal_bound(codes, bp.bits, d.a_off, d.b_off, min(d.a_len, d.b_len), simT, bp.M);
-      if (lane == 0) s32_flag[q] = bound > bp.s16_limit ? 1 : 0;
+      if (lane == 0) s32_flag[q] = bound > bp.big_limit ? 2 : bound > bp.s16_limit ? 1 : 0;
     }
   }
 }
 
-static __global__ void k_bin_count(BinParams bp, const uint8_t* __restrict__ codes, const int8_t* __restrict__ sim,
-                            const PairDesc* __restrict__ pairs, int n, int* hist, uint8_t* s32_flag,
-                            unsigned long long* class_cells, unsigned long long* class_cost, DevStatus* st,
-                            int* score, int* arange, int* brange) {
-  // Per-class sums of the block, added to the global ones once at the end
-  // (a batch has a handful of classes: one global address per class would
-  // take every pair's atomic).
-  __shared__ unsigned long long s_cells[NCLASS_MAX + 1], s_cost[NCLASS_MAX + 1];
-  for (int k = threadIdx.x; k <= NCLASS_MAX; k += blockDim.x) {
-    s_cells[k] = 0;
-    s_cost[k] = 0;
+// Sums of the pairs of one class: cells, modelled cost (ps) and pairs.
+struct ClassSums {
+  unsigned long long cells, cost;
+  int count, pad;
+};
+
+// Key of one listed pair; its cells and cost go to the block's class sums
+// with one atomic per class among the warp's lanes (shared 64-bit atomics of
+// 256 threads on a handful of classes took 17 of the kernel's 22 us for
+// 20,000 pairs).  Called by the lanes of `act`.
+__device__ __forceinline__ int tally_pair(const BinParams& bp, const PairDesc& d, int flag, ClassSums* s_sum,
+                                          unsigned act) {
+  float cost = 0.f;
+  const int key = pair_key(bp, d.a_len, d.b_len, flag, thread_cap(bp), &cost);
+  const unsigned same = __match_any_sync(act, key / NBUCKET);
+  const unsigned cells = (unsigned)d.a_len * (unsigned)d.b_len;  // < 2^32: lengths below 65536
+  const unsigned ps = (unsigned)fminf(fmaxf(cost, 1.f), 4.0e9f);
+  // Sums in 16-bit halves, which 32 lanes cannot carry out of 32 bits.
+  const unsigned c0 = __reduce_add_sync(same, cells & 0xffffu), c1 = __reduce_add_sync(same, cells >> 16);
+  const unsigned p0 = __reduce_add_sync(same, ps & 0xffffu), p1 = __reduce_add_sync(same, ps >> 16);
+  if ((int)(threadIdx.x & 31) == __ffs(same) - 1) {
+    ClassSums& s = s_sum[key / NBUCKET];
+    atomicAdd(&s.cells, ((unsigned long long)c1 << 16) + c0);
+    atomicAdd(&s.cost, ((unsigned long long)p1 << 16) + p0);
+    atomicAdd(&s.count, __popc(same));
   }
+  return key;
+}
+
+// Zero result of a pair that is not listed (empty, too long or outside the
+// code array).
+__device__ __forceinline__ void reject_pair(int state, long p, DevStatus* st, int* score, int* arange, int* brange) {
+  report_pair(state, st);
+  score[p] = 0;
+  arange[p] = 0;
+  brange[p] = 0;
+}
+
+static __global__ void k_bin_count(BinParams bp, const PairDesc* __restrict__ pairs, int n, int* hist,
+                                   uint8_t* s32_flag, ClassSums* sums, DevStatus* st, int* score, int* arange,
+                                   int* brange) {
+  __shared__ ClassSums s_sum[NCLASS_MAX];
+  for (int k = threadIdx.x; k < NCLASS_MAX; k += blockDim.x) s_sum[k] = ClassSums{0, 0, 0, 0};
   __syncthreads();
   for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
     const PairDesc d = pairs[p];
     const int state = pair_state(d, bp.n_codes, bp.max_a, bp.max_b);
     if (state != PAIR_OK) {
-      // Empty, too long or outside the code array: zero result, not listed.
-      report_pair(state, st);
-      score[p] = 0;
-      arange[p] = 0;
-      brange[p] = 0;
+      reject_pair(state, p, st, score, arange, brange);
       continue;
     }
     // Candidates (both sequences longer than s16_max_len) got their flag
     // from k_bin_bound.
-    bool s32 = false;
-    if (bound_candidate(bp, d)) s32 = s32_flag[p] != 0;
-    s32_flag[p] = s32 ? 1 : 0;
-    float cost = 0.f;
-    const int key = pair_key(bp, d.a_len, d.b_len, s32, thread_cap(bp), &cost);
+    int flag = 0;
+    if (bound_candidate(bp, d)) flag = s32_flag[p];
+    s32_flag[p] = (uint8_t)flag;
+    const unsigned act = __activemask();
+    const int key = tally_pair(bp, d, flag, s_sum, act);
     // One histogram update per distinct key among the warp's lanes.
-    const unsigned same = __match_any_sync(__activemask(), key);
+    const unsigned same = __match_any_sync(act, key);
     if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[key], __popc(same));
-    atomicAdd(&s_cells[key / NBUCKET], (unsigned long long)d.a_len * (unsigned long long)d.b_len);
-    atomicAdd(&s_cost[key / NBUCKET], (unsigned long long)fmaxf(cost, 1.f));
   }
   __syncthreads();
   for (int k = threadIdx.x; k < bp.nclass; k += blockDim.x) {
-    if (s_cells[k]) atomicAdd(&class_cells[k], s_cells[k]);
-    if (s_cost[k]) atomicAdd(&class_cost[k], s_cost[k]);
+    if (!s_sum[k].count) continue;
+    atomicAdd(&sums[k].cells, s_sum[k].cells);
+    atomicAdd(&sums[k].cost, s_sum[k].cost);
+    atomicAdd(&sums[k].count, s_sum[k].count);
   }
 }
 
-__device__ __forceinline__ int run_total(const int* hist, const int* offs, int nkeys) {
-  return offs[nkeys - 1] + hist[nkeys - 1];
+// One warp: the {start, count} list range of every class, and its block
+// share -- sequential launches each take the whole GPU; concurrent ones
+// split it by modelled cost, scratch regions laid end to end.
+__device__ __forceinline__ void allot_classes(const BinParams& bp, const ClassSums* sums, int* class_range,
+                                              ClassAllot* allot, DevStatus* st) {
+  static_assert(NCLASS_MAX <= 32, "a lane per class");
+  const int c = threadIdx.x & 31;
+  const bool real = c < bp.nclass;
+  const int count = real ? sums[c].count : 0;
+  const double cost = count > 0 ? (double)sums[c].cost : 0.0;
+  int start = count;  // inclusive prefix, then exclusive
+  double total = cost;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int y = __shfl_up_sync(FULL, start, off);
+    if (c >= off) start += y;
+    total += __shfl_xor_sync(FULL, total, off);
+  }
+  start -= count;
+  int blocks = count > 0 ? bp.grid[c] : 0;
+  if (count > 0 && bp.concurrent == 1 && total > 0.0)
+    blocks = min(bp.grid[c], max(1, (int)ceil(cost / total * bp.grid[c])));
+  const long long need = real ? (long long)blocks * bp.scr_per_block[c] : 0;
+  long long base = need;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long y = __shfl_up_sync(FULL, base, off);
+    if (c >= off) base += y;
+  }
+  base -= need;
+  if (real) {
+    base = bp.concurrent == 1 ? base : bp.concurrent == 2 ? bp.slot_of[c] * bp.region : 0;
+    if (base + need > bp.scr_cap) {
+      // Never reached when the host sized the scratch for these shares.
+      if (bp.scr_per_block[c] > 0) blocks = (int)max(0ll, (bp.scr_cap - base) / bp.scr_per_block[c]);
+      if (blocks == 0 && count > 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
+    }
+    class_range[2 * c] = start;
+    class_range[2 * c + 1] = count;
+    allot[c].blocks = blocks;
+    allot[c].base = base;
+  }
+  if (c == 0) {
+    // The s32 rerun runs alone after every class: the whole GPU, base 0.
+    allot[bp.nclass].blocks = bp.grid[bp.cls_s32];
+    allot[bp.nclass].base = 0;
+  }
 }
 
-// Single block (blockDim.x a multiple of 32): exclusive scan of the
-// histogram into `offs`, and per class the {start, count} range consumed by
-// k_batched.  The keys go tile by tile (blockDim.x keys, coalesced, kTiles
-// tiles of loads in flight), each tile scanned across the block and offset
-// by the running total of the tiles before.
-static __global__ void k_bin_scan(BinParams bp, int nkeys, const int* hist, int* offs, int* class_range,
-                                  const unsigned long long* class_cost, ClassAllot* allot, DevStatus* st) {
-  constexpr int kTiles = 8;
+// Block c (1024 threads): exclusive scan of class c's part of the histogram
+// into `offs`, from the class's list start; block 0 also writes the ranges
+// and shares of all classes.  A block per class: one block over all keys,
+// tile after tile, took 53 us.
+static __global__ void k_bin_scan(BinParams bp, const int* hist, int* offs, const ClassSums* sums, int* class_range,
+                                  ClassAllot* allot, DevStatus* st) {
+  constexpr int PER = NBUCKET / 1024;
+  static_assert(PER == 4, "a 16-byte load per thread");
   __shared__ int s_warp[32];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  int carry = 0;
-  for (int base = 0; base < nkeys; base += kTiles * blockDim.x) {
-    int v[kTiles];
+  const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (c == 0 && wid == 0) allot_classes(bp, sums, class_range, allot, st);
+  if (sums[c].count == 0) return;
+  int start = lane < c ? sums[lane].count : 0;  // pairs of the classes before
+  start = __reduce_add_sync(FULL, start);
+  const int4 v = reinterpret_cast<const int4*>(hist + c * NBUCKET)[tid];
+  const int own = v.x + v.y + v.z + v.w;
+  int x = own;
 #pragma unroll
-    for (int j = 0; j < kTiles; ++j) {
-      const int k = base + j * blockDim.x + tid;
-      v[j] = k < nkeys ? hist[k] : 0;
-    }
-#pragma unroll
-    for (int j = 0; j < kTiles; ++j) {
-      int x = v[j];  // inclusive prefix within the warp
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(FULL, x, off);
-        if (lane >= off) x += y;
-      }
-      if (lane == 31) s_warp[wid] = x;
-      __syncthreads();
-      if (wid == 0) {
-        int w = lane < nw ? s_warp[lane] : 0;  // inclusive prefix of the warp totals
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const int y = __shfl_up_sync(FULL, w, off);
-          if (lane >= off) w += y;
-        }
-        if (lane < nw) s_warp[lane] = w;
-      }
-      __syncthreads();
-      const int k = base + j * blockDim.x + tid;
-      if (k < nkeys) offs[k] = carry + (wid > 0 ? s_warp[wid - 1] : 0) + x - v[j];
-      carry += s_warp[nw - 1];
-      __syncthreads();  // s_warp is rewritten by the next tile
-    }
+  for (int off = 1; off < 32; off <<= 1) {
+    const int y = __shfl_up_sync(FULL, x, off);
+    if (lane >= off) x += y;
   }
-  if (tid < nkeys / NBUCKET) {
-    const int c = tid;
-    class_range[2 * c] = offs[c * NBUCKET];
-    class_range[2 * c + 1] = ((c + 1) * NBUCKET < nkeys ? offs[(c + 1) * NBUCKET] : run_total(hist, offs, nkeys)) -
-                             offs[c * NBUCKET];
+  if (lane == 31) s_warp[wid] = x;
+  __syncthreads();
+  const int before = __reduce_add_sync(FULL, lane < wid ? s_warp[lane] : 0);
+  int4 o;
+  o.x = start + before + x - own;
+  o.y = o.x + v.x;
+  o.z = o.y + v.y;
+  o.w = o.z + v.z;
+  reinterpret_cast<int4*>(offs + c * NBUCKET)[tid] = o;
+}
+
+// The whole pre-pass of a batch of at most kSmallBin pairs in one block:
+// batch cells, keys, class sums and the list, sorted by key in shared memory
+// (bitonic).  Four launches and their 110,000-key histogram took 85 us for
+// 64 pairs, this 9.  s32_flag as in k_bin_count.
+constexpr int kSmallBin = 4096;
+static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const PairDesc* __restrict__ pairs, int n,
+                                                           const uint8_t* s32_flag, unsigned long long* total,
+                                                           ClassSums* sums, int* class_range, ClassAllot* allot,
+                                                           DevStatus* st, int* list, int* score, int* arange,
+                                                           int* brange) {
+  __shared__ unsigned long long s_key[kSmallBin];  // key << 32 | pair; rejected pairs and padding last
+  __shared__ ClassSums s_sum[NCLASS_MAX];
+  const int tid = threadIdx.x;
+  if (tid < NCLASS_MAX) s_sum[tid] = ClassSums{0, 0, 0, 0};
+  __syncthreads();
+  unsigned long long local = 0;
+  for (int p = tid; p < n; p += 1024) {
+    const PairDesc d = pairs[p];
+    if (pair_state(d, bp.n_codes, bp.max_a, bp.max_b) == PAIR_OK)
+      local += (unsigned long long)d.a_len * (unsigned long long)d.b_len;
+  }
+  for (int off = 16; off > 0; off >>= 1) local += __shfl_xor_sync(FULL, local, off);
+  if ((tid & 31) == 0 && local) atomicAdd(total, local);  // bp.total_cells, cleared before the run
+  __threadfence();
+  __syncthreads();
+  int m = 32;  // entries sorted: the power of two that holds n
+  while (m < n) m <<= 1;
+  for (int p = tid; p < m; p += 1024) {
+    unsigned long long e = ~0ull;
+    if (p < n) {
+      const PairDesc d = pairs[p];
+      const int state = pair_state(d, bp.n_codes, bp.max_a, bp.max_b);
+      if (state != PAIR_OK) {
+        reject_pair(state, p, st, score, arange, brange);
+      } else {
+        const int flag = bound_candidate(bp, d) ? s32_flag[p] : 0;
+        const int key = tally_pair(bp, d, flag, s_sum, __activemask());
+        e = ((unsigned long long)key << 32) | (unsigned)p;
+      }
+    }
+    s_key[p] = e;
   }
   __syncthreads();
-  if (tid == 0) {
-    // Block shares: sequential launches each take the whole GPU; concurrent
-    // ones split it by modelled cost, scratch regions laid end to end.
-    const int nc = nkeys / NBUCKET;
-    double total = 0.0;
-    for (int c = 0; c < nc; ++c)
-      if (class_range[2 * c + 1] > 0) total += (double)class_cost[c];
-    long long base = 0;
-    for (int c = 0; c < nc; ++c) {
-      int blocks = 0;
-      if (class_range[2 * c + 1] > 0) {
-        blocks = bp.grid[c];
-        if (bp.concurrent == 1 && total > 0.0)
-          blocks = min(bp.grid[c], max(1, (int)ceil((double)class_cost[c] / total * bp.grid[c])));
+  for (int k = 2; k <= m; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = tid; i < m / 2; i += 1024) {
+        const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), hi = lo + j;
+        const unsigned long long a = s_key[lo], b = s_key[hi];
+        if ((a > b) == ((lo & k) == 0)) {
+          s_key[lo] = b;
+          s_key[hi] = a;
+        }
       }
-      const long long start = bp.concurrent == 1 ? base : bp.concurrent == 2 ? bp.slot_of[c] * bp.region : 0;
-      const long long need = (long long)blocks * bp.scr_per_block[c];
-      if (start + need > bp.scr_cap) {
-        // Never reached when the host sized the scratch for these shares.
-        blocks = bp.scr_per_block[c] > 0 ? (int)max(0ll, (bp.scr_cap - start) / bp.scr_per_block[c]) : blocks;
-        if (blocks == 0 && class_range[2 * c + 1] > 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
-      }
-      allot[c].blocks = blocks;
-      allot[c].base = start;
-      if (bp.concurrent == 1) base += (long long)blocks * bp.scr_per_block[c];
+      __syncthreads();
     }
-    // The s32 rerun runs alone after every class: the whole GPU, base 0.
-    allot[nc].blocks = bp.grid[bp.cls_s32];
-    allot[nc].base = 0;
-  }
+  for (int p = tid; p < n; p += 1024)
+    if (s_key[p] != ~0ull) list[p] = (int)(unsigned)s_key[p];
+  if (tid < bp.nclass) sums[tid] = s_sum[tid];
+  if (tid < 32) allot_classes(bp, s_sum, class_range, allot, st);
 }
 
 static __global__ void k_bin_scatter(BinParams bp, const PairDesc* __restrict__ pairs, int n,
@@ -1148,7 +1298,7 @@ static __global__ void k_bin_scatter(BinParams bp, const PairDesc* __restrict__ 
   for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
     const PairDesc d = pairs[p];
     if (pair_state(d, bp.n_codes, bp.max_a, bp.max_b) != PAIR_OK) continue;
-    const int key = pair_key(bp, d.a_len, d.b_len, s32_flag[p] != 0, thread_cap(bp));
+    const int key = pair_key(bp, d.a_len, d.b_len, s32_flag[p], thread_cap(bp));
     // One atomic per distinct key among the warp's lanes; each lane takes
     // the slot of its rank in the group.
     const unsigned act = __activemask();

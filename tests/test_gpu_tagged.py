@@ -92,3 +92,47 @@ def test_scores_around_the_tag_limit(scoring, tile_k, lengths):
         _same(got, want, "%s tile_k %d fwd %s" % (scoring, tile_k, fwd))
         if tile_k:
             assert st.overflow_reruns >= 1
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1025, 4095, 4096, 4097])
+def test_list_of_a_small_batch(n):
+    """The one-block pre-pass (up to 4,096 pairs) and the histogram one:
+    every pair gets its own result, empty pairs zero, whatever their order."""
+    rng = np.random.default_rng(903)
+    codes, a_off, a_len, b_off, b_len = _pairs_at_edges(rng, 120)
+    k = rng.integers(0, 120, n)
+    pairs = ib.make_pairs(a_off[k], a_len[k], b_off[k], b_len[k])
+    empty = rng.random(n) < 0.05
+    pairs["b_len"][empty] = 0
+    gi, ge, match, mismatch = SCORINGS["affine"]
+    sim = oracle.select_matrix("na", match, mismatch, mismatch)
+    want = oracle.sw_batch(codes, a_off, a_len, b_off, b_len, sim, gi, ge, forward_only=False)
+    got, _ = _run("affine", False, codes, pairs, 8)
+    _same(got, [np.where(empty, 0, w[k]) for w in want], "n %d" % n)
+
+
+@pytest.mark.parametrize("n,team_warps", [(3, 8), (40, 8), (40, 6), (40, 0)])
+def test_high_scores_in_teams(n, team_warps):
+    """Near-identical proteins scoring above int16: strip teams of biased
+    halves (one, two or four teams a block), or one warp each."""
+    rng = np.random.default_rng(904)
+    a_list = [rng.integers(0, 20, int(la)).astype(np.uint8) for la in rng.integers(6600, 7400, n)]
+    b_list = []
+    for a in a_list:
+        b = a.copy()
+        at = rng.integers(0, a.size, 20)
+        b[at] = rng.integers(0, 20, 20)
+        b_list.append(b)
+    codes, a_off, a_len, b_off, b_len = oracle.pack_pairs(a_list, b_list)
+    pairs = ib.make_pairs(a_off, a_len, b_off, b_len)
+    for fwd in (True, False):
+        with ib.Engine(ib.sw_config(-10, -1, similarity="blosum62", datatype="aa"),
+                       ib.algo_config(forward_only=fwd)) as e:
+            e.set_option("team_warps", team_warps)
+            got = e.compare(codes, pairs)
+            st = e.stats()
+        want = oracle.sw_batch(codes, a_off, a_len, b_off, b_len, oracle.select_matrix("blosum62"), -10, -1,
+                               forward_only=fwd)
+        assert want[0].min() > 32767
+        _same(got, want, "n %d warps %d fwd %s" % (n, team_warps, fwd))
+        assert st.overflow_reruns == 0 and st.s32_pairs == n
