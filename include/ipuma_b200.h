@@ -187,6 +187,10 @@ typedef struct ipuma_stats {
 #define IPUMA_KERNEL_S16_TEAM 27   /* s16x2, 512-column strips shared by a team of warps (one block per
                                       two pairs; long pairs of small batches) */
 
+/* whole-warp strips of 256 and 128 columns (small batches) */
+#define IPUMA_KERNEL_S16_L32_K8 28
+#define IPUMA_KERNEL_S16_L32_K4 29
+
 typedef struct ipuma_engine ipuma_engine;
 
 /* ---- library ------------------------------------------------------------ */
@@ -236,15 +240,12 @@ void ipuma_gpu_destroy(ipuma_engine* e);
  *                 IPUMA_KERNEL_S16_L16_K5, _K7, _K9, _K11, _K13, _K15,
  *                 17 .. 21 = IPUMA_KERNEL_S16_L8_K8, _K10, _K12, _K14, _K16,
  *                 24 = every pair through strip teams (IPUMA_KERNEL_S16_TEAM)
- *   "concurrent"  3 = by batch size (default): mode 1 below 48,000 pairs,
- *                 mode 2 above; 2 = class launches alternate between two
- *                 streams, so each starts on the SMs the previous one
- *                 frees; 1 = all classes at once, each on a share of the
- *                 SMs proportional to its modelled work; 0 = one launch
- *                 after the other (always the case with time_launches)
- *   "latency_share" share of the batch's modelled time (per mille,
- *                 default 250) one pair's item may take in its class; a
- *                 pair over it takes a class that finishes it sooner
+ *   "concurrent"  0 = one launch after the other (always the case with
+ *                 time_launches); 1, 2, 3 (default) = the launches of long
+ *                 pairs and of the other classes share the GPU on streams
+ *   "latency_share" weight of a pair's own latency beside the modelled
+ *                 time of a batch of such pairs when its class is chosen
+ *                 (per mille, default 1500)
  *   "hybrid"      1 = pairs whose score can pass int16 run their strips
  *                 in biased 16-bit halves while a strip's values provably
  *                 fit, then in s32 (IPUMA_KERNEL_S16_HYBRID, default);

@@ -20,6 +20,7 @@
 
 #include "errors.h"
 #include "ipuma_b200.h"
+#include "class_mix.cuh"
 #include "sw_kernels.cuh"
 #include "sw_thread.cuh"
 #include "../host/swatlib/encoding.h"
@@ -97,7 +98,7 @@ struct ClassDef {
   int lanes, k, kind, width;
 };
 constexpr int kNumS16 = 21;     // s16x2 classes chosen by cost
-constexpr int kNumClasses = kNumS16 + 6;  // + the s32, hybrid, strip-team, long, big and big strip-team classes
+constexpr int kNumClasses = kNumS16 + 8;  // + the s32, hybrid, strip-team, long, big, big strip-team and two narrow classes
 constexpr ClassDef kClasses[kNumClasses] = {
     {16, 4, IPUMA_KERNEL_S16_L16_K4, 64},    {16, 8, IPUMA_KERNEL_S16_L16_K8, 128},
     {16, 12, IPUMA_KERNEL_S16_L16_K12, 192}, {16, 16, IPUMA_KERNEL_S16_L16_K16, 256},
@@ -113,6 +114,7 @@ constexpr ClassDef kClasses[kNumClasses] = {
     {32, 16, IPUMA_KERNEL_S32_K16, 512},     {32, 16, IPUMA_KERNEL_S16_HYBRID, 512},
     {32, 16, IPUMA_KERNEL_S16_TEAM, 512},    {32, 16, IPUMA_KERNEL_S16_L32_K16, 512},
     {32, 16, IPUMA_KERNEL_S16_HYBRID, 512},  {32, 16, IPUMA_KERNEL_S16_TEAM, 512},
+    {32, 8, IPUMA_KERNEL_S16_L32_K8, 256},   {32, 4, IPUMA_KERNEL_S16_L32_K4, 128},
 };
 static_assert(kNumClasses <= NCLASS_MAX, "class tables");
 constexpr int kClsWidest = 5;  // widest wavefront class (very long |A|)
@@ -138,35 +140,20 @@ constexpr int kClsLong = kNumS16 + 3;
 // whose diagonal passes even that go to the hybrid class.
 constexpr int kClsBig = kNumS16 + 4;
 constexpr int kClsBigTeam = kNumS16 + 5;
+// Whole-warp strips of 256 and 128 columns: a step of few columns is over
+// soonest, which is what counts when the batch leaves warps without work.
+constexpr int kClsLat256 = kNumS16 + 6, kClsLat128 = kNumS16 + 7;
+constexpr unsigned kLatClasses = (1u << kClsLat256) | (1u << kClsLat128);
 // Per-thread class: rows it accepts (its boundary scratch is rows x threads)
 // and the share of the batch's time one of its pairs may take.
 constexpr int kThrMaxRows = 2048;
 constexpr float kThrLatencyShare = 0.5f;
-// Latency bound of every class (BinParams::lat_share): an item may take at
-// most this share of the batch's modelled time (cells x fastest slot time
-// / packing efficiency).  In small batches that sends pairs to the class
-// that finishes them soonest: there one long pair, not throughput, sets the
-// batch's time.
-// (B200, 300,000 DNA pairs with start coordinates: 7.07 ms at 0.06, 4.93 at
-// 0.25, 4.90 at 0.5; 200,000 protein pairs 11.0, 11.7 and 11.9 ms.)
-constexpr float kLatencyShare = 0.25f;
+// Weight of a pair's own latency beside the modelled time of a batch of such
+// pairs (pair_key): in a small batch it sends pairs to the class that
+// finishes them soonest, in a large one it counts for the longest only.
+constexpr float kLatencyWeight = 1.5f;
 constexpr float kPackingEfficiency = 0.85f;
-constexpr float kLatencyMinBatchPs = 0.f;
-// Option "concurrent" = 3 (default) picks the launch mode by batch size:
-// smaller batches leave most class launches with fewer items than resident
-// warps, so the classes share the SMs (mode 1); larger ones alternate two
-// streams (mode 2), which keeps one class per SM.
-constexpr int kShareModeMaxPairs = 48000;
-// The 16-lane classes at 16-column steps (every K from 4 to 16) cut column
-// padding on large batches; a smaller batch uses the 64-column steps only
-// (K = 4, 8, 12, 16), since every class launch costs a few microseconds
-// even when empty.
-constexpr int kFineClassMinPairs = 150000;
-// 8-lane groups of linear-gap strips (strip_ref) from this many pairs: an
-// item holds eight pairs instead of four, which leaves warps without work
-// in smaller batches (10,000 pairs of 150 x 150-300 on B200: 329 us with 8
-// lanes, 250 with 16; 69,000 of 100-200 x 100-200: 1.07 against 0.91 ms).
-constexpr int kEightLaneMinPairs = 150000;
+// Classes at 64-column steps; the ones between are added below.
 constexpr unsigned kCoarseClasses = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 5);
 // 8-lane groups for the five narrowest strip widths (64 to 128 columns):
 // twice the columns per lane over a wavefront half as deep, so the per-step
@@ -180,6 +167,21 @@ constexpr int kNarrowPairs[5][2] = {{0, 16}, {10, 17}, {7, 18}, {11, 19}, {1, 20
 constexpr unsigned kFineClasses = (1u << 7) | (1u << 8) | (1u << 9) | (1u << 10) | (1u << 11) | (1u << 12) |
                                   (1u << 13) | (1u << 14) | (1u << 15);
 constexpr int kWarpsPerBlock = 4;
+// 8-lane groups of linear-gap strips (kMixLin8) from this many pairs: an
+// item holds eight pairs instead of four, which leaves warps without work
+// in smaller batches (10,000 pairs of 150 x 150-300 on B200: 329 us with 8
+// lanes, 250 with 16; 69,000 of 100-200 x 100-200: 1.07 against 0.91 ms).
+constexpr int kEightLaneMinPairs = 150000;
+// Batches below this size may use the latency classes.
+constexpr int kLatClassMaxPairs = 20000;
+// One step (row) of a warp item of k columns a lane: `full` ps when the GPU
+// is full, less when the batch's items leave schedulers with one warp --
+// down to that warp's own latency, about 60 + 11 k cycles.
+float step_time(float full, int k, int n, int grid) {
+  const float alone = (60.f + 11.f * (float)k) * 520.f;
+  const float fill = std::min(1.f, (float)n / (2.f * (float)std::max(1, grid * kWarpsPerBlock)));
+  return std::min(full, alone) + std::max(0.f, full - alone) * fill;
+}
 // Chunked upload/compute overlap of ipuma_gpu_compare.
 constexpr int kMaxChunks = 8;
 constexpr int kChunkMinPairs = 250000;        // automatic chunking from 2 x this many pairs
@@ -277,7 +279,7 @@ struct ipuma_engine {
   cudaEvent_t join_ev[NCLASS_MAX] = {};
   int concurrent = 3;
   int hybrid = 1;  // option "hybrid": high-scoring pairs run s16x2 strips while provably safe
-  float latency_share = kLatencyShare;  // option "latency_share" (per mille)
+  float latency_weight = kLatencyWeight;  // option "latency_share" (per mille)
   cudaStream_t stream2 = nullptr, copy_stream = nullptr;
   cudaEvent_t cev[2 * kMaxChunks + 2] = {};
   int chunks = 0;  // option "chunks": 0 automatic, 1 off, n fixed
@@ -378,14 +380,18 @@ int smem_for(const ipuma_engine* e, int P = -1) {
   return SmemLayout<T, K, LANES>::total(e->M, P < 0 ? e->M : P, kWarpsPerBlock);
 }
 
-// The k_batched instantiation a class launches (all share one signature).
+// How a class runs: in k_mix with the other classes of its model, or in a
+// k_batched launch of its own (all instantiations share one signature).
 using BatchedKernel = decltype(&k_batched<LaneS32, 16, 32>);
 struct KernelRef {
-  BatchedKernel fn = nullptr;  // null: the class has no kernel for this scoring
-  int lanes = 0, k = 0, smem = 0;
+  bool mix = false;
+  BatchedKernel fn = nullptr;
+  int lanes = 0, k = 0;        // 0 lanes: the class has no kernel for this scoring
+  int warp_bytes = 0;          // shared memory per warp, without the table
   int buffers = 2;             // strip-boundary columns per lane group
   int shift = 0;               // bits the lanes hold scores shifted by
   int limit = 0;               // largest score the lanes may hold
+  bool ok() const { return lanes > 0; }
 };
 
 template <class T, int K, int LANES, bool HYB = false>
@@ -394,85 +400,123 @@ KernelRef kernel_ref(const ipuma_engine* e, int P) {
   r.fn = e->sc.forwardOnly ? k_batched<T, K, LANES, HYB, true> : k_batched<T, K, LANES, HYB, false>;
   r.lanes = LANES;
   r.k = K;
-  r.smem = smem_for<T, K, LANES>(e, P);
+  r.warp_bytes = SmemLayout<T, K, LANES>::warp_bytes(P);
   r.buffers = HYB ? 3 : 2;
   r.shift = kProfShift<T>;
   r.limit = Cell<T>::limit(e->sc);
   return r;
 }
 
-// Lanes of the 16-bit classes.  Linear gaps keep four tag bits (2,047
-// points), which fit every pair their strips are meant for; affine scorings,
-// proteins mostly, keep two (8,191 points) so that only very long or
-// near-identical pairs need the long class, whose lanes hold 16 bits.
-// Matrices whose scaled values pass a profile byte run unscaled.
-using LaneLin = LaneTag<4, true, true>;
-using LaneAff = LaneTag<2, false, true>;
-using LaneAny = LaneTag<2, false, false>;
+// One tag bit: the long class and the strip teams.
 using LaneLinLong = LaneTag<1, true, false>;
 using LaneAffLong = LaneTag<1, false, false>;
 
-// Strips of 16 * K columns: 16 lanes of K, or 8 lanes of 2 K with the
-// four-row profile, whose shared memory then allows it (measured on B200,
-// 60,000 pairs of 240 x 320, linear gaps: 16 lanes 6488, 8 lanes 7061
-// GCUPS -- a lane's work per step covers twice the cells).  Affine lanes of
-// more than 24 columns spill; they stay at 16.
-template <int K>
-KernelRef strip_ref(const ipuma_engine* e, int P, bool eight) {
-  if (e->cells == ipuma_engine::kLinear)
-    return P < e->M && eight ? kernel_ref<LaneLin, 2 * K, 8>(e, P) : kernel_ref<LaneLin, K, 16>(e, P);
-  if (e->cells == ipuma_engine::kAffine) return kernel_ref<LaneAff, K, 16>(e, P);
-  if constexpr (K % 4 == 0) return kernel_ref<LaneAny, K, 16>(e, P);
-  return KernelRef{};
-}
-template <int K>
-KernelRef narrow_ref(const ipuma_engine* e, int P) {
-  if (e->cells == ipuma_engine::kLinear) return kernel_ref<LaneLin, K, 8>(e, P);
-  if (e->cells == ipuma_engine::kAffine) return kernel_ref<LaneAff, K, 8>(e, P);
-  return KernelRef{};
-}
-template <int K>
-KernelRef wide_ref(const ipuma_engine* e, int P) {
-  if (e->cells == ipuma_engine::kLinear) return kernel_ref<LaneLin, K, 32>(e, P);
-  if (e->cells == ipuma_engine::kAffine) return kernel_ref<LaneAff, K, 32>(e, P);
-  return kernel_ref<LaneAny, K, 32>(e, P);
+// Model of the batch's 16-bit classes (eight: the batch fills 8-lane
+// groups of linear-gap strips, whose profiles need the four-row alphabet).
+int mix_model(const ipuma_engine* e, int P, bool eight) {
+  if (e->cells == ipuma_engine::kLinear) return P < e->M && eight ? kSepLin8 : kMixLin;
+  if (e->cells == ipuma_engine::kAnyScore) return kMixAny;
+  return P > 16 ? kMixProt : kMixAff;
 }
 
-// Kernel of a wavefront class for a P-letter profile (not the per-thread
-// and the team class); eight: the batch fills 8-lane groups.
-KernelRef kernel_of(const ipuma_engine* e, int cls, int P, bool eight) {
+MixKernel mix_kernel_of(int model, bool fwd) {
+  switch (model) {
+    case kMixLin: return fwd ? mix_kernel<kMixLin, true>() : mix_kernel<kMixLin, false>();
+    case kMixAff: return fwd ? mix_kernel<kMixAff, true>() : mix_kernel<kMixAff, false>();
+    case kMixProt: return fwd ? mix_kernel<kMixProt, true>() : mix_kernel<kMixProt, false>();
+    default: return fwd ? mix_kernel<kMixAny, true>() : mix_kernel<kMixAny, false>();
+  }
+}
+
+// Class kernel of kSepLin8: strips of 16 * K columns.
+template <int CLS>
+KernelRef sep_ref(const ipuma_engine* e, int P) {
+  constexpr MixShape sh = mix_shape(kSepLin8, CLS);
+  return kernel_ref<LaneLin, sh.k, sh.lanes>(e, P);
+}
+KernelRef sep_kernel(const ipuma_engine* e, int cls, int P) {
   switch (cls) {
-    case 0: return strip_ref<4>(e, P, eight);
-    case 10: return strip_ref<5>(e, P, eight);
-    case 7: return strip_ref<6>(e, P, eight);
-    case 11: return strip_ref<7>(e, P, eight);
-    case 1: return strip_ref<8>(e, P, eight);
-    case 12: return strip_ref<9>(e, P, eight);
-    case 8: return strip_ref<10>(e, P, eight);
-    case 13: return strip_ref<11>(e, P, eight);
-    case 2: return strip_ref<12>(e, P, eight);
-    case 14: return strip_ref<13>(e, P, eight);
-    case 9: return strip_ref<14>(e, P, eight);
-    case 15: return strip_ref<15>(e, P, eight);
-    case 3: return strip_ref<16>(e, P, eight);
-    case 16: return narrow_ref<8>(e, P);
-    case 17: return narrow_ref<10>(e, P);
-    case 18: return narrow_ref<12>(e, P);
-    case 19: return narrow_ref<14>(e, P);
-    case 20: return narrow_ref<16>(e, P);
-    case 4: return wide_ref<12>(e, P);
-    case 5: return wide_ref<16>(e, P);
+    case 0: return sep_ref<0>(e, P);
+    case 1: return sep_ref<1>(e, P);
+    case 2: return sep_ref<2>(e, P);
+    case 3: return sep_ref<3>(e, P);
+    case 4: return sep_ref<4>(e, P);
+    case 5: return sep_ref<5>(e, P);
+    case 7: return sep_ref<7>(e, P);
+    case 8: return sep_ref<8>(e, P);
+    case 9: return sep_ref<9>(e, P);
+    case 10: return sep_ref<10>(e, P);
+    case 11: return sep_ref<11>(e, P);
+    case 12: return sep_ref<12>(e, P);
+    case 13: return sep_ref<13>(e, P);
+    case 14: return sep_ref<14>(e, P);
+    case 15: return sep_ref<15>(e, P);
+    default: return KernelRef{};
+  }
+}
+
+// Shared memory of a lane group's warp (SmemLayout::warp_bytes of two-pair
+// lanes, for a shape known at run time).
+int mix_warp_bytes(const MixShape& sh, int P) {
+  const int kp = (sh.k + 3) / 4 * 4;
+  return 32 / sh.lanes * ((2 * (P + 1) * sh.lanes * kp + 512 + 15) & ~15);
+}
+
+// Kernel of a wavefront class for a P-letter profile in a model (not the
+// per-thread and the team classes).
+KernelRef kernel_of(const ipuma_engine* e, int cls, int P, int model) {
+  switch (cls) {
+    case kClsThread: case kClsTeam: case kClsBigTeam: return KernelRef{};
     case kClsLong:
       return e->cells == ipuma_engine::kLinear ? kernel_ref<LaneLinLong, 16, 32>(e, P)
                                                : kernel_ref<LaneAffLong, 16, 32>(e, P);
     case kClsBig: return kernel_ref<LaneBig, 16, 32>(e, P);
     case kClsHi: return kernel_ref<LaneHi, 16, 32, true>(e, P);
     case kClsS32: return kernel_ref<LaneS32, 16, 32>(e, P);
-    default: return KernelRef{};
+    default: break;
   }
+  if (model == kSepLin8) return sep_kernel(e, cls, P);
+  KernelRef r;
+  const MixShape sh = mix_shape(model, cls);
+  if (sh.lanes == 0) return r;
+  r.mix = true;
+  r.lanes = sh.lanes;
+  r.k = sh.k;
+  r.warp_bytes = mix_warp_bytes(sh, P);
+  const bool lin = e->cells == ipuma_engine::kLinear;
+  r.shift = lin ? kProfShift<LaneLin> : e->cells == ipuma_engine::kAffine ? kProfShift<LaneAff> : kProfShift<LaneAny>;
+  r.limit = lin ? LaneLin::limit(e->maxSub)
+                : e->cells == ipuma_engine::kAffine ? LaneAff::limit(e->maxSub) : LaneAny::limit(e->maxSub);
+  return r;
 }
 
-int kernel_grid(ipuma_engine* e, const KernelRef& r) { return r.fn ? occupancy_grid(e, r.fn, r.smem) : 0; }
+// Shared memory of a block of kWarpsPerBlock warps.
+int block_smem(const ipuma_engine* e, int P, int warp_bytes) {
+  return SubTable::bytes(e->M, P) + kWarpsPerBlock * warp_bytes;
+}
+
+int kernel_grid(ipuma_engine* e, const KernelRef& r, int P, int model) {
+  if (!r.ok()) return 0;
+  const int smem = block_smem(e, P, r.warp_bytes);
+  return r.mix ? occupancy_grid(e, mix_kernel_of(model, e->sc.forwardOnly), smem) : occupancy_grid(e, r.fn, smem);
+}
+
+// Launch order of the classes: the long tails first, then k_mix's by strip
+// width.
+constexpr int kLaunchOrder[kNumClasses] = {26, 23, 25, 22, 24, 21, 6, 5,  4,  3,  27, 15, 9, 14, 2,
+                                           13, 8,  12, 1,  20, 28, 11, 19, 7, 18, 10, 17, 0, 16};
+
+// The classes of `mask` that k_mix runs, for one launch.
+MixArgs mix_args(const KernelRef* kr, unsigned mask, long rowsCap) {
+  MixArgs ma{};
+  for (int c = 0; c < kNumClasses; ++c) {
+    if (!((mask >> c) & 1u) || !kr[c].mix) continue;
+    ma.mask |= 1u << c;
+    ma.warp_bytes = std::max(ma.warp_bytes, kr[c].warp_bytes);
+    ma.scr_per_warp = std::max<long>(ma.scr_per_warp, 32 / kr[c].lanes * kr[c].buffers * rowsCap);
+  }
+  return ma;
+}
 
 // Kernel of a strip-team class: linear gaps or affine with one tag bit, or
 // the big class's lanes.
@@ -532,8 +576,10 @@ long thread_threads(ipuma_engine* e) {
 // profile size.
 void warm_grids(ipuma_engine* e) {
   for (int P : {e->M, prof_letters(e, 2)}) {
-    for (int c = 0; c < kNumClasses; ++c)
-      for (bool eight : {false, true}) kernel_grid(e, kernel_of(e, c, P, eight));
+    for (bool eight : {false, true}) {
+      const int model = mix_model(e, P, eight);
+      for (int c = 0; c < kNumClasses; ++c) kernel_grid(e, kernel_of(e, c, P, model), P, model);
+    }
     for (int w = 2; w <= std::min(e->team_warps, kTeamMaxWarps); ++w)
       if (team_smem(e, P, w) + kTeamStaticSmem <= e->smem_optin)
         for (bool big : {false, true}) team_grid(e, P, w, big);
@@ -549,10 +595,9 @@ struct RunBufs {
   DevBuf* list;
   DevBuf* ovf;
   DevBuf* flag;
-  // First of the two class streams of alternating launches (0 or 2): a
-  // second buffer set runs its classes on streams of its own, so its
-  // launches fill the tails of a run on the first set instead of queueing
-  // behind them.
+  // First of the run's streams (0 or kRunStreams): a second buffer set runs
+  // its launches on streams of its own, so they fill the tails of a run on
+  // the first set instead of queueing behind them.
   int cls_base = 0;
 };
 
@@ -581,41 +626,66 @@ int timed_end(ipuma_engine* e, cudaStream_t s) {
   return IPUMA_OK;
 }
 
+// What every alignment launch of a run reads and writes.
+BatchIo batch_io(const RunBufs& rb, const uint8_t* codes, const PairDesc* pairs, long rowsCap, int* score, int* arange,
+                 int* brange) {
+  return BatchIo{codes,
+                 pairs,
+                 rowsCap,
+                 score,
+                 arange,
+                 brange,
+                 rb.ovf->as<int>(),
+                 reinterpret_cast<unsigned long long*>(rb.ctl + CTL_CELLS) + CELLS_RERUN,
+                 reinterpret_cast<DevStatus*>(rb.ctl + CTL_STATUS)};
+}
+
+unsigned long long* trace_of(const ipuma_engine* e, const RunBufs& rb) {
+  return e->trace ? reinterpret_cast<unsigned long long*>(rb.ctl + CTL_TRACE) : nullptr;
+}
+
 // allot_idx = entry of the control block's ClassAllot table (the class, or
 // NCLASS_MAX for the s32 rerun).
 int launch_batched(ipuma_engine* e, const KernelRef& kr, const SwConst& sc, const RunBufs& rb, cudaStream_t s,
-                   const uint8_t* codes, const PairDesc* pairs, const int* list, const int* range, int* head,
-                   long rowsCap, int* score, int* arange, int* brange, int kind, int cls, int allot_idx) {
-  const int grid = kernel_grid(e, kr);
-  int* ctl = rb.ctl;
-  auto* cells = reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS);
+                   const BatchIo& io, const int* list, const int* range, int* head, int kind, int cls,
+                   int allot_idx) {
+  const int grid = kernel_grid(e, kr, sc.P, 0);
   int rc;
   if ((rc = timed_begin(e, s, kind, cls))) return rc;
-  kr.fn<<<grid, kThreads, kr.smem, s>>>(
-      lane_const(sc, kr.shift), e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(),
-      rowsCap, score, arange, brange, rb.ovf->as<int>(), cells + CELLS_RERUN,
-      reinterpret_cast<DevStatus*>(ctl + CTL_STATUS),
-      reinterpret_cast<const ClassAllot*>(ctl + CTL_ALLOT) + allot_idx,
-      e->trace ? reinterpret_cast<unsigned long long*>(ctl + CTL_TRACE) + 2 * allot_idx : nullptr);
+  unsigned long long* trace = trace_of(e, rb);
+  kr.fn<<<grid, kThreads, block_smem(e, sc.P, kr.warp_bytes), s>>>(
+      lane_const(sc, kr.shift), e->d_sim.as<int8_t>(), io, list, range, head, rb.scratch->as<int2>(),
+      reinterpret_cast<const ClassAllot*>(rb.ctl + CTL_ALLOT) + allot_idx, trace ? trace + 2 * allot_idx : nullptr);
+  CUDA_TRY(cudaGetLastError());
+  return timed_end(e, s);
+}
+
+// The classes of `ma` in one launch (kind, cls: what a timed launch reports).
+int launch_mix(ipuma_engine* e, int model, int shift, const MixArgs& ma, const SwConst& sc, const RunBufs& rb,
+               cudaStream_t s, long long scratchBase, const BatchIo& io, const int* list, const int* ranges, int* heads,
+               int kind, int cls) {
+  const int smem = block_smem(e, sc.P, ma.warp_bytes);
+  const MixKernel fn = mix_kernel_of(model, e->sc.forwardOnly);
+  const int grid = occupancy_grid(e, fn, smem);
+  int rc;
+  if ((rc = timed_begin(e, s, kind, cls))) return rc;
+  fn<<<grid, kThreads, smem, s>>>(lane_const(sc, shift), ma, e->d_sim.as<int8_t>(), io, list, ranges, heads,
+                                  rb.scratch->as<int2>() + scratchBase, trace_of(e, rb));
   CUDA_TRY(cudaGetLastError());
   return timed_end(e, s);
 }
 
 // Launches a strip-team class (`warps` warps per block) over its list range.
-int launch_team(ipuma_engine* e, const SwConst& sc, const RunBufs& rb, cudaStream_t s, const uint8_t* codes,
-                const PairDesc* pairs, const int* list, const int* range, int* head, long rowsCap, int* score,
-                int* arange, int* brange, int warps, int cls) {
+int launch_team(ipuma_engine* e, const SwConst& sc, const RunBufs& rb, cudaStream_t s, const BatchIo& io,
+                const int* list, const int* range, int* head, int warps, int cls) {
   const int smem = team_smem(e, sc.P, warps);
   const int grid = team_grid(e, sc.P, warps, cls == kClsBigTeam);
-  int* ctl = rb.ctl;
-  auto* cells = reinterpret_cast<unsigned long long*>(ctl + CTL_CELLS);
   int rc;
   if ((rc = timed_begin(e, s, kClasses[cls].kind, cls))) return rc;
+  unsigned long long* trace = trace_of(e, rb);
   team_kernel(e, cls == kClsBigTeam)<<<grid, 32 * warps, smem, s>>>(
-      lane_const(sc, 0), e->d_sim.as<int8_t>(), codes, pairs, list, range, head, rb.scratch->as<int2>(), rowsCap, score, arange,
-      brange, rb.ovf->as<int>(), cells + CELLS_RERUN, reinterpret_cast<DevStatus*>(ctl + CTL_STATUS),
-      reinterpret_cast<const ClassAllot*>(ctl + CTL_ALLOT) + cls,
-      e->trace ? reinterpret_cast<unsigned long long*>(ctl + CTL_TRACE) + 2 * cls : nullptr);
+      lane_const(sc, 0), e->d_sim.as<int8_t>(), io, list, range, head, rb.scratch->as<int2>(),
+      reinterpret_cast<const ClassAllot*>(rb.ctl + CTL_ALLOT) + cls, trace ? trace + 2 * cls : nullptr);
   CUDA_TRY(cudaGetLastError());
   return timed_end(e, s);
 }
@@ -651,13 +721,15 @@ long thread_rows(const ipuma_engine* e, int maxA, int maxB) {
   return e->tile_k == kClsThread + 1 ? maxB : std::min(maxB, kThrMaxRows);
 }
 
-// Strip-boundary scratch (int2) of one run: the wavefront classes need two
-// columns of rowsCap per lane group, the per-thread class one column of
-// thread_rows per thread.
-// Full-occupancy grid and strip scratch (int2) per block of every class,
-// for a P-letter profile.
-void class_grids(ipuma_engine* e, int P, bool eight, int maxA, int maxB, int* grid, long long* spb) {
-  const long long rowsCap = std::max(1, maxB);
+// Full-occupancy grid and strip scratch (int2) per block of every class, for
+// a P-letter profile.  The classes k_mix runs share its launch: their entry
+// is that of a launch of all of them.
+void class_grids(ipuma_engine* e, int P, int model, const KernelRef* kr, unsigned mask, int maxA, int maxB, int* grid,
+                 long long* spb) {
+  const long rowsCap = std::max(1, maxB);
+  const MixArgs ma = mix_args(kr, mask, rowsCap);
+  const int mixGrid =
+      ma.mask ? occupancy_grid(e, mix_kernel_of(model, e->sc.forwardOnly), block_smem(e, P, ma.warp_bytes)) : 0;
   for (int c = 0; c < kNumClasses; ++c) {
     if (c == kClsTeam || c == kClsBigTeam) {
       const int w = team_warps_for(e, P, maxA);
@@ -666,45 +738,74 @@ void class_grids(ipuma_engine* e, int P, bool eight, int maxA, int maxB, int* gr
     } else if (c == kClsThread) {
       grid[c] = (int)(thread_threads<16>(e) / kThreads);
       spb[c] = (long long)kThreads * thread_rows(e, maxA, maxB);
+    } else if (kr[c].mix) {
+      grid[c] = mixGrid;
+      spb[c] = (long long)kWarpsPerBlock * ma.scr_per_warp;
     } else {
-      const KernelRef kr = kernel_of(e, c, P, eight);
-      grid[c] = kernel_grid(e, kr);
-      spb[c] = kr.fn ? (long long)kWarpsPerBlock * (32 / kr.lanes) * kr.buffers * rowsCap : 0;
+      grid[c] = kernel_grid(e, kr[c], P, model);
+      spb[c] = kr[c].ok() ? (long long)kWarpsPerBlock * (32 / kr[c].lanes) * kr[c].buffers * rowsCap : 0;
     }
   }
 }
 
-// Scratch for any split of the GPU between the classes: shares are
-// fractions f_c of each class's full grid with sum f_c = 1, rounded up.
-// With two alternating streams (option concurrent = 2) two full-grid
-// launches may run at once: two regions of the largest full grid.
-size_t scratch_int2(ipuma_engine* e, int maxA, int maxB) {
-  int grid[NCLASS_MAX + 1];
-  long long spb[NCLASS_MAX + 1];
-  long long full = 0, round = 0;
-  for (int P : {e->M, prof_letters(e, 2)})  // the smaller profile may fit more blocks
-    for (bool eight : {false, true}) {
-      class_grids(e, P, eight, maxA, maxB, grid, spb);
-      long long r = 0;
-      for (int c = 0; c < kNumClasses; ++c) {
-        full = std::max(full, (long long)grid[c] * spb[c]);
-        r += spb[c];
-      }
-      round = std::max(round, r);
-    }
-  return (size_t)std::max(full + round, 2 * full);
+// Classes a pair is given to by its modelled time (the others by its scores
+// or latency).
+bool by_cost_class(int c) { return c < kNumS16 || c == kClsLat256 || c == kClsLat128; }
+
+// Streams (and scratch regions) of a batch's launches.  The long pairs go
+// first: strip teams on the run's own stream 0, the other special classes on
+// stream 2, before k_mix (stream 1; stream 0 when no special class is
+// launched) fills what they leave.  Separate class launches alternate
+// between streams 1 and 3, so each starts on the SMs the one before frees.
+constexpr int kRunStreams = 4;
+void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
+  bool special = false;
+  for (int c = 0; c < kNumClasses; ++c) special |= ((enabled >> c) & 1u) && !by_cost_class(c);
+  int pos = 0;
+  for (const int c : kLaunchOrder) {
+    if (!by_cost_class(c))
+      slot[c] = c == kClsTeam || c == kClsBigTeam ? 0 : 2;
+    else if (kr[c].mix || c == kClsThread)
+      slot[c] = special ? 1 : 0;
+    else
+      slot[c] = ((enabled >> c) & 1u) && (pos++ & 1) ? 3 : special ? 1 : 0;
+  }
 }
 
-// Launch order of the classes (longest-tail classes first) and, for two
-// alternating streams, the stream (and scratch region) of each.
-// The hybrid class and the widest class (the long pairs of a heavy-tailed
-// batch) come first and land on different streams, so the widest class's
-// blocks start on the SMs the hybrid class frees during its tail.
-constexpr int kLaunchOrder[kNumClasses] = {26, 23, 25, 22, 24, 5, 21, 4, 6, 3, 15, 9, 14, 2, 13, 8, 12, 1, 20, 11, 19, 7, 18, 10, 17, 0, 16};
+// Strip-boundary scratch (int2) of one run: a region per stream, each as
+// large as any launch's full grid needs -- for the models and class sets a
+// batch of this shape may use.
+size_t scratch_int2(ipuma_engine* e, int n, int maxA, int maxB) {
+  int grid[NCLASS_MAX + 1];
+  long long spb[NCLASS_MAX + 1];
+  KernelRef kr[kNumClasses];
+  long long full = 0;
+  for (int P : {e->M, prof_letters(e, 2)})  // the smaller profile may fit more blocks
+    for (bool eight : {false, n >= kEightLaneMinPairs}) {
+      const int model = mix_model(e, P, eight);
+      for (int c = 0; c < kNumClasses; ++c) kr[c] = kernel_of(e, c, P, model);
+      // Launches of every class alone and of all: a launch of some classes
+      // lies between (fewer columns per warp and less shared memory than
+      // all, no more blocks than the smallest alone).
+      int blocks = 0;
+      long long per = 0;
+      for (int c = 0; c < kNumClasses; ++c) {
+        class_grids(e, P, model, kr, 1u << c, maxA, maxB, grid, spb);
+        if (kr[c].mix) {
+          blocks = std::max(blocks, grid[c]);
+          per = std::max(per, spb[c]);
+        } else {
+          full = std::max(full, (long long)grid[c] * spb[c]);
+        }
+      }
+      full = std::max(full, blocks * per);
+    }
+  return (size_t)(kRunStreams * full);
+}
 
 int reserve_bufs(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, int n, int maxA, int maxB) {
   int rc;
-  if ((rc = rb.scratch->ensure(sizeof(int2) * scratch_int2(e, maxA, maxB), s))) return rc;
+  if ((rc = rb.scratch->ensure(sizeof(int2) * scratch_int2(e, n, maxA, maxB), s))) return rc;
   if ((rc = rb.list->ensure(sizeof(int) * (size_t)n + 64, s))) return rc;
   if ((rc = rb.ovf->ensure(sizeof(int) * (size_t)n + 64, s))) return rc;
   if ((rc = rb.flag->ensure((size_t)n + 64, s))) return rc;
@@ -751,27 +852,27 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
 
   // Scratch for strip boundaries and the lists.
   const long rowsCap = std::max(1, maxB);
-  if ((rc = rb.scratch->ensure(sizeof(int2) * scratch_int2(e, maxA, maxB), s))) return rc;
+  if ((rc = rb.scratch->ensure(sizeof(int2) * scratch_int2(e, n, maxA, maxB), s))) return rc;
   if ((rc = rb.list->ensure(sizeof(int) * (size_t)n + 64, s))) return rc;
   if ((rc = rb.ovf->ensure(sizeof(int) * (size_t)n + 64, s))) return rc;
 
   BinParams bp{};
-  bp.n_s16_classes = kNumS16;
   bp.cls_s32 = kClsS32;
   bp.cls_hi = e->hybrid ? kClsHi : kClsS32;
   bp.cls_big = e->hybrid ? kClsBig : kClsS32;
   bp.nclass = kNumClasses;
   bp.force_s32 = e->s16_ok ? 0 : 1;
   const bool eight = n >= kEightLaneMinPairs;
+  const int model = mix_model(e, sc.P, eight);
   KernelRef kr[kNumClasses];
   for (int c = 0; c < kNumClasses; ++c) {
-    kr[c] = kernel_of(e, c, sc.P, eight);
-    bp.lanes[c] = kr[c].fn ? kr[c].lanes : kClasses[c].lanes;
+    kr[c] = kernel_of(e, c, sc.P, model);
+    bp.lanes[c] = kr[c].ok() ? kr[c].lanes : kClasses[c].lanes;
     bp.width[c] = kClasses[c].width;
     bp.inv_width[c] = (unsigned)(((1ull << 32) + kClasses[c].width - 1) / kClasses[c].width);
     bp.slot_ps[c] = e->slot_ps[c];
     bp.strip_ps[c] = e->strip_ps[c];
-    bp.fit[c] = (kr[c].fn ? kr[c].limit : e->sc.s16Limit) / e->typical;
+    bp.fit[c] = (kr[c].ok() ? kr[c].limit : e->sc.s16Limit) / e->typical;
   }
   bp.widest = kClsWidest;
   bp.cls_long = kClsLong;
@@ -783,23 +884,21 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.thr_max_rows = kThrMaxRows;
   bp.thr_cap_scale = kThrLatencyShare / (2.0f * (float)thrThreads);
   bp.total_cells = reinterpret_cast<const unsigned long long*>(ctl + CTL_CELLS) + CELLS_TOTAL;
-  // Concurrent class launches, except when every launch is timed alone.
-  const int mode = e->time_launches ? 0
-                   : e->concurrent == 3 ? (n < kShareModeMaxPairs ? 1 : 2)
-                                        : e->concurrent;
-  const bool conc = mode != 0;
-  bp.concurrent = mode;
+  // Concurrent launches, except when every launch is timed alone.
+  const bool conc = !e->time_launches && e->concurrent != 0;
+  bp.concurrent = conc ? 1 : 0;
   // Classes this batch may use (the others are not launched).
   unsigned enabled = kCoarseClasses;
   // Pairs that may pass 16 bits need both sequences longer than s16_max_len.
   const bool highScores = std::min(maxA, maxB) > bp.s16_max_len;
   if (!e->s16_ok || (highScores && !e->hybrid)) enabled |= 1u << kClsS32;
   if (highScores && e->hybrid) enabled |= (1u << kClsHi) | (1u << kClsBig);
-  if (n >= kFineClassMinPairs) enabled |= kFineClasses;
+  enabled |= kFineClasses;
+  if (n < kLatClassMaxPairs) enabled |= kLatClasses;
   // The long class, when the batch may hold a pair past the widest's scores.
   if (std::min(maxA, maxB) > bp.fit[kClsWidest]) enabled |= 1u << kClsLong;
   if (e->thread_class && bits == 8) enabled |= 1u << kClsThread;  // k_thread reads bytes only
-  if (sc.P < e->M && (eight || e->cells != ipuma_engine::kLinear)) {
+  if (sc.P < e->M && model == kMixAff) {
     // Four-row profiles: the narrow widths in 8-lane groups.
     for (const auto& w : kNarrowPairs)
       if ((enabled >> w[0]) & 1u) enabled = (enabled & ~(1u << w[0])) | (1u << w[1]);
@@ -812,44 +911,43 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d (strip teams) needs team_warps >= 2 and room for two warps",
                 kClsTeam + 1);
   if (teamW >= 2 && maxA > kClasses[kClsTeam].width && e->tile_k == 0) enabled |= 1u << kClsTeam;
-  if (e->tile_k > 0) enabled |= 1u << (e->tile_k - 1);
+  if (e->tile_k > 0) {  // no pair is given to a class by cost
+    for (int c = 0; c < kNumClasses; ++c)
+      if (by_cost_class(c)) enabled &= ~(1u << c);
+    enabled |= 1u << (e->tile_k - 1);
+  }
   if (((enabled >> kClsTeam) & 1u) && ((enabled >> kClsBig) & 1u)) enabled |= 1u << kClsBigTeam;
   for (int c = 0; c < kNumClasses; ++c)
-    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].fn) {
+    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].ok()) {
       if (e->tile_k == c + 1) return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d has no kernel for this scoring", e->tile_k);
       enabled &= ~(1u << c);
     }
   bp.enabled = enabled;
+  for (int c = 0; c < kNumClasses; ++c)
+    if (((enabled >> c) & 1u) && by_cost_class(c)) bp.by_cost |= 1u << c;
   bp.team_cls = ((enabled >> kClsTeam) & 1u) ? kClsTeam : -1;
   bp.team_big = ((enabled >> kClsBigTeam) & 1u) ? kClsBigTeam : -1;
   bp.team_warps = std::max(teamW, 1);
-  class_grids(e, sc.P, eight, maxA, maxB, bp.grid, bp.scr_per_block);
+  class_grids(e, sc.P, model, kr, e->time_launches ? 0u : enabled, maxA, maxB, bp.grid, bp.scr_per_block);
   bp.scr_cap = (long long)(rb.scratch->cap / sizeof(int2));
   float slot_min = 1e30f;
-  for (int c = 0; c < kNumS16; ++c) {
+  for (int c = 0; c < kNumClasses; ++c) {
+    if (c == kClsTeam || c == kClsBigTeam) continue;
     // cell slots one warp step covers: 32 lanes x k columns x 2 pairs
     // (the per-thread class: 32 threads x 16 columns x 2 pairs per row)
-    const int k = kr[c].fn ? kr[c].k : kClasses[c].k;
-    bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)k * (float)(bp.grid[c] * kWarpsPerBlock);
-    if (kr[c].fn) slot_min = std::min(slot_min, e->slot_ps[c]);
+    const int k = kr[c].ok() ? kr[c].k : kClasses[c].k;
+    const int grid = kr[c].mix ? kernel_grid(e, kr[c], sc.P, model) : bp.grid[c];
+    bp.step_ps[c] = step_time(e->slot_ps[c] * 64.f * (float)k * (float)(grid * kWarpsPerBlock), k, n, grid);
+    if (((bp.by_cost >> c) & 1u) && kr[c].ok()) slot_min = std::min(slot_min, e->slot_ps[c]);
   }
-  for (int c : {kClsLong, kClsBig})
-    bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * kWarpsPerBlock);
   // A warp of a team steps like one of the widest class's warps.
   for (int c : {kClsTeam, kClsBigTeam})
     bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * bp.team_warps);
   bp.batch_ps_per_cell = slot_min / kPackingEfficiency;
-  bp.lat_share = e->latency_share;
-  bp.lat_min_ps = kLatencyMinBatchPs;
-  bp.region = 0;
-  for (int c = 0; c < kNumClasses; ++c) bp.region = std::max(bp.region, (long long)bp.grid[c] * bp.scr_per_block[c]);
-  // Two alternating streams: stream (and scratch region) by position
-  // among the launched classes.
-  for (int k = 0, pos = 0; k < kNumClasses; ++k) {
-    const int c = kLaunchOrder[k];
-    bp.slot_of[c] = pos & 1;
-    if ((enabled >> c) & 1u) ++pos;
-  }
+  bp.lat_weight = e->latency_weight;
+  bp.team_share = e->sc.forwardOnly ? kTeamShareForward : kTeamShareFull;
+  bp.region = bp.scr_cap / kRunStreams;
+  run_slots(kr, enabled, bp.slot_of);
   bp.long_a = e->long_a;
   // tile_k > 0 forces one s16x2 class: every pair uses the chosen kernel,
   // long A crossing several strips.
@@ -879,66 +977,74 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     *launches += 1;
   } else {
     k_bin_total<<<gb, tb, 0, s>>>(bp, pairs, n, total, ctl + CTL_HIST, nkeys);
-    k_bin_count<<<gb, tb, 0, s>>>(bp, pairs, n, ctl + CTL_HIST, flags, sums, st, score, arange, brange);
+    int* keys = rb.ovf->as<int>();  // free until the alignment launches
+    k_bin_count<<<gb, tb, 0, s>>>(bp, pairs, n, ctl + CTL_HIST, flags, keys, sums, st, score, arange, brange);
     k_bin_scan<<<bp.nclass, 1024, 0, s>>>(bp, ctl + CTL_HIST, ctl + CTL_OFFS, sums, ctl + CTL_RANGES, allot, st);
-    k_bin_scatter<<<gb, tb, 0, s>>>(bp, pairs, n, flags, ctl + CTL_OFFS, rb.list->as<int>());
+    k_bin_scatter<<<gb, tb, 0, s>>>(keys, n, ctl + CTL_OFFS, rb.list->as<int>());
     *launches += 4;
   }
   CUDA_TRY(cudaGetLastError());
 
   int* list = rb.list->as<int>();
   int* heads = ctl + CTL_HEADS;
-  // Class launches: concurrently on the class streams (each on the share
-  // of the SMs k_bin_scan gave it, so every class starts its longest items
-  // at once and the classes finish together), or one after the other on
-  // `s`, longest-tail classes first.
+  const int* R = ctl + CTL_RANGES;
+  const BatchIo io = batch_io(rb, codes, pairs, rowsCap, score, arange, brange);
+  // Launches: the long pairs' first, then k_mix over the other classes, on
+  // up to three streams (or one after the other on `s`).
   if (conc) CUDA_TRY(cudaEventRecord(e->fork_ev, s));
-  // Stream of a class: its own (shares) or one of two by launch position.
-  auto stream_of = [&](int cls) -> int {
-    if (mode == 2) return rb.cls_base + bp.slot_of[cls];
-    return cls;
-  };
-  auto on = [&](int cls) -> cudaStream_t {
-    if (!conc) return s;
-    cudaStream_t cs = e->cls_stream[stream_of(cls)];
-    cudaStreamWaitEvent(cs, e->fork_ev, 0);
+  bool used[kRunStreams] = {};
+  // Streams of a run: 0 is `s` itself.
+  auto on = [&](int slot) -> cudaStream_t {
+    if (!conc || slot == 0) return s;
+    cudaStream_t cs = e->cls_stream[rb.cls_base + slot];
+    if (!used[slot]) cudaStreamWaitEvent(cs, e->fork_ev, 0);
+    used[slot] = true;
     return cs;
   };
-  auto done = [&](int cls) -> int {
-    if (!conc) return IPUMA_OK;
-    cudaStream_t cs = e->cls_stream[stream_of(cls)];
-    CUDA_TRY(cudaEventRecord(e->join_ev[cls], cs));
-    CUDA_TRY(cudaStreamWaitEvent(s, e->join_ev[cls], 0));
-    return IPUMA_OK;
-  };
-  const int* R = ctl + CTL_RANGES;
+  unsigned mixMask = 0;
   for (const int c : kLaunchOrder) {
     if (!((enabled >> c) & 1u)) continue;
-    cudaStream_t cs = on(c);
-    if (c == kClsTeam || c == kClsBigTeam)
-      rc = launch_team(e, sc, rb, cs, codes, pairs, list, R + 2 * c, heads + c, rowsCap, score, arange, brange,
-                       teamW, c);
-    else if (c == kClsThread)
+    cudaStream_t cs = kr[c].mix && !e->time_launches ? s : on(bp.slot_of[c]);
+    if (c == kClsTeam || c == kClsBigTeam) {
+      rc = launch_team(e, sc, rb, cs, io, list, R + 2 * c, heads + c, teamW, c);
+    } else if (c == kClsThread) {
       rc = launch_thread<16>(e, rb, cs, codes, pairs, list, R + 2 * c, heads + c, thread_rows(e, maxA, maxB), score,
                              arange, brange, c);
-    else
-      rc = launch_batched(e, kr[c], sc, rb, cs, codes, pairs, list, R + 2 * c, heads + c, rowsCap, score, arange,
-                          brange, kClasses[c].kind, c, c);
-    if (rc || (rc = done(c))) return rc;
+    } else if (!kr[c].mix) {
+      rc = launch_batched(e, kr[c], sc, rb, cs, io, list, R + 2 * c, heads + c, kClasses[c].kind, c, c);
+    } else if (e->time_launches) {  // a timed launch per class
+      rc = launch_mix(e, model, kr[c].shift, mix_args(kr, 1u << c, rowsCap), sc, rb, cs, 0, io, list, R, heads,
+                      kClasses[c].kind, c);
+    } else {
+      mixMask |= 1u << c;
+      continue;
+    }
+    if (rc) return rc;
     ++*launches;
   }
+  if (mixMask) {
+    const int c = __builtin_ctz(mixMask);
+    if ((rc = launch_mix(e, model, kr[c].shift, mix_args(kr, mixMask, rowsCap), sc, rb, on(bp.slot_of[c]),
+                         conc ? bp.slot_of[c] * bp.region : 0, io, list, R, heads, kClasses[c].kind, c)))
+      return rc;
+    ++*launches;
+  }
+  for (int k = 1; k < kRunStreams; ++k)
+    if (used[k]) {
+      CUDA_TRY(cudaEventRecord(e->join_ev[rb.cls_base + k], e->cls_stream[rb.cls_base + k]));
+      CUDA_TRY(cudaStreamWaitEvent(s, e->join_ev[rb.cls_base + k], 0));
+    }
   // No pair of this batch can leave the range of the lanes it ran in?
   const long long maxScore = (long long)std::min(maxA, maxB) * std::max(0, e->maxSub);
   bool overflow = e->thread_class || e->tile_k == kClsThread + 1;
   for (int c = 0; c < kNumClasses; ++c)
     if (((enabled >> c) & 1u) && c != kClsS32)
-      overflow |= maxScore > (kr[c].fn ? kr[c].limit : kr[kClsLong].limit);
+      overflow |= maxScore > (kr[c].ok() ? kr[c].limit : kr[kClsLong].limit);
   if (!overflow) return IPUMA_OK;
   // Exact 32-bit rerun of the s16x2 pairs whose score may have overflowed
   // (after every class: it reads their overflow list).
-  if ((rc = launch_batched(e, kr[kClsS32], sc, rb, s, codes, pairs, rb.ovf->as<int>(), ctl + CTL_STATUS + 1,
-                           heads + NCLASS_MAX, rowsCap, score, arange, brange, IPUMA_KERNEL_S32_RERUN, kTimedRerun,
-                           NCLASS_MAX)))
+  if ((rc = launch_batched(e, kr[kClsS32], sc, rb, s, io, rb.ovf->as<int>(), ctl + CTL_STATUS + 1, heads + NCLASS_MAX,
+                           IPUMA_KERNEL_S32_RERUN, kTimedRerun, NCLASS_MAX)))
     return rc;
   *launches += 1;
   return IPUMA_OK;
@@ -1105,6 +1211,10 @@ void set_s32_rates(ipuma_engine* e) {
   e->strip_ps[kClsTeam] = e->strip_ps[kClsWidest];
   e->slot_ps[kClsLong] = e->slot_ps[kClsWidest];
   e->strip_ps[kClsLong] = e->strip_ps[kClsWidest];
+  for (int c : {kClsLat256, kClsLat128}) {  // a step's fixed work on fewer columns
+    e->slot_ps[c] = (c == kClsLat256 ? 1.25f : 1.6f) * e->slot_ps[kClsWidest];
+    e->strip_ps[c] = e->strip_ps[kClsWidest];
+  }
   for (int c : {kClsBig, kClsBigTeam}) {  // their whole best row costs a seventh more per cell
     e->slot_ps[c] = 1.15f * e->slot_ps[kClsWidest];
     e->strip_ps[c] = e->strip_ps[kClsWidest];
@@ -1264,9 +1374,10 @@ int run_autotune(ipuma_engine* e, const char* cache_path) {
     // far more pairs resident, so two rounds of items suffice there.
     const int perItem = L > 0 ? (32 / L) * 2 : 64;
     const int rounds = L > 0 ? 6 : 2;
-    const KernelRef kr = kernel_of(e, c, e->M, true);
-    if (c != kClsThread && !kr.fn) continue;  // no kernel of this class for this scoring
-    const int grid = c == kClsThread ? (int)(thread_threads<16>(e) / kThreads) : kernel_grid(e, kr);
+    const int model = mix_model(e, e->M, true);
+    const KernelRef kr = kernel_of(e, c, e->M, model);
+    if (c != kClsThread && !kr.ok()) continue;  // no kernel of this class for this scoring
+    const int grid = c == kClsThread ? (int)(thread_threads<16>(e) / kThreads) : kernel_grid(e, kr, e->M, model);
     const int minPairs = grid * kWarpsPerBlock * perItem * rounds;
     // (strips, rows) of the two calibration batches.  The per-thread class
     // passes a boundary column through global memory at every strip, so
@@ -1478,7 +1589,7 @@ WireSet wire_set(ipuma_engine* e, int k) {
   if (k == 0) return WireSet{&e->d_inputs, &e->d_wres, &e->d_pairs, &e->d_ctl, main_bufs(e), e->stream};
   WireBufs& w = e->w1;
   return WireSet{&w.inputs, &w.results, &w.pairs, &w.ctl,
-                 RunBufs{w.ctl.as<int>(), &w.scratch, &w.list, &w.ovf, &w.flag, 2}, e->wstream1};
+                 RunBufs{w.ctl.as<int>(), &w.scratch, &w.list, &w.ovf, &w.flag, kRunStreams}, e->wstream1};
 }
 
 int take_event(ipuma_engine* e, cudaEvent_t* ev) {
@@ -1803,7 +1914,7 @@ int ipuma_gpu_set_option(ipuma_engine* e, const char* name, int64_t value) {
     e->time_launches = value ? 1 : 0;
   } else if (k == "latency_share") {
     if (value < 1 || value > 100000) return fail(IPUMA_ERR_INVALID_ARG, "latency_share is in per mille, 1..100000");
-    e->latency_share = (float)value / 1000.f;
+    e->latency_weight = (float)value / 1000.f;
   } else if (k == "hybrid") {
     e->hybrid = value ? 1 : 0;
   } else if (k == "concurrent") {
@@ -1923,7 +2034,7 @@ static int compare_dev(ipuma_engine* e, const uint8_t* d_codes, size_t n_codes, 
                                        (uint64_t)(uintptr_t)e->d_ovf.p, (uint64_t)(uintptr_t)e->d_flag.p,
                                        (uint64_t)e->tile_k, (uint64_t)e->long_a, (uint64_t)e->thread_class,
                                        (uint64_t)e->concurrent, (uint64_t)e->hybrid, (uint64_t)e->trace,
-                                       (uint64_t)(e->latency_share * 1e6f), (uint64_t)e->team_warps};
+                                       (uint64_t)(e->latency_weight * 1e6f), (uint64_t)e->team_warps};
     auto it = e->graphs_cache.find(key);
     if (it == e->graphs_cache.end()) {
       if (e->graphs_cache.size() >= 16) {
@@ -2082,7 +2193,7 @@ static int compare_host(ipuma_engine* e, const uint8_t* codes, size_t n_codes, i
       if (!ev) CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     int nmax = 0;
     for (int k = 0; k < nch; ++k) nmax = std::max(nmax, cbeg[k + 1] - cbeg[k]);
-    const RunBufs rb1{nullptr, &e->x_scratch, &e->x_list, &e->x_ovf, &e->x_flag, 2};
+    const RunBufs rb1{nullptr, &e->x_scratch, &e->x_list, &e->x_ovf, &e->x_flag, kRunStreams};
     if ((rc = e->d_ctl.ensure(sizeof(int) * CTL_INTS * (size_t)nch, s))) return rc;
     if ((rc = reserve_bufs(e, main_bufs(e), s, nmax, maxA, maxB))) return rc;
     if ((rc = reserve_bufs(e, rb1, s, nmax, maxA, maxB))) return rc;

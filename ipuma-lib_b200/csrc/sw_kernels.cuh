@@ -54,11 +54,10 @@ struct DevStatus {
   int pad;
 };
 
-// Share of the GPU one class launch may use: blocks with blockIdx.x >=
-// `blocks` exit at once, and the launch's strip scratch starts `base` int2
-// into the scratch buffer.  Written on the device by the binning pre-pass
-// (k_bin_scan) so that concurrent class launches split the SMs in
-// proportion to their modelled work and never share scratch.
+// Blocks of a class launch that work (those past `blocks` exit at once: all
+// of them when the class is empty), and where its strip scratch starts in
+// the scratch buffer (int2), so that concurrent launches never share any.
+// Written on the device by the binning pre-pass.
 struct ClassAllot {
   long long base;
   int blocks;
@@ -284,43 +283,108 @@ __device__ __forceinline__ void write_result(const SwConst& sc, const Best& fw, 
   brange[idx] = pack_range(bstart, bend);
 }
 
-// Persistent batched kernel.  `list` holds pair ids in processing order;
-// a warp takes items of 32 / LANES * NP consecutive entries (ids < 0 are
-// padding), lane group g aligning entries [g * NP, g * NP + NP).
+// What the kernels read and write besides their work list.
+struct BatchIo {
+  const uint8_t* codes;
+  const PairDesc* pairs;
+  long rowsCap;
+  int *score, *arange, *brange, *overflow_list;
+  unsigned long long* rerun_cells;
+  DevStatus* st;
+};
+
+// One work item of a warp: the 32 / LANES * NP list entries from `first`
+// on (those below n), lane group g aligning entries [g * NP, g * NP + NP).
+//   wsmem : the warp's shared memory (SmemLayout::warp_bytes)
+//   wscr  : the warp's strip-boundary scratch
+template <class T, int K, int LANES, bool HYB, bool FWD>
+__device__ __forceinline__ void batched_item(const SwConst& sc, const BatchIo& io, const int8_t* s_simp, uint8_t* wsmem,
+                                             int2* wscr, const int* list, int first, int n) {
+  using L = SmemLayout<T, K, LANES>;
+  constexpr int NP = T::NP;
+  constexpr int NBUF = HYB ? 3 : 2;  // strip-boundary buffers per group
+  const int lane32 = threadIdx.x & 31;
+  const int group = lane32 / LANES;
+  const int glane = lane32 & (LANES - 1);
+  uint8_t* s_prof = wsmem + group * L::group_bytes(sc.P);
+  uint16_t* s_bring = reinterpret_cast<uint16_t*>(s_prof + L::prof_bytes(sc.P));
+  int2* scr = wscr + group * NBUF * io.rowsCap;
+  int pid[NP], alen[NP], blen[NP];
+  long long a0[NP], b0[NP];
+  bool tooLong = false;
+#pragma unroll
+  for (int h = 0; h < NP; ++h) {
+    const int k = first + group * NP + h;
+    pid[h] = (k < n) ? list[k] : -1;
+    PairDesc d = (pid[h] >= 0) ? io.pairs[pid[h]] : PairDesc{0, 0, 0, 0};
+    alen[h] = d.a_len;
+    blen[h] = d.b_len;
+    a0[h] = d.a_off;
+    b0[h] = d.b_off;
+    tooLong |= d.b_len > io.rowsCap;
+  }
+  if (__any_sync(FULL, tooLong)) {
+    // The host sizes the scratch for the longest B; report, never trap.
+    if (lane32 == 0) atomicCAS(&io.st->error, 0, ERR_SCRATCH);
+    return;
+  }
+  Best fw[NP], rv[NP];
+  bool ovf[NP];
+  if constexpr (HYB) {
+    static_assert(NP == 2 && LANES == 32, "the hybrid class pairs two pairs per 32-lane warp");
+    // Mode chosen at run time: specialising the hybrid class made its
+    // forward-only kernel spill and slowed the heavy-tailed protein batch.
+    align_pairs_hybrid<K, 0>(sc, s_prof, s_simp, s_bring, io.codes, a0, b0, alen, blen, scr, io.rowsCap, fw, rv, ovf);
+  } else {
+    // 16-bit classes: one kernel per mode (fewer registers, no spills for
+    // forward-only; the early reverse stop for full alignments); the s32
+    // class keeps the run-time choice for the same reason as the hybrid.
+    constexpr int MODE = (T::NP == 1) ? 0 : (FWD ? 1 : 2);
+    align_pairs<T, K, LANES, MODE>(sc, s_prof, s_simp, s_bring, io.codes, a0, b0, alen, blen, scr, io.rowsCap, fw, rv,
+                                   ovf);
+  }
+  if (glane == 0) {
+#pragma unroll
+    for (int h = 0; h < NP; ++h) {
+      if (pid[h] < 0) continue;
+      if (ovf[h]) {
+        const int slot = atomicAdd(&io.st->overflow_count, 1);
+        io.overflow_list[slot] = pid[h];
+        atomicAdd(io.rerun_cells, (unsigned long long)alen[h] * (unsigned long long)blen[h]);
+        continue;
+      }
+      write_result(sc, fw[h], rv[h], io.score, io.arange, io.brange, pid[h]);
+    }
+  }
+}
+
+// Persistent kernel of one class.  `list` holds pair ids in processing
+// order; warps take items from an atomic queue head.
 // Register budget: the forward-only kernels get at most 128 registers (4
 // blocks of 128 threads per SM when the profile is small); the kernels
 // with a reverse pass or a run-time mode (FWD false, or the hybrid class)
 // up to 170 (3 blocks per SM, which their shared memory allows anyway), as
-// at 128 they spilled.
+// at 128 they spilled.  The affine classes of long pairs, proteins mostly,
+// fit two blocks by their shared memory.
+template <class T, bool HYB, bool FWD>
+constexpr int kBatchedBlocks = (kTagged<T> && !T::LINEAR) ? 2 : (FWD && !HYB) ? 4 : 3;
 template <class T, int K, int LANES, bool HYB = false, bool FWD = false>
-__global__ void __launch_bounds__(128, (FWD && !HYB) ? 4 : 3) k_batched(SwConst sc, const int8_t* __restrict__ sim,
-                                                 const uint8_t* __restrict__ codes,
-                                                 const PairDesc* __restrict__ pairs,
-                                                 const int* __restrict__ list,
-                                                 const int* __restrict__ range, int* queue_head,
-                                                 int2* scratch, long rowsCap, int* score,
-                                                 int* arange, int* brange, int* overflow_list,
-                                                 unsigned long long* rerun_cells, DevStatus* st,
-                                                 const ClassAllot* __restrict__ allot,
-                                                 unsigned long long* trace) {
+__global__ void __launch_bounds__(128, kBatchedBlocks<T, HYB, FWD>)
+    k_batched(SwConst sc, const int8_t* __restrict__ sim, BatchIo io, const int* __restrict__ list,
+              const int* __restrict__ range, int* queue_head, int2* scratch, const ClassAllot* __restrict__ allot,
+              unsigned long long* trace) {
   if ((int)blockIdx.x >= allot->blocks) return;  // outside this launch's share
   scratch += allot->base;
   // trace (option "trace"): {~first block start, last warp end} of the launch.
   if (trace && threadIdx.x == 0) atomicMax(&trace[0], ~global_ns());
   using L = SmemLayout<T, K, LANES>;
-  constexpr int NP = T::NP;
-  constexpr int GROUPS = L::GROUPS;
-  constexpr int PER_ITEM = GROUPS * NP;
+  constexpr int PER_ITEM = L::GROUPS * T::NP;
   extern __shared__ __align__(16) uint8_t smem[];
   const int warps = blockDim.x >> 5;
   const int wib = threadIdx.x >> 5;
   const int lane32 = threadIdx.x & 31;
-  const int group = lane32 / LANES;
-  const int glane = lane32 & (LANES - 1);
   int8_t* s_simp = reinterpret_cast<int8_t*>(smem);
-  uint8_t* gbase = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P) + group * L::group_bytes(sc.P);
-  uint8_t* s_prof = gbase;
-  uint16_t* s_bring = reinterpret_cast<uint16_t*>(gbase + L::prof_bytes(sc.P));
+  uint8_t* wsmem = smem + L::simp_bytes(sc.M, sc.P) + wib * L::warp_bytes(sc.P);
   load_table(s_simp, sim, sc, kProfBias<T> ? -sc.gE : 0, kProfShift<T>);
   __syncthreads();
 
@@ -330,62 +394,13 @@ __global__ void __launch_bounds__(128, (FWD && !HYB) ? 4 : 3) k_batched(SwConst 
   list += range[0];
   const int items = (n + PER_ITEM - 1) / PER_ITEM;
   const long gw = (long)blockIdx.x * warps + wib;
-  constexpr int NBUF = HYB ? 3 : 2;  // strip-boundary buffers per group
-  int2* scr = scratch + (gw * GROUPS + group) * NBUF * rowsCap;
+  int2* wscr = scratch + gw * L::GROUPS * (HYB ? 3 : 2) * io.rowsCap;
   while (true) {
     int item = 0;
     if (lane32 == 0) item = atomicAdd(queue_head, 1);
     item = __shfl_sync(FULL, item, 0);
     if (item >= items) break;
-    int pid[NP], alen[NP], blen[NP];
-    long long a0[NP], b0[NP];
-    bool tooLong = false;
-#pragma unroll
-    for (int h = 0; h < NP; ++h) {
-      const int k = item * PER_ITEM + group * NP + h;
-      pid[h] = (k < n) ? list[k] : -1;
-      PairDesc d = (pid[h] >= 0) ? pairs[pid[h]] : PairDesc{0, 0, 0, 0};
-      alen[h] = d.a_len;
-      blen[h] = d.b_len;
-      a0[h] = d.a_off;
-      b0[h] = d.b_off;
-      tooLong |= d.b_len > rowsCap;
-    }
-    if (__any_sync(FULL, tooLong)) {
-      // The host sizes the scratch for the longest B; report, never trap.
-      if (lane32 == 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
-      continue;
-    }
-    Best fw[NP], rv[NP];
-    bool ovf[NP];
-    if constexpr (HYB) {
-      static_assert(NP == 2 && LANES == 32, "the hybrid class pairs two s16x2 pairs per 32-lane warp");
-      // Mode chosen at run time: specialising the hybrid class made its
-      // forward-only kernel spill and slowed the heavy-tailed protein batch.
-      align_pairs_hybrid<K, 0>(sc, s_prof, s_simp, s_bring, codes, a0, b0, alen, blen, scr, rowsCap, fw, rv,
-                               ovf);
-    } else {
-      // s16x2 classes: one kernel per mode (fewer registers, no spills for
-      // forward-only; the early reverse stop for full alignments); the s32
-      // class keeps the run-time choice for the same reason as the hybrid.
-      constexpr int MODE = (T::NP == 1) ? 0 : (FWD ? 1 : 2);
-      align_pairs<T, K, LANES, MODE>(sc, s_prof, s_simp, s_bring, codes, a0, b0, alen, blen, scr, rowsCap, fw, rv,
-                                     ovf);
-    }
-    if (glane == 0) {
-#pragma unroll
-      for (int h = 0; h < NP; ++h) {
-        if (pid[h] < 0) continue;
-        if (ovf[h]) {
-          const int slot = atomicAdd(&st->overflow_count, 1);
-          overflow_list[slot] = pid[h];
-          if (rerun_cells)
-            atomicAdd(rerun_cells, (unsigned long long)alen[h] * (unsigned long long)blen[h]);
-          continue;
-        }
-        write_result(sc, fw[h], rv[h], score, arange, brange, pid[h]);
-      }
-    }
+    batched_item<T, K, LANES, HYB, FWD>(sc, io, s_simp, wsmem, wscr, list, item * PER_ITEM, n);
   }
   if (trace && lane32 == 0) atomicMax(&trace[1], global_ns());
 }
@@ -433,15 +448,10 @@ __device__ __forceinline__ int team_size(int warps, long blocks, int items, int 
 }
 
 template <class T, int K>
-__global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __restrict__ sim,
-                                                   const uint8_t* __restrict__ codes,
-                                                   const PairDesc* __restrict__ pairs,
-                                                   const int* __restrict__ list, const int* __restrict__ range,
-                                                   int* queue_head, int2* scratch, long rowsCap, int* score,
-                                                   int* arange, int* brange, int* overflow_list,
-                                                   unsigned long long* rerun_cells, DevStatus* st,
-                                                   const ClassAllot* __restrict__ allot,
-                                                   unsigned long long* trace) {
+__global__ void __launch_bounds__(256, T::LINEAR ? 2 : 1)
+    k_strips(SwConst sc, const int8_t* __restrict__ sim, BatchIo io, const int* __restrict__ list,
+             const int* __restrict__ range, int* queue_head, int2* scratch, const ClassAllot* __restrict__ allot,
+             unsigned long long* trace) {
   if ((int)blockIdx.x >= allot->blocks) return;
   scratch += allot->base;
   if (trace && threadIdx.x == 0) atomicMax(&trace[0], ~global_ns());
@@ -468,7 +478,7 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
   list += range[0];
   const int items = (n + NP - 1) / NP;
   if (n <= 0) return;
-  const PairDesc longest = pairs[list[0]];
+  const PairDesc longest = io.pairs[list[0]];
   const int tsize = team_size(warps, min((long)gridDim.x, (long)allot->blocks), items,
                               (longest.a_len + 32 * K - 1) / (32 * K), longest.b_len);
   const int q = wib / tsize, tw = wib % tsize;  // this warp's team, and its place there
@@ -480,8 +490,8 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
   };
   Best(&s_best)[2][NP] = s_bestT[q];
   bool(&s_ovf)[NP] = s_ovfT[q];
-  int2* scr = scratch + ((long)blockIdx.x * warps + q * tsize) * rowsCap;
-  const StripTeam team{s_prog + q * tsize, &s_abort[q], &st->error, ERR_WAIT, tw, tsize};
+  int2* scr = scratch + ((long)blockIdx.x * warps + q * tsize) * io.rowsCap;
+  const StripTeam team{s_prog + q * tsize, &s_abort[q], &io.st->error, ERR_WAIT, tw, tsize};
   while (true) {
     team_sync();  // the previous item's merge is done
     if (tid == 0) {
@@ -499,19 +509,19 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
     for (int h = 0; h < NP; ++h) {
       const int k = item * NP + h;
       pid[h] = (k < n) ? list[k] : -1;
-      d[h] = (pid[h] >= 0) ? pairs[pid[h]] : PairDesc{0, 0, 0, 0};
-      tooLong |= d[h].b_len > rowsCap;
+      d[h] = (pid[h] >= 0) ? io.pairs[pid[h]] : PairDesc{0, 0, 0, 0};
+      tooLong |= d[h].b_len > io.rowsCap;
     }
     if (tooLong) {
       // The host sizes the scratch for the longest B; report, never trap.
-      if (tid == 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
+      if (tid == 0) atomicCAS(&io.st->error, 0, ERR_SCRATCH);
       continue;
     }
     PassSeq ps[NP];
 #pragma unroll
     for (int h = 0; h < NP; ++h) {
       const bool empty = d[h].a_len <= 0 || d[h].b_len <= 0;
-      ps[h] = PassSeq{codes, d[h].a_off, d[h].b_off, empty ? 0 : d[h].a_len, empty ? 0 : d[h].b_len, 1, 1};
+      ps[h] = PassSeq{io.codes, d[h].a_off, d[h].b_off, empty ? 0 : d[h].a_len, empty ? 0 : d[h].b_len, 1, 1};
     }
     // Pass 0: forward.  Pass 1 (with start coordinates): the same pass over
     // the reversed reads from each pair's end cell (as align_pairs, without
@@ -520,7 +530,7 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
       Best out[NP];
-      tag_pass<T, K, 32, false, true>(sc, s_prof, s_simp, s_bring, ps, scr, rowsCap, out, PassStop{}, team);
+      tag_pass<T, K, 32, false, true>(sc, s_prof, s_simp, s_bring, ps, scr, io.rowsCap, out, PassStop{}, team);
       if (lane == 0) {
 #pragma unroll
         for (int h = 0; h < NP; ++h) s_res[wib][h] = out[h];
@@ -549,8 +559,8 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
         const Best fw = s_best[0][h];
         const bool run = pid[h] >= 0 && !s_ovf[h] && fw.s > 0;
         any |= run;
-        ps[h] = run ? PassSeq{codes, d[h].a_off + fw.j, d[h].b_off + fw.i, fw.j + 1, fw.i + 1, -1, -1}
-                    : PassSeq{codes, d[h].a_off, d[h].b_off, 0, 0, 1, 1};
+        ps[h] = run ? PassSeq{io.codes, d[h].a_off + fw.j, d[h].b_off + fw.i, fw.j + 1, fw.i + 1, -1, -1}
+                    : PassSeq{io.codes, d[h].a_off, d[h].b_off, 0, 0, 1, 1};
       }
       if (!any) break;  // block-uniform: every thread read the same words
       // A fresh team for the reverse pass (after every warp read s_ovf).
@@ -563,11 +573,11 @@ __global__ void __launch_bounds__(256, 2) k_strips(SwConst sc, const int8_t* __r
       const int h = tid;
       if (pid[h] >= 0) {
         if (s_ovf[h]) {
-          const int slot = atomicAdd(&st->overflow_count, 1);
-          overflow_list[slot] = pid[h];
-          if (rerun_cells) atomicAdd(rerun_cells, (unsigned long long)d[h].a_len * (unsigned long long)d[h].b_len);
+          const int slot = atomicAdd(&io.st->overflow_count, 1);
+          io.overflow_list[slot] = pid[h];
+          atomicAdd(io.rerun_cells, (unsigned long long)d[h].a_len * (unsigned long long)d[h].b_len);
         } else {
-          write_result(sc, s_best[0][h], s_best[1][h], score, arange, brange, pid[h]);
+          write_result(sc, s_best[0][h], s_best[1][h], io.score, io.arange, io.brange, pid[h]);
         }
       }
     }
@@ -771,7 +781,7 @@ static __global__ void k_exact(SwConst sc, const int8_t* __restrict__ sim, const
 constexpr int NROWB = 256;    // row buckets (16 per power of two)
 constexpr int NSTRIPB = 16;   // strip-count buckets
 constexpr int NBUCKET = NROWB * NSTRIPB;
-constexpr int NCLASS_MAX = 27;
+constexpr int NCLASS_MAX = 29;
 
 // Log-linear bucket of |B| (16 sub-buckets per power of two): pairs that
 // share a bucket differ by at most 1/16 in rows, so the groups of a warp
@@ -802,23 +812,20 @@ struct BinParams {
   unsigned inv_width[NCLASS_MAX];  // ceil(2^32 / width): strips_of
   float slot_ps[NCLASS_MAX];   // time per cell slot of a strip (autotuned)
   float strip_ps[NCLASS_MAX];  // fixed time per strip (autotuned)
-  // Latency bound: one warp item of class c advances one step (row) every
-  // step_ps[c] when the GPU is full, so a pair of `strips` strips takes
-  // strips * (|B| + lanes) * step_ps[c].  A class is not chosen for a pair
-  // whose item would take longer than lat_share * (modelled batch time =
-  // cells of the batch * batch_ps_per_cell), when that batch time is at
-  // least lat_min_ps: a few such items would end their launch alone.
+  // One warp item of class c advances one step (row) every step_ps[c], so a
+  // pair of `strips` strips takes strips * (|B| + lanes) * step_ps[c]; it
+  // counts lat_weight times that beside the batch's modelled time (pair_key).
   float step_ps[NCLASS_MAX];
-  float batch_ps_per_cell;
-  float lat_share;
-  float lat_min_ps;
+  float batch_ps_per_cell;     // modelled batch time per cell (strip teams)
+  float lat_weight;
+  float team_share;            // kTeamShareForward or kTeamShareFull
   int long_a;                  // |A| above which the widest strips are used
   int widest;                  // class of the widest strips
   int cls_long;                // the same strips with room for the longest scores (past fit[widest])
   int forced_class;        // >= 0: every s16x2 pair goes to this class
   int team_cls;            // strip-team class (-1: none in this batch)
   int team_warps;          // warps per team
-  int n_s16_classes;
+  unsigned by_cost;        // classes a pair is given to by its modelled time
   int max_a, max_b;        // stated maxima (violations set ERR_LENGTH)
   long long n_codes;       // residues in the code array (pairs past it set ERR_RANGE)
   int bits;                // bits per residue of the code array (code_at)
@@ -829,13 +836,13 @@ struct BinParams {
   // stay below thr_cap_scale * (cells of the whole batch): that bounds its
   // latency to a fraction of the batch's time (thr_cap_scale = fraction /
   // pair slots the class keeps resident).
-  // Concurrent class launches (k_bin_scan turns modelled costs into block
-  // shares): full-occupancy grid and strip scratch (int2) per block of
-  // each class, and the scratch available.
   unsigned int enabled;    // bit c: class c may be chosen by cost (and is launched)
-  int concurrent;          // 0 sequential, 1 shares, 2 two alternating streams
-  int slot_of[NCLASS_MAX + 1];  // mode 2: scratch region (0 / 1) of each class
-  long long region;             // mode 2: int2 per region
+  // Concurrent launches: full-occupancy grid and strip scratch (int2) per
+  // block of each class, the scratch region of its stream, and the scratch
+  // available.
+  int concurrent;          // 0: one launch after the other
+  int slot_of[NCLASS_MAX + 1];
+  long long region;        // int2 per region
   int grid[NCLASS_MAX + 1];
   long long scr_per_block[NCLASS_MAX + 1];
   long long scr_cap;
@@ -910,12 +917,15 @@ static __device__ int warp_diagonal_bound(const uint8_t* codes, int bits, long l
   return __shfl_sync(FULL, r.best, 0);
 }
 
-// Share of the batch's modelled time above which a pair's one-warp latency
-// sends it to a strip team (measured on B200: a 500,000-pair heavy-tailed
-// protein batch, whose 8,000-residue pairs take about a third of its time
-// on one warp, ran 10 % slower with them in teams; batches of a few hundred
-// long pairs ran 3.7-5.6 times faster).
-constexpr float kTeamLatencyShare = 0.5f;
+// A pair goes to a strip team when its one-warp latency passes this many
+// times the batch's modelled time: below it the other pairs' work hides the
+// pair, and a team's fill and idle warps only cost throughput (B200, at 0.5
+// / 1 / 1.5 / 2.5: 12,000 proteins 1.64 / 1.18 / 1.17 / 1.62 ms, 8,000
+// heavy-tailed 16.3 / 16.6 / 11.5 / 11.5, 60,000 22.7 / 22.7 / 21.5 / 37.3,
+// 700 pairs of 2,000-2,500 2.69 / 2.68 / 2.69 / 4.20).  With start
+// coordinates a team costs more -- its reverse pass has no early stop -- and
+// the line lies higher (4,006 proteins 2.01 ms at 1.5, 1.43 at 2.5).
+constexpr float kTeamShareForward = 1.5f, kTeamShareFull = 2.5f;
 
 // Class of a pair: the kernel with the lowest modelled time
 //   strips * ((|B| + lanes) * width * slot_ps + strip_ps)
@@ -931,14 +941,14 @@ __device__ __forceinline__ int strips_of(const BinParams& bp, int c, int alen) {
 
 // A strip team's class `tc` for a pair whose one-warp latency is `lat`, or
 // cls: taken when even the fastest warp would take a large share of the
-// whole batch's modelled time (kTeamLatencyShare: below it the other pairs'
+// whole batch's modelled time (team_share: below it the other pairs'
 // work hides the pair, and a team's fill and idle warps only cost
 // throughput) and the team finishes the pair sooner.  Its warps take the
 // strips round robin, each starting about kTeamLagSteps behind the warp
 // before it.
 __device__ __forceinline__ int team_class(const BinParams& bp, int cls, int tc, int alen, int blen, float lat,
                                           float batch_ps) {
-  if (tc < 0 || lat <= kTeamLatencyShare * batch_ps) return cls;
+  if (tc < 0 || lat <= bp.team_share * batch_ps) return cls;
   const int strips = strips_of(bp, tc, alen);
   if (strips < 2) return cls;
   const int rounds = (strips + bp.team_warps - 1) / bp.team_warps;
@@ -949,8 +959,7 @@ __device__ __forceinline__ int team_class(const BinParams& bp, int cls, int tc, 
 }
 
 // `flag`: 0, 1 (the diagonal bound passes s16_limit) or 2 (big_limit).
-__device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen, int flag, float thr_cap,
-                                        float* cost_out = nullptr) {
+__device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen, int flag, float thr_cap) {
   int cls;
   if (bp.force_s32) {
     cls = bp.cls_s32;
@@ -979,41 +988,31 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
     } else {
       cls = wide;
       float bestCost = -1.f;
-      int latCls = wide;
       const bool thr_ok = bp.thr_on && blen <= bp.thr_max_rows && (float)alen * (float)blen <= thr_cap;
-      const float lat_cap = batch_ps >= bp.lat_min_ps ? bp.lat_share * batch_ps : 3.0e38f;
-      for (int c = 0; c < bp.n_s16_classes; ++c) {
-        if (!((bp.enabled >> c) & 1u)) continue;
+      // The time of a batch made of this pair alone, as many as hold the
+      // batch's cells: its share of the GPU's rate, and once a part of its
+      // own latency (the last ones finish alone).
+      const float like = bp.total_cells ? (float)(*bp.total_cells) / ((float)alen * (float)blen) : 1.f;
+      for (unsigned left = bp.by_cost; left; left &= left - 1) {
+        const int c = __ffs(left) - 1;
         if ((c == bp.thr_cls && !thr_ok) || fit > bp.fit[c]) continue;
         const int strips = strips_of(bp, c, alen);
         const float lat = (float)strips * (float)(blen + bp.lanes[c]) * bp.step_ps[c];
-        if (bestLat < 0.f || lat < bestLat) {
-          bestLat = lat;
-          latCls = c;
-        }
-        if (lat > lat_cap) continue;
         const float cost =
-            (float)strips * ((float)(blen + bp.lanes[c]) * (float)bp.width[c] * bp.slot_ps[c] + bp.strip_ps[c]);
+            (float)strips * ((float)(blen + bp.lanes[c]) * (float)bp.width[c] * bp.slot_ps[c] + bp.strip_ps[c]) *
+                like + (c == bp.thr_cls ? 0.f : bp.lat_weight * lat);
         if (bestCost < 0.f || cost < bestCost) {
           bestCost = cost;
+          bestLat = lat;
           cls = c;
         }
       }
-      if (bestLat < 0.f) {  // no class holds its scores but the long one
-        bestLat = (float)strips_of(bp, cls, alen) * (float)(blen + bp.lanes[cls]) *
-                  bp.step_ps[cls];
-      } else if (bestCost < 0.f) {
-        cls = latCls;  // every class is too slow: the fastest
-      } else {
-        bestLat = 0.f;  // a class keeps the pair under the latency cap
-      }
+      if (bestCost < 0.f)  // no class holds its scores but the long one
+        bestLat = (float)strips_of(bp, cls, alen) * (float)(blen + bp.lanes[cls]) * bp.step_ps[cls];
     }
     cls = team_class(bp, cls, bp.team_cls, alen, blen, bestLat, batch_ps);
   }
   const int strips = strips_of(bp, cls, alen);
-  if (cost_out)
-    *cost_out = (float)strips *
-                ((float)(blen + bp.lanes[cls]) * (float)bp.width[cls] * bp.slot_ps[cls] + bp.strip_ps[cls]);
   if (cls == bp.thr_cls) {
     const int sb = THR_NSB - 1 - min(strips - 1, THR_NSB - 1);
     return cls * NBUCKET + sb * THR_NRB + (THR_NRB - 1 - min(rows_bucket(blen), THR_NRB - 1));
@@ -1079,30 +1078,26 @@ static __global__ void k_bin_bound(BinParams bp, const uint8_t* __restrict__ cod
   }
 }
 
-// Sums of the pairs of one class: cells, modelled cost (ps) and pairs.
+// Sums of the pairs of one class.
 struct ClassSums {
-  unsigned long long cells, cost;
+  unsigned long long cells;
   int count, pad;
 };
 
-// Key of one listed pair; its cells and cost go to the block's class sums
+// Key of one listed pair; its cells go to the block's class sums
 // with one atomic per class among the warp's lanes (shared 64-bit atomics of
 // 256 threads on a handful of classes took 17 of the kernel's 22 us for
 // 20,000 pairs).  Called by the lanes of `act`.
 __device__ __forceinline__ int tally_pair(const BinParams& bp, const PairDesc& d, int flag, ClassSums* s_sum,
                                           unsigned act) {
-  float cost = 0.f;
-  const int key = pair_key(bp, d.a_len, d.b_len, flag, thread_cap(bp), &cost);
+  const int key = pair_key(bp, d.a_len, d.b_len, flag, thread_cap(bp));
   const unsigned same = __match_any_sync(act, key / NBUCKET);
   const unsigned cells = (unsigned)d.a_len * (unsigned)d.b_len;  // < 2^32: lengths below 65536
-  const unsigned ps = (unsigned)fminf(fmaxf(cost, 1.f), 4.0e9f);
   // Sums in 16-bit halves, which 32 lanes cannot carry out of 32 bits.
   const unsigned c0 = __reduce_add_sync(same, cells & 0xffffu), c1 = __reduce_add_sync(same, cells >> 16);
-  const unsigned p0 = __reduce_add_sync(same, ps & 0xffffu), p1 = __reduce_add_sync(same, ps >> 16);
   if ((int)(threadIdx.x & 31) == __ffs(same) - 1) {
     ClassSums& s = s_sum[key / NBUCKET];
     atomicAdd(&s.cells, ((unsigned long long)c1 << 16) + c0);
-    atomicAdd(&s.cost, ((unsigned long long)p1 << 16) + p0);
     atomicAdd(&s.count, __popc(same));
   }
   return key;
@@ -1118,25 +1113,25 @@ __device__ __forceinline__ void reject_pair(int state, long p, DevStatus* st, in
 }
 
 static __global__ void k_bin_count(BinParams bp, const PairDesc* __restrict__ pairs, int n, int* hist,
-                                   uint8_t* s32_flag, ClassSums* sums, DevStatus* st, int* score, int* arange,
+                                   const uint8_t* s32_flag, int* keys, ClassSums* sums, DevStatus* st, int* score, int* arange,
                                    int* brange) {
   __shared__ ClassSums s_sum[NCLASS_MAX];
-  for (int k = threadIdx.x; k < NCLASS_MAX; k += blockDim.x) s_sum[k] = ClassSums{0, 0, 0, 0};
+  for (int k = threadIdx.x; k < NCLASS_MAX; k += blockDim.x) s_sum[k] = ClassSums{0, 0, 0};
   __syncthreads();
   for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
     const PairDesc d = pairs[p];
     const int state = pair_state(d, bp.n_codes, bp.max_a, bp.max_b);
     if (state != PAIR_OK) {
       reject_pair(state, p, st, score, arange, brange);
+      keys[p] = -1;
       continue;
     }
     // Candidates (both sequences longer than s16_max_len) got their flag
     // from k_bin_bound.
-    int flag = 0;
-    if (bound_candidate(bp, d)) flag = s32_flag[p];
-    s32_flag[p] = (uint8_t)flag;
+    const int flag = bound_candidate(bp, d) ? s32_flag[p] : 0;
     const unsigned act = __activemask();
     const int key = tally_pair(bp, d, flag, s_sum, act);
+    keys[p] = key;
     // One histogram update per distinct key among the warp's lanes.
     const unsigned same = __match_any_sync(act, key);
     if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[key], __popc(same));
@@ -1145,47 +1140,32 @@ static __global__ void k_bin_count(BinParams bp, const PairDesc* __restrict__ pa
   for (int k = threadIdx.x; k < bp.nclass; k += blockDim.x) {
     if (!s_sum[k].count) continue;
     atomicAdd(&sums[k].cells, s_sum[k].cells);
-    atomicAdd(&sums[k].cost, s_sum[k].cost);
     atomicAdd(&sums[k].count, s_sum[k].count);
   }
 }
 
-// One warp: the {start, count} list range of every class, and its block
-// share -- sequential launches each take the whole GPU; concurrent ones
-// split it by modelled cost, scratch regions laid end to end.
+// One warp: the {start, count} list range of every class, and where its
+// launch may run -- on the whole GPU, in the scratch region of its stream.
 __device__ __forceinline__ void allot_classes(const BinParams& bp, const ClassSums* sums, int* class_range,
                                               ClassAllot* allot, DevStatus* st) {
   static_assert(NCLASS_MAX <= 32, "a lane per class");
   const int c = threadIdx.x & 31;
   const bool real = c < bp.nclass;
   const int count = real ? sums[c].count : 0;
-  const double cost = count > 0 ? (double)sums[c].cost : 0.0;
   int start = count;  // inclusive prefix, then exclusive
-  double total = cost;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
     const int y = __shfl_up_sync(FULL, start, off);
     if (c >= off) start += y;
-    total += __shfl_xor_sync(FULL, total, off);
   }
   start -= count;
-  int blocks = count > 0 ? bp.grid[c] : 0;
-  if (count > 0 && bp.concurrent == 1 && total > 0.0)
-    blocks = min(bp.grid[c], max(1, (int)ceil(cost / total * bp.grid[c])));
-  const long long need = real ? (long long)blocks * bp.scr_per_block[c] : 0;
-  long long base = need;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const long long y = __shfl_up_sync(FULL, base, off);
-    if (c >= off) base += y;
-  }
-  base -= need;
   if (real) {
-    base = bp.concurrent == 1 ? base : bp.concurrent == 2 ? bp.slot_of[c] * bp.region : 0;
-    if (base + need > bp.scr_cap) {
-      // Never reached when the host sized the scratch for these shares.
-      if (bp.scr_per_block[c] > 0) blocks = (int)max(0ll, (bp.scr_cap - base) / bp.scr_per_block[c]);
-      if (blocks == 0 && count > 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
+    int blocks = count > 0 ? bp.grid[c] : 0;
+    const long long base = bp.concurrent ? bp.slot_of[c] * bp.region : 0;
+    if (base + (long long)blocks * bp.scr_per_block[c] > bp.scr_cap) {
+      // Never reached when the host sized the scratch for these regions.
+      blocks = (int)max(0ll, (bp.scr_cap - base) / bp.scr_per_block[c]);
+      if (blocks == 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
     }
     class_range[2 * c] = start;
     class_range[2 * c + 1] = count;
@@ -1245,7 +1225,7 @@ static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const P
   __shared__ unsigned long long s_key[kSmallBin];  // key << 32 | pair; rejected pairs and padding last
   __shared__ ClassSums s_sum[NCLASS_MAX];
   const int tid = threadIdx.x;
-  if (tid < NCLASS_MAX) s_sum[tid] = ClassSums{0, 0, 0, 0};
+  if (tid < NCLASS_MAX) s_sum[tid] = ClassSums{0, 0, 0};
   __syncthreads();
   unsigned long long local = 0;
   for (int p = tid; p < n; p += 1024) {
@@ -1293,12 +1273,11 @@ static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const P
   if (tid < 32) allot_classes(bp, s_sum, class_range, allot, st);
 }
 
-static __global__ void k_bin_scatter(BinParams bp, const PairDesc* __restrict__ pairs, int n,
-                              const uint8_t* __restrict__ s32_flag, int* offs, int* list) {
+// keys: of every pair, as k_bin_count left them (-1: not listed).
+static __global__ void k_bin_scatter(const int* __restrict__ keys, int n, int* offs, int* list) {
   for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
-    const PairDesc d = pairs[p];
-    if (pair_state(d, bp.n_codes, bp.max_a, bp.max_b) != PAIR_OK) continue;
-    const int key = pair_key(bp, d.a_len, d.b_len, s32_flag[p], thread_cap(bp));
+    const int key = keys[p];
+    if (key < 0) continue;
     // One atomic per distinct key among the warp's lanes; each lane takes
     // the slot of its rank in the group.
     const unsigned act = __activemask();

@@ -49,6 +49,11 @@
 
 namespace ipuma_dev {
 
+// On every lambda of the pass: its arrays live in registers only if all of
+// them are inlined, which the compiler stops doing in a translation unit that
+// holds many passes.
+#define IPUMA_INLINE __attribute__((always_inline))
+
 
 __device__ __forceinline__ uint32_t add16x2(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -209,13 +214,13 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
   const uint32_t vgEp = sc.gEp2;
   const uint32_t tagMul = (uint32_t)sc.one << TB;  // 2^TB that the compiler keeps as an imad
   const int lim = T::limit(sc.maxSub);
-  const auto wbuf = [&](int s) -> int { return TEAM ? s % team.warps : s & 1; };
+  const auto wbuf = [&](int s) IPUMA_INLINE -> int { return TEAM ? s % team.warps : s & 1; };
   bool teamGaveUp = false;
   const RowLetters letter[2] = {RowLetters(sc, ps[0]), RowLetters(sc, ps[1])};
 
   // TEAM: waits until the previous warp published `need` rows of strip s's
   // boundary.  Warp-uniform; false once the team gave up (as in sw_pass).
-  auto team_wait = [&](int s, int need) -> bool {
+  auto team_wait = [&](int s, int need) IPUMA_INLINE -> bool {
     bool ok = true;
     if constexpr (TEAM) {
       const int target = (s << 16) | need;
@@ -268,7 +273,7 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
     // B letters: lane k of `bnext` holds the profile row offsets of one row
     // (pair h in halfword h), parked in the rings a block at a time.  A
     // block of steps starting at t0 reads rows up to t0 + LANES.
-    auto fetch_letters = [&](int r) -> uint32_t {
+    auto fetch_letters = [&](int r) IPUMA_INLINE -> uint32_t {
       uint32_t v = 0;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -277,7 +282,7 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
       }
       return v;
     };
-    auto park_letters = [&](int r, uint32_t v) {
+    auto park_letters = [&](int r, uint32_t v) IPUMA_INLINE {
       const int w = r & 63;
       s_bring[w] = s_bring[w + 64] = (uint16_t)v;
       s_bring[128 + w] = s_bring[192 + w] = (uint16_t)(v >> 16);
@@ -319,11 +324,11 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
     // Profile words of the row whose letters lie at `ring`, and its d from
     // the left neighbour's H of the row above, `left`.
     uint32_t wp[KP / 4], wq[KP / 4];
-    auto fetch_profile = [&](const uint16_t* ring) {
+    auto fetch_profile = [&](const uint16_t* ring) IPUMA_INLINE {
       prof.load(wp, s_prof + ring[0]);
       prof.load(wq, profQ + ring[128]);
     };
-    auto ahead = [&](uint32_t left) {
+    auto ahead = [&](uint32_t left) IPUMA_INLINE {
 #pragma unroll
       for (int c = 0; c < K; ++c) {
         uint32_t sb;
@@ -338,7 +343,7 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
     };
     // Row i's maxima; `left` and `e` are the left neighbour's HG and E of
     // this row, rows = i in both halfwords.
-    auto row = [&](int i, uint32_t rows, uint32_t left, uint32_t e, auto multi) {
+    auto row = [&](int i, uint32_t rows, uint32_t left, uint32_t e, auto multi) IPUMA_INLINE {
       uint32_t tv[K];
 #pragma unroll
       for (int c = 0; c < K; ++c) {
@@ -407,7 +412,7 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
     };
     // One wavefront step: lane works on row i = t - lane, then prepares
     // row i + 1 (rows past the end read the padding letter).
-    auto step = [&](int i, int k, uint32_t rows, const uint16_t* ring, auto check, auto multi) {
+    auto step = [&](int i, int k, uint32_t rows, const uint16_t* ring, auto check, auto multi) IPUMA_INLINE {
       uint32_t left = __shfl_up_sync(FULL, outH, 1, LANES);
       uint32_t e = ZERO;
       if constexpr (!LINEAR) e = __shfl_up_sync(FULL, outE, 1, LANES);
@@ -494,7 +499,7 @@ __device__ __forceinline__ bool tag_pass(const SwConst& sc, uint8_t* s_prof, con
       int i = t0 - lane;
       uint32_t rows = (uint32_t)i * 0x00010001u;
       const uint16_t* ring = s_bring + ((i + 1) & 63);  // slot of row i + 1, < 64 + LANES
-      auto block = [&](auto check, auto multi) {
+      auto block = [&](auto check, auto multi) IPUMA_INLINE {
 #pragma unroll 1
         for (int k = 0; k < LANES; ++k) {
           step(i, k, rows, ring, check, multi);

@@ -58,7 +58,8 @@ KERNEL_NAMES = {0: "k_batched<s32,L32,K16>", 1: "k_batched<s16x2,L16,K4>",
                 21: "k_plain16<K>", 22: "k_batched<s16x2,L8,K8>",
                 23: "k_batched<s16x2,L8,K10>", 24: "k_batched<s16x2,L8,K12>",
                 25: "k_batched<s16x2,L8,K14>", 26: "k_batched<s16x2,L8,K16>",
-                27: "k_strips<s16x2,L32,K16> team"}
+                27: "k_strips<s16x2,L32,K16> team", 28: "k_batched<s16x2,L32,K8>",
+                29: "k_batched<s16x2,L32,K4>"}
 MAX_TIMED = 24  # IPUMA_MAX_TIMED
 
 
