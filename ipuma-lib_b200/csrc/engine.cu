@@ -16,6 +16,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "errors.h"
@@ -193,6 +194,7 @@ constexpr int kValidateMaxThreads = 16;       // host threads checking pair desc
 constexpr int kValidatePairsPerThread = 65536;
 constexpr size_t kChunkMinBytes = 32u << 20;  // and the batch uploads at least this much
 constexpr int kThreads = 32 * kWarpsPerBlock;
+constexpr int kRunStreams = 4;  // streams of a run's launches (run_slots)
 
 // Status of one wire-buffer job, copied from its control block to pinned
 // host memory by the job's own stream before any later job can clear it.
@@ -272,18 +274,16 @@ struct ipuma_engine {
   // (ipuma_gpu_compare): chunks alternate between `stream` and `stream2`
   // while `copy_stream` uploads the next chunks.
   DevBuf x_list, x_scratch, x_ovf, x_flag;
-  // One stream per kernel class: the class launches of a batch run
-  // concurrently, each on its share of the SMs (option "concurrent").
-  cudaStream_t cls_stream[NCLASS_MAX] = {};
+  // Streams of the launches of a run, for either buffer set.
+  cudaStream_t cls_stream[2 * kRunStreams] = {};
   cudaEvent_t fork_ev = nullptr;
-  cudaEvent_t join_ev[NCLASS_MAX] = {};
+  cudaEvent_t join_ev[2 * kRunStreams] = {};
   int concurrent = 3;
   int hybrid = 1;  // option "hybrid": high-scoring pairs run s16x2 strips while provably safe
   float latency_weight = kLatencyWeight;  // option "latency_share" (per mille)
   cudaStream_t stream2 = nullptr, copy_stream = nullptr;
   cudaEvent_t cev[2 * kMaxChunks + 2] = {};
   int chunks = 0;  // option "chunks": 0 automatic, 1 off, n fixed
-  std::map<std::pair<const void*, int>, int> grid_cache;  // {kernel, smem} -> grid
   // Captured pipelines of compare_device, by shape and buffers (option "graphs").
   std::map<std::vector<uint64_t>, cudaGraphExec_t> graphs_cache;
   std::map<cudaGraphExec_t, int> graph_launches;
@@ -349,21 +349,23 @@ void raise_smem_limit(int device, K kernel, int smem) {
 }
 
 // Persistent grid of a kernel: resident blocks per SM times SMs.  Computed
-// once per kernel and engine (engine creation warms the cache, so no
-// occupancy query or attribute change happens during a graph capture).
+// once per device, kernel and shared memory size and kept for the process
+// (engine creation asks for every class, so no occupancy query or attribute
+// change happens during a graph capture).
 template <class K>
 int occupancy_grid(ipuma_engine* e, K kernel, int smem, int threads = kThreads) {
-  // Key: the kernel and its shared memory (and block size, when not kThreads).
-  const auto key =
-      std::make_pair(reinterpret_cast<const void*>(kernel), smem + (threads == kThreads ? 0 : threads << 20));
-  auto it = e->grid_cache.find(key);
-  if (it != e->grid_cache.end()) return it->second;
-  int nb = 0;
-  raise_smem_limit(e->device, kernel, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem);
-  if (nb < 1) nb = 1;
-  e->grid_cache[key] = nb * e->nsm;
-  return nb * e->nsm;
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, int>, int> blocks;
+  const auto key = std::make_tuple(e->device, reinterpret_cast<const void*>(kernel), smem, threads);
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = blocks.find(key);
+  if (it == blocks.end()) {
+    int nb = 0;
+    raise_smem_limit(e->device, kernel, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem);
+    it = blocks.emplace(key, std::max(nb, 1)).first;
+  }
+  return it->second * e->nsm;
 }
 
 // Letters of the query profile for codes of `bits` bits: 2-bit codes are
@@ -757,7 +759,6 @@ bool by_cost_class(int c) { return c < kNumS16 || c == kClsLat256 || c == kClsLa
 // stream 2, before k_mix (stream 1; stream 0 when no special class is
 // launched) fills what they leave.  Separate class launches alternate
 // between streams 1 and 3, so each starts on the SMs the one before frees.
-constexpr int kRunStreams = 4;
 void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
   bool special = false;
   for (int c = 0; c < kNumClasses; ++c) special |= ((enabled >> c) & 1u) && !by_cost_class(c);
@@ -772,35 +773,96 @@ void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
   }
 }
 
-// Strip-boundary scratch (int2) of one run: a region per stream, each as
-// large as any launch's full grid needs -- for the models and class sets a
-// batch of this shape may use.
-size_t scratch_int2(ipuma_engine* e, int n, int maxA, int maxB) {
-  int grid[NCLASS_MAX + 1];
-  long long spb[NCLASS_MAX + 1];
+// What a batch of n pairs launches: its classes, their kernels, streams,
+// grids and strip scratch (int2).
+struct ClassPlan {
+  int model = 0, teamW = 0;
+  unsigned enabled = 0;            // classes launched
+  bool highScores = false;         // a pair may pass the long class's scores
+  int s16_max_len = 0;             // both sequences longer: the diagonal bound decides
   KernelRef kr[kNumClasses];
-  long long full = 0;
-  for (int P : {e->M, prof_letters(e, 2)})  // the smaller profile may fit more blocks
-    for (bool eight : {false, n >= kEightLaneMinPairs}) {
-      const int model = mix_model(e, P, eight);
-      for (int c = 0; c < kNumClasses; ++c) kr[c] = kernel_of(e, c, P, model);
-      // Launches of every class alone and of all: a launch of some classes
-      // lies between (fewer columns per warp and less shared memory than
-      // all, no more blocks than the smallest alone).
-      int blocks = 0;
-      long long per = 0;
-      for (int c = 0; c < kNumClasses; ++c) {
-        class_grids(e, P, model, kr, 1u << c, maxA, maxB, grid, spb);
-        if (kr[c].mix) {
-          blocks = std::max(blocks, grid[c]);
-          per = std::max(per, spb[c]);
-        } else {
-          full = std::max(full, (long long)grid[c] * spb[c]);
-        }
-      }
-      full = std::max(full, blocks * per);
+  int slot[NCLASS_MAX + 1] = {};
+  int grid[NCLASS_MAX + 1] = {};
+  long long spb[NCLASS_MAX + 1] = {};
+  long long base[kRunStreams] = {};  // scratch region of each stream
+  long long total = 0;
+};
+
+// Longest min(|A|,|B|) class c is chosen for by cost (BinParams::fit).
+int class_fit(const ipuma_engine* e, const KernelRef& kr) { return (kr.ok() ? kr.limit : e->sc.s16Limit) / e->typical; }
+
+int plan_classes(ipuma_engine* e, int n, int P, int bits, int maxA, int maxB, ClassPlan& pl) {
+  pl.model = mix_model(e, P, n >= kEightLaneMinPairs);
+  for (int c = 0; c < kNumClasses; ++c) pl.kr[c] = kernel_of(e, c, P, pl.model);
+  const KernelRef* kr = pl.kr;
+  unsigned enabled = kCoarseClasses | kFineClasses;
+  if (n < kLatClassMaxPairs) enabled |= kLatClasses;
+  // Pairs that may pass 16 bits need both sequences longer than s16_max_len.
+  pl.s16_max_len = e->maxSub > 0 ? kr[kClsLong].limit / e->maxSub : (1 << 30);
+  pl.highScores = std::min(maxA, maxB) > pl.s16_max_len;
+  if (!e->s16_ok || (pl.highScores && !e->hybrid)) enabled |= 1u << kClsS32;
+  if (pl.highScores && e->hybrid) enabled |= (1u << kClsHi) | (1u << kClsBig);
+  // The long class, when the batch may hold a pair past the widest's scores.
+  if (std::min(maxA, maxB) > class_fit(e, kr[kClsWidest])) enabled |= 1u << kClsLong;
+  if (e->thread_class && bits == 8) enabled |= 1u << kClsThread;  // k_thread reads bytes only
+  if (P < e->M && pl.model == kMixAff) {
+    // Four-row profiles: the narrow widths in 8-lane groups.
+    for (const auto& w : kNarrowPairs)
+      if ((enabled >> w[0]) & 1u) enabled = (enabled & ~(1u << w[0])) | (1u << w[1]);
+  }
+  // Strip teams: batches with pairs of two strips or more, unless tile_k
+  // forces another class (then no pair could reach a team).
+  pl.teamW = e->team_warps >= 2 ? team_warps_for(e, P, maxA) : 0;
+  if (e->tile_k == kClsTeam + 1 && pl.teamW < 2)
+    return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d (strip teams) needs team_warps >= 2 and room for two warps",
+                kClsTeam + 1);
+  if (pl.teamW >= 2 && maxA > kClasses[kClsTeam].width && e->tile_k == 0) enabled |= 1u << kClsTeam;
+  if (e->tile_k > 0) {  // no pair is given to a class by cost
+    for (int c = 0; c < kNumClasses; ++c)
+      if (by_cost_class(c)) enabled &= ~(1u << c);
+    enabled |= 1u << (e->tile_k - 1);
+  }
+  if (((enabled >> kClsTeam) & 1u) && ((enabled >> kClsBig) & 1u)) enabled |= 1u << kClsBigTeam;
+  for (int c = 0; c < kNumClasses; ++c)
+    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].ok()) {
+      if (e->tile_k == c + 1) return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d has no kernel for this scoring", e->tile_k);
+      enabled &= ~(1u << c);
     }
-  return (size_t)(kRunStreams * full);
+  pl.enabled = enabled;
+  run_slots(kr, enabled, pl.slot);
+  class_grids(e, P, pl.model, kr, enabled, maxA, maxB, pl.grid, pl.spb);
+  // A region per stream in use, as large as its largest launch (a class
+  // timed alone may have a larger grid than k_mix of all: the largest grid
+  // and the largest column count together hold both).  The s32 rerun follows
+  // all of them.
+  long long size[kRunStreams] = {};
+  int mixGrid = 0;
+  for (int c = 0; c < kNumClasses; ++c) {
+    if (!((enabled >> c) & 1u)) continue;
+    if (pl.kr[c].mix) mixGrid = std::max(mixGrid, kernel_grid(e, kr[c], P, pl.model));
+  }
+  for (int c = 0; c < kNumClasses; ++c) {
+    if (!((enabled >> c) & 1u)) continue;
+    const long long need = std::max(pl.grid[c], kr[c].mix ? mixGrid : 0) * pl.spb[c];
+    size[pl.slot[c]] = std::max(size[pl.slot[c]], need);
+  }
+  for (int k = 0; k < kRunStreams; ++k) {
+    pl.base[k] = pl.total;
+    pl.total += size[k];
+  }
+  pl.total = std::max(pl.total, pl.grid[kClsS32] * pl.spb[kClsS32]);
+  return IPUMA_OK;
+}
+
+// Strip-boundary scratch (int2) a batch of this shape may need, for byte or
+// packed codes.
+size_t scratch_int2(ipuma_engine* e, int n, int maxA, int maxB) {
+  long long total = 0;
+  for (int bits : {8, 2}) {
+    ClassPlan pl;
+    if (plan_classes(e, n, prof_letters(e, bits), bits, maxA, maxB, pl) == IPUMA_OK) total = std::max(total, pl.total);
+  }
+  return (size_t)total;
 }
 
 int reserve_bufs(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, int n, int maxA, int maxB) {
@@ -852,9 +914,13 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
 
   // Scratch for strip boundaries and the lists.
   const long rowsCap = std::max(1, maxB);
-  if ((rc = rb.scratch->ensure(sizeof(int2) * scratch_int2(e, n, maxA, maxB), s))) return rc;
+  ClassPlan pl;
+  if ((rc = plan_classes(e, n, sc.P, bits, maxA, maxB, pl))) return rc;
+  if ((rc = rb.scratch->ensure(sizeof(int2) * (size_t)pl.total, s))) return rc;
   if ((rc = rb.list->ensure(sizeof(int) * (size_t)n + 64, s))) return rc;
   if ((rc = rb.ovf->ensure(sizeof(int) * (size_t)n + 64, s))) return rc;
+  const KernelRef* kr = pl.kr;
+  const unsigned enabled = pl.enabled;
 
   BinParams bp{};
   bp.cls_s32 = kClsS32;
@@ -862,21 +928,19 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.cls_big = e->hybrid ? kClsBig : kClsS32;
   bp.nclass = kNumClasses;
   bp.force_s32 = e->s16_ok ? 0 : 1;
-  const bool eight = n >= kEightLaneMinPairs;
-  const int model = mix_model(e, sc.P, eight);
-  KernelRef kr[kNumClasses];
   for (int c = 0; c < kNumClasses; ++c) {
-    kr[c] = kernel_of(e, c, sc.P, model);
     bp.lanes[c] = kr[c].ok() ? kr[c].lanes : kClasses[c].lanes;
     bp.width[c] = kClasses[c].width;
     bp.inv_width[c] = (unsigned)(((1ull << 32) + kClasses[c].width - 1) / kClasses[c].width);
     bp.slot_ps[c] = e->slot_ps[c];
     bp.strip_ps[c] = e->strip_ps[c];
-    bp.fit[c] = (kr[c].ok() ? kr[c].limit : e->sc.s16Limit) / e->typical;
+    bp.fit[c] = class_fit(e, kr[c]);
+    bp.grid[c] = pl.grid[c];
+    bp.scr_per_block[c] = pl.spb[c];
   }
   bp.widest = kClsWidest;
   bp.cls_long = kClsLong;
-  bp.s16_max_len = e->maxSub > 0 ? kr[kClsLong].limit / e->maxSub : (1 << 30);
+  bp.s16_max_len = pl.s16_max_len;
   const long thrThreads = thread_threads<16>(e);
   bp.thr_cls = kClsThread;
   bp.thr_on = e->thread_class && bits == 8;
@@ -886,49 +950,12 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.total_cells = reinterpret_cast<const unsigned long long*>(ctl + CTL_CELLS) + CELLS_TOTAL;
   // Concurrent launches, except when every launch is timed alone.
   const bool conc = !e->time_launches && e->concurrent != 0;
-  bp.concurrent = conc ? 1 : 0;
-  // Classes this batch may use (the others are not launched).
-  unsigned enabled = kCoarseClasses;
-  // Pairs that may pass 16 bits need both sequences longer than s16_max_len.
-  const bool highScores = std::min(maxA, maxB) > bp.s16_max_len;
-  if (!e->s16_ok || (highScores && !e->hybrid)) enabled |= 1u << kClsS32;
-  if (highScores && e->hybrid) enabled |= (1u << kClsHi) | (1u << kClsBig);
-  enabled |= kFineClasses;
-  if (n < kLatClassMaxPairs) enabled |= kLatClasses;
-  // The long class, when the batch may hold a pair past the widest's scores.
-  if (std::min(maxA, maxB) > bp.fit[kClsWidest]) enabled |= 1u << kClsLong;
-  if (e->thread_class && bits == 8) enabled |= 1u << kClsThread;  // k_thread reads bytes only
-  if (sc.P < e->M && model == kMixAff) {
-    // Four-row profiles: the narrow widths in 8-lane groups.
-    for (const auto& w : kNarrowPairs)
-      if ((enabled >> w[0]) & 1u) enabled = (enabled & ~(1u << w[0])) | (1u << w[1]);
-  }
-  // Strip teams: batches with pairs of two strips or more, unless tile_k
-  // forces another class (then no pair could reach a team).
-  const bool teamForced = e->tile_k == kClsTeam + 1;
-  const int teamW = e->team_warps >= 2 ? team_warps_for(e, sc.P, maxA) : 0;
-  if (teamForced && teamW < 2)
-    return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d (strip teams) needs team_warps >= 2 and room for two warps",
-                kClsTeam + 1);
-  if (teamW >= 2 && maxA > kClasses[kClsTeam].width && e->tile_k == 0) enabled |= 1u << kClsTeam;
-  if (e->tile_k > 0) {  // no pair is given to a class by cost
-    for (int c = 0; c < kNumClasses; ++c)
-      if (by_cost_class(c)) enabled &= ~(1u << c);
-    enabled |= 1u << (e->tile_k - 1);
-  }
-  if (((enabled >> kClsTeam) & 1u) && ((enabled >> kClsBig) & 1u)) enabled |= 1u << kClsBigTeam;
-  for (int c = 0; c < kNumClasses; ++c)
-    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].ok()) {
-      if (e->tile_k == c + 1) return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d has no kernel for this scoring", e->tile_k);
-      enabled &= ~(1u << c);
-    }
   bp.enabled = enabled;
   for (int c = 0; c < kNumClasses; ++c)
     if (((enabled >> c) & 1u) && by_cost_class(c)) bp.by_cost |= 1u << c;
   bp.team_cls = ((enabled >> kClsTeam) & 1u) ? kClsTeam : -1;
   bp.team_big = ((enabled >> kClsBigTeam) & 1u) ? kClsBigTeam : -1;
-  bp.team_warps = std::max(teamW, 1);
-  class_grids(e, sc.P, model, kr, e->time_launches ? 0u : enabled, maxA, maxB, bp.grid, bp.scr_per_block);
+  bp.team_warps = std::max(pl.teamW, 1);
   bp.scr_cap = (long long)(rb.scratch->cap / sizeof(int2));
   float slot_min = 1e30f;
   for (int c = 0; c < kNumClasses; ++c) {
@@ -936,7 +963,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     // cell slots one warp step covers: 32 lanes x k columns x 2 pairs
     // (the per-thread class: 32 threads x 16 columns x 2 pairs per row)
     const int k = kr[c].ok() ? kr[c].k : kClasses[c].k;
-    const int grid = kr[c].mix ? kernel_grid(e, kr[c], sc.P, model) : bp.grid[c];
+    const int grid = kr[c].mix ? kernel_grid(e, kr[c], sc.P, pl.model) : bp.grid[c];
     bp.step_ps[c] = step_time(e->slot_ps[c] * 64.f * (float)k * (float)(grid * kWarpsPerBlock), k, n, grid);
     if (((bp.by_cost >> c) & 1u) && kr[c].ok()) slot_min = std::min(slot_min, e->slot_ps[c]);
   }
@@ -946,8 +973,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.batch_ps_per_cell = slot_min / kPackingEfficiency;
   bp.lat_weight = e->latency_weight;
   bp.team_share = e->sc.forwardOnly ? kTeamShareForward : kTeamShareFull;
-  bp.region = bp.scr_cap / kRunStreams;
-  run_slots(kr, enabled, bp.slot_of);
+  for (int c = 0; c < kNumClasses; ++c) bp.base[c] = conc ? pl.base[pl.slot[c]] : 0;
   bp.long_a = e->long_a;
   // tile_k > 0 forces one s16x2 class: every pair uses the chosen kernel,
   // long A crossing several strips.
@@ -967,7 +993,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   auto* sums = reinterpret_cast<ClassSums*>(ctl + CTL_SUMS);
   auto* allot = reinterpret_cast<ClassAllot*>(ctl + CTL_ALLOT);
   uint8_t* flags = rb.flag->as<uint8_t>();
-  if (highScores) {  // without long pairs no flag is read
+  if (pl.highScores) {  // without long pairs no flag is read
     k_bin_bound<<<gb, tb, 0, s>>>(bp, codes, e->d_sim.as<int8_t>(), pairs, n, flags);
     *launches += 1;
   }
@@ -1004,16 +1030,16 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   unsigned mixMask = 0;
   for (const int c : kLaunchOrder) {
     if (!((enabled >> c) & 1u)) continue;
-    cudaStream_t cs = kr[c].mix && !e->time_launches ? s : on(bp.slot_of[c]);
+    cudaStream_t cs = kr[c].mix && !e->time_launches ? s : on(pl.slot[c]);
     if (c == kClsTeam || c == kClsBigTeam) {
-      rc = launch_team(e, sc, rb, cs, io, list, R + 2 * c, heads + c, teamW, c);
+      rc = launch_team(e, sc, rb, cs, io, list, R + 2 * c, heads + c, pl.teamW, c);
     } else if (c == kClsThread) {
       rc = launch_thread<16>(e, rb, cs, codes, pairs, list, R + 2 * c, heads + c, thread_rows(e, maxA, maxB), score,
                              arange, brange, c);
     } else if (!kr[c].mix) {
       rc = launch_batched(e, kr[c], sc, rb, cs, io, list, R + 2 * c, heads + c, kClasses[c].kind, c, c);
     } else if (e->time_launches) {  // a timed launch per class
-      rc = launch_mix(e, model, kr[c].shift, mix_args(kr, 1u << c, rowsCap), sc, rb, cs, 0, io, list, R, heads,
+      rc = launch_mix(e, pl.model, kr[c].shift, mix_args(kr, 1u << c, rowsCap), sc, rb, cs, 0, io, list, R, heads,
                       kClasses[c].kind, c);
     } else {
       mixMask |= 1u << c;
@@ -1024,8 +1050,8 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   }
   if (mixMask) {
     const int c = __builtin_ctz(mixMask);
-    if ((rc = launch_mix(e, model, kr[c].shift, mix_args(kr, mixMask, rowsCap), sc, rb, on(bp.slot_of[c]),
-                         conc ? bp.slot_of[c] * bp.region : 0, io, list, R, heads, kClasses[c].kind, c)))
+    if ((rc = launch_mix(e, pl.model, kr[c].shift, mix_args(kr, mixMask, rowsCap), sc, rb, on(pl.slot[c]),
+                         bp.base[c], io, list, R, heads, kClasses[c].kind, c)))
       return rc;
     ++*launches;
   }
@@ -1788,7 +1814,7 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   // Class streams and their fork/join events (created here: no stream or
   // event is created while a stream is being captured).
   CUDA_TRY(cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming));
-  for (int c = 0; c < NCLASS_MAX; ++c) {
+  for (int c = 0; c < 2 * kRunStreams; ++c) {
     CUDA_TRY(cudaStreamCreateWithFlags(&e->cls_stream[c], cudaStreamNonBlocking));
     CUDA_TRY(cudaEventCreateWithFlags(&e->join_ev[c], cudaEventDisableTiming));
   }
@@ -1873,7 +1899,7 @@ void ipuma_gpu_destroy(ipuma_engine* e) {
   if (e->h_ctl) cudaFreeHost(e->h_ctl);
   for (auto& ev : e->cev)
     if (ev) cudaEventDestroy(ev);
-  for (int c = 0; c < NCLASS_MAX; ++c) {
+  for (int c = 0; c < 2 * kRunStreams; ++c) {
     if (e->cls_stream[c]) cudaStreamSynchronize(e->cls_stream[c]);
     if (e->cls_stream[c]) cudaStreamDestroy(e->cls_stream[c]);
     if (e->join_ev[c]) cudaEventDestroy(e->join_ev[c]);

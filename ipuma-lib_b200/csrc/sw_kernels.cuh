@@ -837,12 +837,10 @@ struct BinParams {
   // latency to a fraction of the batch's time (thr_cap_scale = fraction /
   // pair slots the class keeps resident).
   unsigned int enabled;    // bit c: class c may be chosen by cost (and is launched)
-  // Concurrent launches: full-occupancy grid and strip scratch (int2) per
-  // block of each class, the scratch region of its stream, and the scratch
+  // Full-occupancy grid and strip scratch (int2) per block of each class,
+  // where its launch's scratch starts (a region per stream), and the scratch
   // available.
-  int concurrent;          // 0: one launch after the other
-  int slot_of[NCLASS_MAX + 1];
-  long long region;        // int2 per region
+  long long base[NCLASS_MAX + 1];
   int grid[NCLASS_MAX + 1];
   long long scr_per_block[NCLASS_MAX + 1];
   long long scr_cap;
@@ -1161,10 +1159,10 @@ __device__ __forceinline__ void allot_classes(const BinParams& bp, const ClassSu
   start -= count;
   if (real) {
     int blocks = count > 0 ? bp.grid[c] : 0;
-    const long long base = bp.concurrent ? bp.slot_of[c] * bp.region : 0;
+    const long long base = bp.base[c];
     if (base + (long long)blocks * bp.scr_per_block[c] > bp.scr_cap) {
       // Never reached when the host sized the scratch for these regions.
-      blocks = (int)max(0ll, (bp.scr_cap - base) / bp.scr_per_block[c]);
+      blocks = (int)max(0ll, (bp.scr_cap - base) / max(bp.scr_per_block[c], 1ll));
       if (blocks == 0) atomicCAS(&st->error, 0, ERR_SCRATCH);
     }
     class_range[2 * c] = start;
