@@ -121,8 +121,8 @@ typedef struct ipuma_stats {
   double total_ms;      /* device time including copies                      */
   int64_t cells;        /* sum of |A|*|B| (forward pass, ipuma's definition) */
   int64_t pairs;
-  int64_t s32_pairs;    /* pairs the binning sent to the s32 or hybrid class
-                           (main-diagonal score above the 16-bit limit)      */
+  int64_t s32_pairs;    /* pairs whose main-diagonal score passes the 16-bit
+                           limit (s32, hybrid or big class, or its teams)    */
   int64_t overflow_reruns; /* s16x2 pairs that were rerun in 32-bit          */
   int32_t launches;     /* kernels launched by the call                      */
   int32_t used_graph;   /* 1 when the call replayed a captured CUDA graph     */
@@ -152,8 +152,9 @@ typedef struct ipuma_stats {
 } ipuma_stats;
 
 /* Kernel kinds reported in ipuma_stats.timed_kind.  S16_L<lanes>_K<k>:
- * s16x2 lanes (two pairs per lane group), <lanes> lanes per group, <k> A
- * columns per lane. */
+ * 16-bit halves (two pairs per lane group), <lanes> lanes per group, <k> A
+ * columns per lane; 2-bit batches of 150,000 pairs and more with gap_init 0
+ * run the S16_L16_K<k> strips as 8 lanes of 2 k columns. */
 #define IPUMA_KERNEL_S32_K16 0     /* s32 lanes, 32 lanes, 16 columns       */
 #define IPUMA_KERNEL_S16_L16_K4 1
 #define IPUMA_KERNEL_S16_L16_K8 2
@@ -174,8 +175,8 @@ typedef struct ipuma_stats {
 #define IPUMA_KERNEL_S16_L16_K11 17
 #define IPUMA_KERNEL_S16_L16_K13 18
 #define IPUMA_KERNEL_S16_L16_K15 19
-#define IPUMA_KERNEL_S16_HYBRID 20 /* scores above int16: strips in biased 16-bit halves (score - 31744,
-                                      scores up to 65535 - 1024 - max(sim)) while safe, then s32 */
+#define IPUMA_KERNEL_S16_HYBRID 20 /* scores above int16: biased 16-bit halves (the big class, scores up to
+                                      about 64,000); past that strips in biased halves while safe, then s32 */
 #define IPUMA_KERNEL_PLAIN_S16 21  /* one-launch-per-batch wire kernel, 16-bit lanes */
 /* 8-lane groups (four per warp), used instead of S16_L16_K4 .. _K8 of the
  * same strip widths when the codes are 2-bit (four-row profiles) */

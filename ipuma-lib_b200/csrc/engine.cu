@@ -972,7 +972,9 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * bp.team_warps);
   bp.batch_ps_per_cell = slot_min / kPackingEfficiency;
   bp.lat_weight = e->latency_weight;
-  bp.team_share = e->sc.forwardOnly ? kTeamShareForward : kTeamShareFull;
+  // Pairs the widest strips' resident warps hold, two each.
+  const int resident = 2 * kWarpsPerBlock * bp.grid[kClsWidest];
+  bp.team_share = n < resident ? kTeamShareSmall : kTeamShareLarge;
   for (int c = 0; c < kNumClasses; ++c) bp.base[c] = conc ? pl.base[pl.slot[c]] : 0;
   bp.long_a = e->long_a;
   // tile_k > 0 forces one s16x2 class: every pair uses the chosen kernel,

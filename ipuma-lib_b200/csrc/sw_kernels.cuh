@@ -818,7 +818,7 @@ struct BinParams {
   float step_ps[NCLASS_MAX];
   float batch_ps_per_cell;     // modelled batch time per cell (strip teams)
   float lat_weight;
-  float team_share;            // kTeamShareForward or kTeamShareFull
+  float team_share;            // kTeamShareSmall or kTeamShareLarge
   int long_a;                  // |A| above which the widest strips are used
   int widest;                  // class of the widest strips
   int cls_long;                // the same strips with room for the longest scores (past fit[widest])
@@ -916,14 +916,15 @@ static __device__ int warp_diagonal_bound(const uint8_t* codes, int bits, long l
 }
 
 // A pair goes to a strip team when its one-warp latency passes this many
-// times the batch's modelled time: below it the other pairs' work hides the
-// pair, and a team's fill and idle warps only cost throughput (B200, at 0.5
-// / 1 / 1.5 / 2.5: 12,000 proteins 1.64 / 1.18 / 1.17 / 1.62 ms, 8,000
-// heavy-tailed 16.3 / 16.6 / 11.5 / 11.5, 60,000 22.7 / 22.7 / 21.5 / 37.3,
-// 700 pairs of 2,000-2,500 2.69 / 2.68 / 2.69 / 4.20).  With start
-// coordinates a team costs more -- its reverse pass has no early stop -- and
-// the line lies higher (4,006 proteins 2.01 ms at 1.5, 1.43 at 2.5).
-constexpr float kTeamShareForward = 1.5f, kTeamShareFull = 2.5f;
+// times the batch's modelled time (BinParams::team_share): below it the
+// other pairs' work hides the pair, and a team's fill and idle warps only
+// cost throughput -- its block also keeps k_mix off the SM.  The line lies
+// lower when the batch has fewer pairs than the widest strips' warps hold,
+// since then no other work fills the rest.  (B200, line at 1.5 / 1.8 / 2.2:
+// 1,000 pairs of 1,600-2,000, too few to fill the GPU, 1.37 / 2.50 / 2.56
+// ms; 4,006 proteins 0.97 / 0.67 / 0.66; 20,011 1.48 / 1.71 / 2.06; 60,000
+// heavy-tailed proteins 22.7 at 0.5, 21.5 at 1.5, 37.3 at 2.5.)
+constexpr float kTeamShareSmall = 1.0f, kTeamShareLarge = 1.8f;
 
 // Class of a pair: the kernel with the lowest modelled time
 //   strips * ((|B| + lanes) * width * slot_ps + strip_ps)
