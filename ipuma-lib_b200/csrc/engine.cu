@@ -276,7 +276,7 @@ struct ipuma_engine {
   DevBuf x_list, x_scratch, x_ovf, x_flag;
   // Streams of the launches of a run, for either buffer set.
   cudaStream_t cls_stream[2 * kRunStreams] = {};
-  cudaEvent_t fork_ev = nullptr;
+  cudaEvent_t fork_ev = nullptr, gate_ev = nullptr;
   cudaEvent_t join_ev[2 * kRunStreams] = {};
   int concurrent = 3;
   int hybrid = 1;  // option "hybrid": high-scoring pairs run s16x2 strips while provably safe
@@ -755,9 +755,10 @@ void class_grids(ipuma_engine* e, int P, int model, const KernelRef* kr, unsigne
 bool by_cost_class(int c) { return c < kNumS16 || c == kClsLat256 || c == kClsLat128; }
 
 // Streams (and scratch regions) of a batch's launches.  The long pairs go
-// first: strip teams on the run's own stream 0, the other special classes on
-// stream 2, before k_mix (stream 1; stream 0 when no special class is
-// launched) fills what they leave.  Separate class launches alternate
+// first: the big strip teams on the run's own stream 0, the other teams on
+// stream 3 (their blocks start as the big ones leave SMs), the other special
+// classes on stream 2, before k_mix (stream 1; stream 0 when no special class
+// is launched) fills what they leave.  Separate class launches alternate
 // between streams 1 and 3, so each starts on the SMs the one before frees.
 void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
   bool special = false;
@@ -765,7 +766,7 @@ void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
   int pos = 0;
   for (const int c : kLaunchOrder) {
     if (!by_cost_class(c))
-      slot[c] = c == kClsTeam || c == kClsBigTeam ? 0 : 2;
+      slot[c] = c == kClsBigTeam ? 0 : c != kClsTeam ? 2 : (enabled >> kClsBigTeam) & 1u ? 3 : 0;
     else if (kr[c].mix || c == kClsThread)
       slot[c] = special ? 1 : 0;
     else
@@ -974,7 +975,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.lat_weight = e->latency_weight;
   // Pairs the widest strips' resident warps hold, two each.
   const int resident = 2 * kWarpsPerBlock * bp.grid[kClsWidest];
-  bp.team_share = n < resident ? kTeamShareSmall : kTeamShareLarge;
+  bp.team_slack = n < resident ? 0.f : kTeamSlackPs;
   for (int c = 0; c < kNumClasses; ++c) bp.base[c] = conc ? pl.base[pl.slot[c]] : 0;
   bp.long_a = e->long_a;
   // tile_k > 0 forces one s16x2 class: every pair uses the chosen kernel,
@@ -1033,6 +1034,13 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   for (const int c : kLaunchOrder) {
     if (!((enabled >> c) & 1u)) continue;
     cudaStream_t cs = kr[c].mix && !e->time_launches ? s : on(pl.slot[c]);
+    // k_mix is held until the long class is next on its stream: ready
+    // together, the stream's priority starts the long pairs first.  (Behind
+    // k_mix they ended 60,000 heavy-tailed proteins alone: 24.6 ms.)
+    if (conc && c == kClsLong) {
+      CUDA_TRY(cudaEventRecord(e->gate_ev, cs));
+      CUDA_TRY(cudaStreamWaitEvent(on(1), e->gate_ev, 0));
+    }
     if (c == kClsTeam || c == kClsBigTeam) {
       rc = launch_team(e, sc, rb, cs, io, list, R + 2 * c, heads + c, pl.teamW, c);
     } else if (c == kClsThread) {
@@ -1816,8 +1824,12 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   // Class streams and their fork/join events (created here: no stream or
   // event is created while a stream is being captured).
   CUDA_TRY(cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming));
+  CUDA_TRY(cudaEventCreateWithFlags(&e->gate_ev, cudaEventDisableTiming));
+  int prLow = 0, prHigh = 0;  // k_mix's stream (1) last, the long pairs' first
+  CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prLow, &prHigh));
   for (int c = 0; c < 2 * kRunStreams; ++c) {
-    CUDA_TRY(cudaStreamCreateWithFlags(&e->cls_stream[c], cudaStreamNonBlocking));
+    CUDA_TRY(cudaStreamCreateWithPriority(&e->cls_stream[c], cudaStreamNonBlocking,
+                                          c % kRunStreams == 1 ? prLow : prHigh));
     CUDA_TRY(cudaEventCreateWithFlags(&e->join_ev[c], cudaEventDisableTiming));
   }
 
@@ -1907,6 +1919,7 @@ void ipuma_gpu_destroy(ipuma_engine* e) {
     if (e->join_ev[c]) cudaEventDestroy(e->join_ev[c]);
   }
   if (e->fork_ev) cudaEventDestroy(e->fork_ev);
+  if (e->gate_ev) cudaEventDestroy(e->gate_ev);
   if (e->stream2) cudaStreamDestroy(e->stream2);
   if (e->wstream1) cudaStreamDestroy(e->wstream1);
   if (e->copy_stream) cudaStreamDestroy(e->copy_stream);

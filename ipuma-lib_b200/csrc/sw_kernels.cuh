@@ -429,7 +429,10 @@ constexpr float kTeamLagSteps = 64.f;
 
 // Warps per team: the divisor of the block's warps (down to a quarter, two
 // at least) that finishes `items` items like the list's first, its longest,
-// soonest -- rounds of items times the steps of one item.
+// soonest -- rounds of items times the steps of one item.  A smaller team
+// has to win by a twentieth: with 150 items on 148 blocks teams of four tie
+// with teams of eight, but keep every SM half idle for the whole time where
+// eight leave all but two SMs to the next launches after half of it.
 __device__ __forceinline__ int team_size(int warps, long blocks, int items, int strips, int rows) {
   int best = warps;
   float bestCost = 3.0e38f;
@@ -438,7 +441,7 @@ __device__ __forceinline__ int team_size(int warps, long blocks, int items, int 
     const float cost = (float)((items + slots - 1) / slots) *
                        ((float)((strips + t - 1) / t) * (float)(rows + 32) +
                         kTeamLagSteps * (float)(min(strips, t) - 1));
-    if (cost < bestCost) {
+    if (cost < 0.95f * bestCost) {
       bestCost = cost;
       best = t;
     }
@@ -818,7 +821,7 @@ struct BinParams {
   float step_ps[NCLASS_MAX];
   float batch_ps_per_cell;     // modelled batch time per cell (strip teams)
   float lat_weight;
-  float team_share;            // kTeamShareSmall or kTeamShareLarge
+  float team_slack;            // kTeamSlackPs, or 0 for a batch that leaves warps idle
   int long_a;                  // |A| above which the widest strips are used
   int widest;                  // class of the widest strips
   int cls_long;                // the same strips with room for the longest scores (past fit[widest])
@@ -915,16 +918,17 @@ static __device__ int warp_diagonal_bound(const uint8_t* codes, int bits, long l
   return __shfl_sync(FULL, r.best, 0);
 }
 
-// A pair goes to a strip team when its one-warp latency passes this many
-// times the batch's modelled time (BinParams::team_share): below it the
+// A pair goes to a strip team when its one-warp latency passes the batch's
+// modelled time plus this many ps (BinParams::team_slack): below it the
 // other pairs' work hides the pair, and a team's fill and idle warps only
-// cost throughput -- its block also keeps k_mix off the SM.  The line lies
-// lower when the batch has fewer pairs than the widest strips' warps hold,
-// since then no other work fills the rest.  (B200, line at 1.5 / 1.8 / 2.2:
-// 1,000 pairs of 1,600-2,000, too few to fill the GPU, 1.37 / 2.50 / 2.56
-// ms; 4,006 proteins 0.97 / 0.67 / 0.66; 20,011 1.48 / 1.71 / 2.06; 60,000
-// heavy-tailed proteins 22.7 at 0.5, 21.5 at 1.5, 37.3 at 2.5.)
-constexpr float kTeamShareSmall = 1.0f, kTeamShareLarge = 1.8f;
+// cost throughput -- its block also keeps k_mix off the SM.  The slack is
+// what a batch that fills the GPU takes beside its cells; a batch of fewer
+// pairs than the widest strips' warps hold has none, since no other work
+// fills the rest.  (B200: 1,000 pairs of 1,600-2,000, too few to fill the
+// GPU, ran 1.35 ms with every pair in a team, 2.5 without; 4,006 proteins
+// 0.97 ms with pairs from 700 residues in teams, 0.67 from 900; 60,000
+// heavy-tailed proteins 28 ms with the line at 1.8 times their time.)
+constexpr float kTeamSlackPs = 2.5e8f;
 
 // Class of a pair: the kernel with the lowest modelled time
 //   strips * ((|B| + lanes) * width * slot_ps + strip_ps)
@@ -940,14 +944,14 @@ __device__ __forceinline__ int strips_of(const BinParams& bp, int c, int alen) {
 
 // A strip team's class `tc` for a pair whose one-warp latency is `lat`, or
 // cls: taken when even the fastest warp would take a large share of the
-// whole batch's modelled time (team_share: below it the other pairs'
+// whole batch's modelled time (kTeamSlackPs: below it the other pairs'
 // work hides the pair, and a team's fill and idle warps only cost
 // throughput) and the team finishes the pair sooner.  Its warps take the
 // strips round robin, each starting about kTeamLagSteps behind the warp
 // before it.
 __device__ __forceinline__ int team_class(const BinParams& bp, int cls, int tc, int alen, int blen, float lat,
                                           float batch_ps) {
-  if (tc < 0 || lat <= bp.team_share * batch_ps) return cls;
+  if (tc < 0 || lat <= batch_ps + bp.team_slack) return cls;
   const int strips = strips_of(bp, tc, alen);
   if (strips < 2) return cls;
   const int rounds = (strips + bp.team_warps - 1) / bp.team_warps;
