@@ -194,7 +194,8 @@ constexpr int kValidateMaxThreads = 16;       // host threads checking pair desc
 constexpr int kValidatePairsPerThread = 65536;
 constexpr size_t kChunkMinBytes = 32u << 20;  // and the batch uploads at least this much
 constexpr int kThreads = 32 * kWarpsPerBlock;
-constexpr int kRunStreams = 4;  // streams of a run's launches (run_slots)
+// Streams of a run's launches (run_slots).
+enum RunSlot { kSlotRun, kSlotMix, kSlotLong, kSlotAlt, kSlotBig, kSlotHi, kSlotTeam, kRunStreams };
 
 // Status of one wire-buffer job, copied from its control block to pinned
 // host memory by the job's own stream before any later job can clear it.
@@ -755,22 +756,27 @@ void class_grids(ipuma_engine* e, int P, int model, const KernelRef* kr, unsigne
 bool by_cost_class(int c) { return c < kNumS16 || c == kClsLat256 || c == kClsLat128; }
 
 // Streams (and scratch regions) of a batch's launches.  The long pairs go
-// first: the big strip teams on the run's own stream 0, the other teams on
-// stream 3 (their blocks start as the big ones leave SMs), the other special
-// classes on stream 2, before k_mix (stream 1; stream 0 when no special class
-// is launched) fills what they leave.  Separate class launches alternate
-// between streams 1 and 3, so each starts on the SMs the one before frees.
+// first, the (big) strip teams on the run's own stream.  Every class of long
+// pairs has a stream to itself: one pair of 14,000 residues keeps a warp of
+// the hybrid class busy for 86 ms, which nothing may queue behind.  k_mix
+// (kSlotMix; the run's own stream when no other class is launched) fills what
+// they leave.  Separate class launches alternate between two streams, so each
+// starts on the SMs the one before frees.
 void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
   bool special = false;
   for (int c = 0; c < kNumClasses; ++c) special |= ((enabled >> c) & 1u) && !by_cost_class(c);
+  const int rest = special ? kSlotMix : kSlotRun;
   int pos = 0;
   for (const int c : kLaunchOrder) {
-    if (!by_cost_class(c))
-      slot[c] = c == kClsBigTeam ? 0 : c != kClsTeam ? 2 : (enabled >> kClsBigTeam) & 1u ? 3 : 0;
-    else if (kr[c].mix || c == kClsThread)
-      slot[c] = special ? 1 : 0;
-    else
-      slot[c] = ((enabled >> c) & 1u) && (pos++ & 1) ? 3 : special ? 1 : 0;
+    switch (c) {
+      case kClsBigTeam: slot[c] = kSlotRun; break;
+      case kClsTeam: slot[c] = (enabled >> kClsBigTeam) & 1u ? kSlotTeam : kSlotRun; break;
+      case kClsLong: slot[c] = kSlotLong; break;
+      case kClsHi: slot[c] = kSlotHi; break;
+      case kClsBig: case kClsS32: slot[c] = kSlotBig; break;  // never both hold pairs
+      default:
+        slot[c] = !kr[c].mix && c != kClsThread && ((enabled >> c) & 1u) && (pos++ & 1) ? kSlotAlt : rest;
+    }
   }
 }
 
@@ -1019,12 +1025,11 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   const int* R = ctl + CTL_RANGES;
   const BatchIo io = batch_io(rb, codes, pairs, rowsCap, score, arange, brange);
   // Launches: the long pairs' first, then k_mix over the other classes, on
-  // up to three streams (or one after the other on `s`).
+  // the streams of run_slots (or one after the other on `s`).
   if (conc) CUDA_TRY(cudaEventRecord(e->fork_ev, s));
   bool used[kRunStreams] = {};
-  // Streams of a run: 0 is `s` itself.
   auto on = [&](int slot) -> cudaStream_t {
-    if (!conc || slot == 0) return s;
+    if (!conc || slot == kSlotRun) return s;
     cudaStream_t cs = e->cls_stream[rb.cls_base + slot];
     if (!used[slot]) cudaStreamWaitEvent(cs, e->fork_ev, 0);
     used[slot] = true;
@@ -1034,12 +1039,13 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   for (const int c : kLaunchOrder) {
     if (!((enabled >> c) & 1u)) continue;
     cudaStream_t cs = kr[c].mix && !e->time_launches ? s : on(pl.slot[c]);
-    // k_mix is held until the long class is next on its stream: ready
-    // together, the stream's priority starts the long pairs first.  (Behind
-    // k_mix they ended 60,000 heavy-tailed proteins alone: 24.6 ms.)
+    // The classes by cost are held until the long class is next on its
+    // stream, which waits for nothing but the binning: ready together, the
+    // streams' priority starts the long pairs first.
     if (conc && c == kClsLong) {
       CUDA_TRY(cudaEventRecord(e->gate_ev, cs));
-      CUDA_TRY(cudaStreamWaitEvent(on(1), e->gate_ev, 0));
+      CUDA_TRY(cudaStreamWaitEvent(on(kSlotMix), e->gate_ev, 0));
+      if (pl.model == kSepLin8) CUDA_TRY(cudaStreamWaitEvent(on(kSlotAlt), e->gate_ev, 0));
     }
     if (c == kClsTeam || c == kClsBigTeam) {
       rc = launch_team(e, sc, rb, cs, io, list, R + 2 * c, heads + c, pl.teamW, c);
@@ -1825,11 +1831,15 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   // event is created while a stream is being captured).
   CUDA_TRY(cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming));
   CUDA_TRY(cudaEventCreateWithFlags(&e->gate_ev, cudaEventDisableTiming));
-  int prLow = 0, prHigh = 0;  // k_mix's stream (1) last, the long pairs' first
+  // The streams of long pairs start their blocks first (the run's own stream
+  // has the priority the caller gave it): behind k_mix the long pairs ended
+  // 60,000 heavy-tailed proteins alone, 24.6 ms instead of 20.6.
+  int prLow = 0, prHigh = 0;
   CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prLow, &prHigh));
   for (int c = 0; c < 2 * kRunStreams; ++c) {
+    const int slot = c % kRunStreams;
     CUDA_TRY(cudaStreamCreateWithPriority(&e->cls_stream[c], cudaStreamNonBlocking,
-                                          c % kRunStreams == 1 ? prLow : prHigh));
+                                          slot == kSlotMix || slot == kSlotAlt ? prLow : prHigh));
     CUDA_TRY(cudaEventCreateWithFlags(&e->join_ev[c], cudaEventDisableTiming));
   }
 
