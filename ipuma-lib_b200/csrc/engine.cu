@@ -1285,7 +1285,7 @@ std::string tune_key(const ipuma_engine* e) {
   char buf[512];
   // The rates are those of the engine's kernels, which differ by mode: a
   // full alignment (forward + reverse pass) takes longer per cell.
-  snprintf(buf, sizeof(buf), "%s|sm%d%d|M=%d|sim=%d|gI=%d|gE=%d|fwd=%d|cells=%d|v8", prop.name, prop.major, prop.minor, e->M,
+  snprintf(buf, sizeof(buf), "%s|sm%d%d|M=%d|sim=%d|gI=%d|gE=%d|fwd=%d|cells=%d|v9", prop.name, prop.major, prop.minor, e->M,
            e->sw.similarity, e->sw.gap_init, e->sw.gap_extend, e->sc.forwardOnly, (int)e->cells);
   for (char* c = buf; *c; ++c)
     if (*c == '\t' || *c == '\n') *c = ' ';
@@ -1345,8 +1345,10 @@ void append_cache_file(const char* path, const std::string& key, const std::vect
   fclose(f);
 }
 
-// Device time (ms) of the class-`cls` launch for n synthetic pairs.
-int time_class(ipuma_engine* e, int cls, int n, int alen, int blen, const DevBuf& letters, int nletters,
+// Device time (ms) of the class-`cls` launch for n synthetic pairs; -1 when
+// some of them gave up (their time covers part of their cells only).
+// related: as in k_synth_pairs.
+int time_class(ipuma_engine* e, int cls, int n, int alen, int blen, const DevBuf& letters, int nletters, int related,
                uint32_t seed, float* ms) {
   cudaStream_t s = e->stream;
   int rc;
@@ -1356,7 +1358,7 @@ int time_class(ipuma_engine* e, int cls, int n, int alen, int blen, const DevBuf
   if ((rc = e->d_res.ensure(sizeof(int) * 3 * (size_t)n, s))) return rc;
   const int gb = (int)std::min<size_t>((bytes + 255) / 256, (size_t)e->nsm * 16);
   k_synth_pairs<<<gb, 256, 0, s>>>(e->d_codes.as<uint8_t>(), e->d_pairs.as<PairDesc>(), n, alen, blen,
-                                   letters.as<uint8_t>(), nletters, seed);
+                                   letters.as<uint8_t>(), nletters, related, seed);
   CUDA_TRY(cudaGetLastError());
   const int savedK = e->tile_k, savedT = e->time_launches;
   e->tile_k = cls + 1;
@@ -1374,6 +1376,7 @@ int time_class(ipuma_engine* e, int cls, int n, int alen, int blen, const DevBuf
     if ((rc = check_status(e, s))) break;
     for (int k = 0; k < e->stats.n_timed; ++k)
       if (e->timed_cls[k] == cls) *ms = (float)e->stats.timed_ms[k];
+    if (e->stats.overflow_reruns) *ms = -1.f;
   }
   e->tile_k = savedK;
   e->time_launches = savedT;
@@ -1410,6 +1413,7 @@ int run_autotune(ipuma_engine* e, const char* cache_path) {
   if ((rc = dl.ensure(letters.size(), e->stream))) return rc;
   CUDA_TRY(cudaMemcpy(dl.p, letters.data(), letters.size(), cudaMemcpyHostToDevice));
   v.assign(2 * kNumS16, 0.f);
+  std::copy(e->slot_ps, e->slot_ps + kNumS16, v.begin());  // kept where nothing can be measured
   for (int c = 0; c < kNumS16 && rc == IPUMA_OK; ++c) {
     const int W = kClasses[c].width, L = kClasses[c].lanes;
     // Pairs per warp item; the per-thread class keeps 64 pairs per warp and
@@ -1427,15 +1431,21 @@ int run_autotune(ipuma_engine* e, const char* cache_path) {
     // than L2, as real batches do.
     const int shapes[2][2] = {{1, 1024}, {8, 128}};
     const int thr_shapes[2][2] = {{4, 1024}, {16, 512}};
+    const int limit = kr.ok() ? kr.limit : e->sc.s16Limit;
     double tpp[2] = {0, 0};
     for (int sh = 0; sh < 2 && rc == IPUMA_OK; ++sh) {
       const int* shp = L > 0 ? shapes[sh] : thr_shapes[sh];
       const int alen = shp[0] * W, blen = shp[1];
       const int n = std::max(minPairs, (int)std::min(2.0e6, 1.5e9 / ((double)alen * blen)));
+      // Pairs that could pass the lanes' scores get fewer related residues:
+      // one that gives up half way is timed for half of its cells.
+      const int fits = limit / std::max(1, e->maxSub);
       float ms = -1.f;
-      rc = time_class(e, c, n, alen, blen, dl, (int)letters.size(), 0x5eed0000u + 16 * c + sh, &ms);
+      rc = time_class(e, c, n, alen, blen, dl, (int)letters.size(), std::min(alen, blen) > fits ? fits : -1,
+                      0x5eed0000u + 16 * c + sh, &ms);
       tpp[sh] = ms > 0 ? ms * 1e9 / n : 0;  // ps per pair
     }
+    if (tpp[0] <= 0 || tpp[1] <= 0) continue;
     // tpp = strips * ((rows + L) * W * slot + strip)
     const int* s1 = L > 0 ? shapes[0] : thr_shapes[0];
     const int* s2 = L > 0 ? shapes[1] : thr_shapes[1];

@@ -1295,9 +1295,13 @@ static __global__ void k_bin_scatter(const int* __restrict__ keys, int n, int* o
 
 // Synthetic calibration batch for the autotuner: n pairs of |A| = alen,
 // |B| = blen; A uniform over `letters`, B = A with 1 in 8 residues
-// substituted, then random letters past |A|.
+// substituted, then random letters past |A|.  related >= 0: A is drawn from
+// the first half of the letters and B from the second, but for `related`
+// residues of A's diagonal in equal distances, so that no alignment scores
+// more than they do.
 static __global__ void k_synth_pairs(uint8_t* codes, PairDesc* pairs, int n, int alen, int blen,
-                                     const uint8_t* __restrict__ letters, int nletters, uint32_t seed) {
+                                     const uint8_t* __restrict__ letters, int nletters, int related, uint32_t seed) {
+  const int half = nletters / 2, diag = min(alen, blen);
   const long per = (long)alen + blen;
   for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < (long)n * per;
        k += (long)gridDim.x * blockDim.x) {
@@ -1312,7 +1316,11 @@ static __global__ void k_synth_pairs(uint8_t* codes, PairDesc* pairs, int n, int
     };
     uint8_t v;
     if (i < alen) {
-      v = letters[hash(p * 131071 + i) % nletters];
+      v = letters[hash(p * 131071 + i) % (related < 0 ? nletters : half)];
+    } else if (related >= 0) {
+      const long j = i - alen;
+      const bool kept = j < diag && j * related / diag != (j + 1) * related / diag;
+      v = letters[kept ? hash(p * 131071 + j) % half : half + hash(p * 524287 + j + 7) % (nletters - half)];
     } else {
       const long j = i - alen;
       const uint32_t r = hash(p * 524287 + j + 7);
