@@ -240,7 +240,11 @@ void ipuma_gpu_destroy(ipuma_engine* e);
  *                 IPUMA_KERNEL_S16_L16_K6, _K10, _K14, 11 .. 16 =
  *                 IPUMA_KERNEL_S16_L16_K5, _K7, _K9, _K11, _K13, _K15,
  *                 17 .. 21 = IPUMA_KERNEL_S16_L8_K8, _K10, _K12, _K14, _K16,
- *                 24 = every pair through strip teams (IPUMA_KERNEL_S16_TEAM)
+ *                 24 = every pair through strip teams (IPUMA_KERNEL_S16_TEAM).
+ *                 Where a scoring or batch has no kernel of the value (8 ..
+ *                 21 when four times a score passes 8 bits, 17 .. 21 in 2-bit
+ *                 batches of 150,000 pairs and more with gap_init 0), the
+ *                 narrowest strips at least as wide run
  *   "concurrent"  0 = one launch after the other (always the case with
  *                 time_launches); 1, 2, 3 (default) = the launches of long
  *                 pairs and of the other classes share the GPU on streams

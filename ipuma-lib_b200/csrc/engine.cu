@@ -784,6 +784,7 @@ void run_slots(const KernelRef* kr, unsigned enabled, int* slot) {
 // grids and strip scratch (int2).
 struct ClassPlan {
   int model = 0, teamW = 0;
+  int forced = -1;                 // class every pair goes to (option tile_k), -1: by cost
   unsigned enabled = 0;            // classes launched
   bool highScores = false;         // a pair may pass the long class's scores
   int s16_max_len = 0;             // both sequences longer: the diagonal bound decides
@@ -797,6 +798,18 @@ struct ClassPlan {
 
 // Longest min(|A|,|B|) class c is chosen for by cost (BinParams::fit).
 int class_fit(const ipuma_engine* e, const KernelRef& kr) { return (kr.ok() ? kr.limit : e->sc.s16Limit) / e->typical; }
+
+// Class that runs a forced class's pairs: itself, or where the model has no
+// kernel of it the narrowest at least as wide (kSepLin8 holds all 8-lane
+// widths under the classes of their 16-lane twins, kMixAny those of 64-column
+// steps).
+int forced_class(const KernelRef* kr, int cls) {
+  if (cls >= kNumS16 || cls == kClsThread || kr[cls].ok()) return cls;
+  int best = kClsWidest;
+  for (int c = 0; c < kNumS16; ++c)
+    if (kr[c].ok() && kClasses[c].width >= kClasses[cls].width && kClasses[c].width < kClasses[best].width) best = c;
+  return best;
+}
 
 int plan_classes(ipuma_engine* e, int n, int P, int bits, int maxA, int maxB, ClassPlan& pl) {
   pl.model = mix_model(e, P, n >= kEightLaneMinPairs);
@@ -827,14 +840,12 @@ int plan_classes(ipuma_engine* e, int n, int P, int bits, int maxA, int maxB, Cl
   if (e->tile_k > 0) {  // no pair is given to a class by cost
     for (int c = 0; c < kNumClasses; ++c)
       if (by_cost_class(c)) enabled &= ~(1u << c);
-    enabled |= 1u << (e->tile_k - 1);
+    pl.forced = forced_class(kr, e->tile_k - 1);
+    enabled |= 1u << pl.forced;
   }
   if (((enabled >> kClsTeam) & 1u) && ((enabled >> kClsBig) & 1u)) enabled |= 1u << kClsBigTeam;
   for (int c = 0; c < kNumClasses; ++c)
-    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].ok()) {
-      if (e->tile_k == c + 1) return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d has no kernel for this scoring", e->tile_k);
-      enabled &= ~(1u << c);
-    }
+    if (c != kClsThread && c != kClsTeam && c != kClsBigTeam && !kr[c].ok()) enabled &= ~(1u << c);
   pl.enabled = enabled;
   run_slots(kr, enabled, pl.slot);
   class_grids(e, P, pl.model, kr, enabled, maxA, maxB, pl.grid, pl.spb);
@@ -986,7 +997,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   bp.long_a = e->long_a;
   // tile_k > 0 forces one s16x2 class: every pair uses the chosen kernel,
   // long A crossing several strips.
-  bp.forced_class = e->tile_k > 0 ? e->tile_k - 1 : -1;
+  bp.forced_class = pl.forced;
   bp.max_a = maxA;
   bp.max_b = maxB;
   bp.n_codes = (long long)n_codes;
