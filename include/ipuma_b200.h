@@ -347,9 +347,10 @@ int ipuma_gpu_compare_device_packed(ipuma_engine* e, const uint8_t* d_packed, si
                                     int32_t* d_brange, void* stream);
 
 /* Grows every device buffer that ipuma_gpu_compare_device needs for up to
- * n pairs with |A| <= max_a_len and |B| <= max_b_len, so that such calls
- * allocate (and synchronise the device) no more -- for serving loops and
- * before a stream capture.  No counterpart in the reference. */
+ * n pairs with |A| <= max_a_len and |B| <= max_b_len under the engine's
+ * present options, so that such calls allocate (and synchronise the device)
+ * no more -- for serving loops and before a stream capture.  No counterpart
+ * in the reference. */
 int ipuma_gpu_reserve(ipuma_engine* e, int32_t n, int32_t max_a_len, int32_t max_b_len);
 
 /* Wire-buffer batch with inputs and results already in device memory,

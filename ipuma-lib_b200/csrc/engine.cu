@@ -898,6 +898,20 @@ int reserve_batched(ipuma_engine* e, cudaStream_t s, int n, int maxA, int maxB) 
   return reserve_bufs(e, main_bufs(e), s, n, maxA, maxB);
 }
 
+// Strip scratch (int2) for every batch of at most these sizes.  A smaller
+// one may need more in two ways: a team has a warp per 512-column strip of
+// the longest A, and blocks of fewer warps may fill an SM better; and the
+// pair count picks the kernels.  Everything else only shrinks with the batch.
+size_t scratch_int2_up_to(ipuma_engine* e, int n, int maxA, int maxB) {
+  size_t most = 0;
+  for (int m : {n, std::min(n, kEightLaneMinPairs - 1), std::min(n, kLatClassMaxPairs - 1)})
+    for (int strips = 0; strips <= kTeamMaxWarps; ++strips) {
+      const int a = strips == 0 ? maxA : strips * kClasses[kClsTeam].width;
+      if (a <= maxA) most = std::max(most, scratch_int2(e, m, a, maxB));
+    }
+  return most;
+}
+
 // Runs the persistent cost-binned pipeline over n device-resident pairs.
 // Results land at score[p], arange[p], brange[p].
 // n_codes = residues the code array holds: pairs reaching past it are
@@ -2049,6 +2063,8 @@ int ipuma_gpu_reserve(ipuma_engine* e, int32_t n, int32_t max_a_len, int32_t max
   std::lock_guard<std::mutex> lk(e->mu);
   CUDA_TRY(cudaSetDevice(e->device));
   int rc;
+  const size_t scratch = scratch_int2_up_to(e, n, max_a_len, max_b_len);
+  if ((rc = e->d_scratch.ensure(sizeof(int2) * scratch, e->stream))) return rc;
   if ((rc = reserve_batched(e, e->stream, n, max_a_len, max_b_len))) return rc;
   CUDA_TRY(cudaStreamSynchronize(e->stream));
   return IPUMA_OK;
