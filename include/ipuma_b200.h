@@ -248,9 +248,10 @@ void ipuma_gpu_destroy(ipuma_engine* e);
  *   "concurrent"  0 = one launch after the other (always the case with
  *                 time_launches); 1, 2, 3 (default) = the launches of long
  *                 pairs and of the other classes share the GPU on streams
- *   "latency_share" weight of a pair's own latency beside the modelled
- *                 time of a batch of such pairs when its class is chosen
- *                 (per mille, default 1500)
+ *   "latency_share" share of the batch's modelled time (per mille,
+ *                 default 60) one pair's latency may take: the smaller,
+ *                 the more a pair's own latency counts beside the batch's
+ *                 time when its class is chosen
  *   "hybrid"      1 = pairs whose score can pass int16 run their strips
  *                 in biased 16-bit halves while a strip's values provably
  *                 fit, then in s32 (IPUMA_KERNEL_S16_HYBRID, default);

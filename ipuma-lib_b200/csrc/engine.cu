@@ -152,7 +152,11 @@ constexpr float kThrLatencyShare = 0.5f;
 // Weight of a pair's own latency beside the modelled time of a batch of such
 // pairs (pair_key): in a small batch it sends pairs to the class that
 // finishes them soonest, in a large one it counts for the longest only.
-constexpr float kLatencyWeight = 1.5f;
+// Option "latency_share" states it as the per mille of the batch's time that
+// one pair's latency may take: weight 1.5 at the default of 60, and the more
+// the smaller the share.
+constexpr int kLatencyShareDefault = 60;
+constexpr float kLatencyWeight = 1.5f * (float)kLatencyShareDefault;  // / latency_share
 constexpr float kPackingEfficiency = 0.85f;
 // Classes at 64-column steps; the ones between are added below.
 constexpr unsigned kCoarseClasses = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 5);
@@ -281,7 +285,7 @@ struct ipuma_engine {
   cudaEvent_t join_ev[2 * kRunStreams] = {};
   int concurrent = 3;
   int hybrid = 1;  // option "hybrid": high-scoring pairs run s16x2 strips while provably safe
-  float latency_weight = kLatencyWeight;  // option "latency_share" (per mille)
+  int latency_share = kLatencyShareDefault;  // option "latency_share" (per mille)
   cudaStream_t stream2 = nullptr, copy_stream = nullptr;
   cudaEvent_t cev[2 * kMaxChunks + 2] = {};
   int chunks = 0;  // option "chunks": 0 automatic, 1 off, n fixed
@@ -1003,7 +1007,7 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   for (int c : {kClsTeam, kClsBigTeam})
     bp.step_ps[c] = e->slot_ps[c] * 64.f * (float)kClasses[c].k * (float)(bp.grid[c] * bp.team_warps);
   bp.batch_ps_per_cell = slot_min / kPackingEfficiency;
-  bp.lat_weight = e->latency_weight;
+  bp.lat_weight = kLatencyWeight / (float)e->latency_share;
   // Pairs the widest strips' resident warps hold, two each.
   const int resident = 2 * kWarpsPerBlock * bp.grid[kClsWidest];
   bp.team_slack = n < resident ? 0.f : kTeamSlackPs;
@@ -2000,7 +2004,7 @@ int ipuma_gpu_set_option(ipuma_engine* e, const char* name, int64_t value) {
     e->time_launches = value ? 1 : 0;
   } else if (k == "latency_share") {
     if (value < 1 || value > 100000) return fail(IPUMA_ERR_INVALID_ARG, "latency_share is in per mille, 1..100000");
-    e->latency_weight = (float)value / 1000.f;
+    e->latency_share = (int)value;
   } else if (k == "hybrid") {
     e->hybrid = value ? 1 : 0;
   } else if (k == "concurrent") {
@@ -2122,7 +2126,7 @@ static int compare_dev(ipuma_engine* e, const uint8_t* d_codes, size_t n_codes, 
                                        (uint64_t)(uintptr_t)e->d_ovf.p, (uint64_t)(uintptr_t)e->d_flag.p,
                                        (uint64_t)e->tile_k, (uint64_t)e->long_a, (uint64_t)e->thread_class,
                                        (uint64_t)e->concurrent, (uint64_t)e->hybrid, (uint64_t)e->trace,
-                                       (uint64_t)(e->latency_weight * 1e6f), (uint64_t)e->team_warps};
+                                       (uint64_t)e->latency_share, (uint64_t)e->team_warps};
     auto it = e->graphs_cache.find(key);
     if (it == e->graphs_cache.end()) {
       if (e->graphs_cache.size() >= 16) {
