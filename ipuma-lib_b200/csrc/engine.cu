@@ -134,7 +134,7 @@ constexpr int kClsHi = kNumS16 + 1;
 constexpr int kClsTeam = kNumS16 + 2;
 constexpr int kTeamWarpsDefault = 8;
 // Long class: the widest strips with one tag bit, for pairs whose score may
-// pass what class kClsWidest holds (BinParams::fit).
+// pass what the classes by cost hold (BinParams::fit_len).
 constexpr int kClsLong = kNumS16 + 3;
 // Big class: pairs whose main diagonal passes the long class's scores, in
 // biased halves (LaneBig, scores up to 64,000); and its strip teams.  Pairs
@@ -242,7 +242,9 @@ struct ipuma_engine {
   bool s16_ok = false;   // s16x2 lanes valid for this scoring
   // Which lanes the 16-bit classes run (kernel_of), fixed by the scoring.
   enum Cells { kLinear, kAffine, kAnyScore } cells = kAnyScore;
-  int typical = 1;       // score of a typical identical residue (BinParams::fit)
+  int8_t top[32] = {};   // largest score of each letter, at least 0 (BinParams::top)
+  bool same_top = true;  // every letter's is the same (or 0)
+  int typical = 1;       // mean score of an identical residue, rounded up
 
   // options
   int scheduler = 0;
@@ -792,6 +794,9 @@ struct ClassPlan {
   unsigned enabled = 0;            // classes launched
   bool highScores = false;         // a pair may pass the long class's scores
   int s16_max_len = 0;             // both sequences longer: the diagonal bound decides
+  int fit_len = 0;                 // neither longer: the classes by cost hold every score
+  int over = 0;                    // class of the pairs they may not hold
+  bool by_letters = false;         // one may be: its letters decide (letters_pass)
   KernelRef kr[kNumClasses];
   int slot[NCLASS_MAX + 1] = {};
   int grid[NCLASS_MAX + 1] = {};
@@ -799,9 +804,6 @@ struct ClassPlan {
   long long base[kRunStreams] = {};  // scratch region of each stream
   long long total = 0;
 };
-
-// Longest min(|A|,|B|) class c is chosen for by cost (BinParams::fit).
-int class_fit(const ipuma_engine* e, const KernelRef& kr) { return (kr.ok() ? kr.limit : e->sc.s16Limit) / e->typical; }
 
 // Class that runs a forced class's pairs: itself, or where the model has no
 // kernel of it the narrowest at least as wide (kSepLin8 holds all 8-lane
@@ -826,8 +828,12 @@ int plan_classes(ipuma_engine* e, int n, int P, int bits, int maxA, int maxB, Cl
   pl.highScores = std::min(maxA, maxB) > pl.s16_max_len;
   if (!e->s16_ok || (pl.highScores && !e->hybrid)) enabled |= 1u << kClsS32;
   if (pl.highScores && e->hybrid) enabled |= (1u << kClsHi) | (1u << kClsBig);
-  // The long class, when the batch may hold a pair past the widest's scores.
-  if (std::min(maxA, maxB) > class_fit(e, kr[kClsWidest])) enabled |= 1u << kClsLong;
+  // The classes by cost hold the same scores (MixLane).  Pairs that may pass
+  // them: by their length alone where every letter scores maxSub at best,
+  // else by their letters.
+  const int shorter = std::min(maxA, maxB), limit = kr[kClsWidest].limit;
+  pl.fit_len = e->maxSub > 0 ? limit / e->maxSub : (1 << 30);
+  pl.by_letters = !e->same_top && shorter > pl.fit_len;
   if (e->thread_class && bits == 8) enabled |= 1u << kClsThread;  // k_thread reads bytes only
   if (P < e->M && pl.model == kMixAff) {
     // Four-row profiles: the narrow widths in 8-lane groups.
@@ -841,6 +847,12 @@ int plan_classes(ipuma_engine* e, int n, int P, int bits, int maxA, int maxB, Cl
     return fail(IPUMA_ERR_INVALID_ARG, "tile_k %d (strip teams) needs team_warps >= 2 and room for two warps",
                 kClsTeam + 1);
   if (pl.teamW >= 2 && maxA > kClasses[kClsTeam].width && e->tile_k == 0) enabled |= 1u << kClsTeam;
+  // They go to the long class -- in a batch that leaves warps idle to the
+  // teams, as long as only letters far above the mean can take a pair there:
+  // the long class's launch on a stream of its own cost 64 proteins 25 us.
+  const bool idle = n < 2 * kWarpsPerBlock * kernel_grid(e, kr[kClsWidest], P, pl.model);
+  pl.over = pl.by_letters && idle && ((enabled >> kClsTeam) & 1u) && shorter <= limit / e->typical ? kClsTeam : kClsLong;
+  if (shorter > pl.fit_len && pl.over == kClsLong) enabled |= 1u << kClsLong;
   if (e->tile_k > 0) {  // no pair is given to a class by cost
     for (int c = 0; c < kNumClasses; ++c)
       if (by_cost_class(c)) enabled &= ~(1u << c);
@@ -970,13 +982,17 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     bp.inv_width[c] = (unsigned)(((1ull << 32) + kClasses[c].width - 1) / kClasses[c].width);
     bp.slot_ps[c] = e->slot_ps[c];
     bp.strip_ps[c] = e->strip_ps[c];
-    bp.fit[c] = class_fit(e, kr[c]);
     bp.grid[c] = pl.grid[c];
     bp.scr_per_block[c] = pl.spb[c];
   }
   bp.widest = kClsWidest;
-  bp.cls_long = kClsLong;
+  bp.cls_over = pl.over;
   bp.s16_max_len = pl.s16_max_len;
+  bp.fit_len = pl.fit_len;
+  bp.fit_score = kr[kClsWidest].limit;
+  bp.by_letters = pl.by_letters ? 1 : 0;
+  std::copy(e->top, e->top + 32, bp.top);
+  bp.thr_fit = e->sc.s16Limit / e->typical;
   const long thrThreads = thread_threads<16>(e);
   bp.thr_cls = kClsThread;
   bp.thr_on = e->thread_class && bits == 8;
@@ -1036,13 +1052,13 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
     *launches += 1;
   }
   if (n <= kSmallBin) {
-    k_bin_small<<<1, 1024, 0, s>>>(bp, pairs, n, flags, total, sums, ctl + CTL_RANGES, allot, st, rb.list->as<int>(),
+    k_bin_small<<<1, 1024, 0, s>>>(bp, codes, pairs, n, flags, total, sums, ctl + CTL_RANGES, allot, st, rb.list->as<int>(),
                                    score, arange, brange);
     *launches += 1;
   } else {
     k_bin_total<<<gb, tb, 0, s>>>(bp, pairs, n, total, ctl + CTL_HIST, nkeys);
     int* keys = rb.ovf->as<int>();  // free until the alignment launches
-    k_bin_count<<<gb, tb, 0, s>>>(bp, pairs, n, ctl + CTL_HIST, flags, keys, sums, st, score, arange, brange);
+    k_bin_count<<<gb, tb, 0, s>>>(bp, codes, pairs, n, ctl + CTL_HIST, flags, keys, sums, st, score, arange, brange);
     k_bin_scan<<<bp.nclass, 1024, 0, s>>>(bp, ctl + CTL_HIST, ctl + CTL_OFFS, sums, ctl + CTL_RANGES, allot, st);
     k_bin_scatter<<<gb, tb, 0, s>>>(keys, n, ctl + CTL_OFFS, rb.list->as<int>());
     *launches += 4;
@@ -1929,6 +1945,10 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   e->cells = gI == 0 && scaled(-gE, kProfShift<LaneLin>) ? ipuma_engine::kLinear
              : scaled(0, kProfShift<LaneAff>)            ? ipuma_engine::kAffine
                                                          : ipuma_engine::kAnyScore;
+  for (int x = 0; x < m; ++x) {
+    for (int y = 0; y < m; ++y) e->top[x] = std::max({e->top[x], e->sim[x * m + y], e->sim[y * m + x]});
+    e->same_top &= e->top[x] == 0 || e->top[x] == e->maxSub;
+  }
   int diag = 0, letters = 0;
   for (int x = 0; x < m; ++x)
     if (e->sim[x * m + x] > 0) {

@@ -806,10 +806,12 @@ struct BinParams {
   int big_limit;           // scores above this need more than 16 biased bits
   int s16_max_len;         // min(|A|,|B|) above which the 16-bit lanes could overflow
   int s16_limit;           // scores above this need more than the long class's 16 bits
-  // Longest min(|A|,|B|) a class is chosen for by cost: a typical identical
-  // pair of that length still fits the scores its lanes hold (a pair that
-  // does not is rerun in s32 lanes).
-  int fit[NCLASS_MAX];
+  // Scores the lanes of the classes by cost hold (a pair past them is rerun in
+  // s32 lanes), and the longest min(|A|,|B|) that cannot pass them.  A longer
+  // pair goes to cls_over: where by_letters is 0 by its length alone, else if
+  // its letters' top scores say so (letters_pass).
+  int fit_score, fit_len, by_letters, cls_over;
+  int8_t top[32];
   int lanes[NCLASS_MAX];   // lanes per group of each class
   int width[NCLASS_MAX];   // strip width (lanes * K) of each class
   unsigned inv_width[NCLASS_MAX];  // ceil(2^32 / width): strips_of
@@ -824,7 +826,6 @@ struct BinParams {
   float team_slack;            // kTeamSlackPs, or 0 for a batch that leaves warps idle
   int long_a;                  // |A| above which the widest strips are used
   int widest;                  // class of the widest strips
-  int cls_long;                // the same strips with room for the longest scores (past fit[widest])
   int forced_class;        // >= 0: every s16x2 pair goes to this class
   int team_cls;            // strip-team class (-1: none in this batch)
   int team_warps;          // warps per team
@@ -850,7 +851,7 @@ struct BinParams {
   int thr_cls;             // class index
   int thr_on;              // 0: the class is never chosen (unless forced)
   int thr_k;               // columns per strip
-  int thr_max_rows;
+  int thr_max_rows, thr_fit;   // rows it accepts, and the longest min(|A|,|B|)
   float thr_cap_scale;
   const unsigned long long* total_cells;  // written by k_bin_total
 };
@@ -961,7 +962,8 @@ __device__ __forceinline__ int team_class(const BinParams& bp, int cls, int tc, 
   return tl < lat ? tc : cls;
 }
 
-// `flag`: 0, 1 (the diagonal bound passes s16_limit) or 2 (big_limit).
+// `flag`: 0, 1 (the diagonal bound passes s16_limit), 2 (big_limit) or 3
+// (letters_pass).
 __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen, int flag, float thr_cap) {
   int cls;
   if (bp.force_s32) {
@@ -979,8 +981,9 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
   } else {
     const float batch_ps = bp.total_cells ? (float)(*bp.total_cells) * bp.batch_ps_per_cell : 0.f;
     float bestLat = -1.f;  // one-warp latency of the class picked below
-    const int fit = min(alen, blen);
-    const int wide = fit <= bp.fit[bp.widest] ? bp.widest : bp.cls_long;
+    const int shorter = min(alen, blen);
+    const bool over = shorter > bp.fit_len && (flag == 3 || !bp.by_letters);
+    const int wide = over ? bp.cls_over : bp.widest;
     if (alen > bp.long_a) {
       // Very long pairs are few and each keeps one warp busy for long: their
       // latency, not throughput, sets the end of the launch, and the widest
@@ -991,14 +994,15 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
     } else {
       cls = wide;
       float bestCost = -1.f;
-      const bool thr_ok = bp.thr_on && blen <= bp.thr_max_rows && (float)alen * (float)blen <= thr_cap;
+      const bool thr_ok = bp.thr_on && blen <= bp.thr_max_rows && shorter <= bp.thr_fit &&
+                          (float)alen * (float)blen <= thr_cap;
       // The time of a batch made of this pair alone, as many as hold the
       // batch's cells: its share of the GPU's rate, and once a part of its
       // own latency (the last ones finish alone).
       const float like = bp.total_cells ? (float)(*bp.total_cells) / ((float)alen * (float)blen) : 1.f;
       for (unsigned left = bp.by_cost; left; left &= left - 1) {
         const int c = __ffs(left) - 1;
-        if ((c == bp.thr_cls && !thr_ok) || fit > bp.fit[c]) continue;
+        if (c == bp.thr_cls ? !thr_ok : over) continue;
         const int strips = strips_of(bp, c, alen);
         const float lat = (float)strips * (float)(blen + bp.lanes[c]) * bp.step_ps[c];
         const float cost =
@@ -1010,7 +1014,7 @@ __device__ __forceinline__ int pair_key(const BinParams& bp, int alen, int blen,
           cls = c;
         }
       }
-      if (bestCost < 0.f)  // no class holds its scores but the long one
+      if (bestCost < 0.f)  // none of them holds its scores
         bestLat = (float)strips_of(bp, cls, alen) * (float)(blen + bp.lanes[cls]) * bp.step_ps[cls];
     }
     cls = team_class(bp, cls, bp.team_cls, alen, blen, bestLat, batch_ps);
@@ -1081,6 +1085,66 @@ static __global__ void k_bin_bound(BinParams bp, const uint8_t* __restrict__ cod
   }
 }
 
+// May this lane's pair, longer than fit_len (`cand`), pass fit_score?  An
+// alignment scores no more than the top scores of its shorter sequence's
+// letters add up to.  32 of them, at equal distances, give the sum to about a
+// sixteenth; from three of those below the limit to a fourth above it 128 do,
+// to a thirtieth, against a line a sixteenth below the limit.  The lanes of a
+// warp read one candidate's letters, the first samples of up to four at a
+// time.  s_top: bp.top in shared memory.
+// (B200, 10,000 near-identical proteins of 700-1,300 residues, 80 % of them C,
+// H or W: with the mean letter for all 6,328 were rerun in s32, 7.1 ms; now
+// 3.7.  Adding up all letters took 9 us of a request of 500; 32 alone, with
+// a line an eighth below, sent pairs of 1,200 average residues to the long
+// class, 8 % slower with start coordinates.)
+__device__ __forceinline__ bool letters_pass(const BinParams& bp, const int8_t* s_top, const uint8_t* codes,
+                                             const PairDesc& d, bool cand) {
+  const int lane = threadIdx.x & 31;
+  const int own_len = min(d.a_len, d.b_len);
+  const long long own_off = d.a_len <= d.b_len ? d.a_off : d.b_off;
+  const auto top = [&](int x) { return x < 32 ? (int)s_top[x] : 0; };  // past the alphabet: scores nothing
+  bool pass = false;
+  unsigned m = __ballot_sync(FULL, cand);
+  while (m) {
+    int src[4], len[4], x[4];
+    long long off[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      src[u] = m ? __ffs(m) - 1 : -1;
+      m &= m - 1;
+      len[u] = __shfl_sync(FULL, own_len, max(src[u], 0));
+      off[u] = __shfl_sync(FULL, own_off, max(src[u], 0));
+      x[u] = src[u] >= 0 ? code_at(codes, off[u] + lane * len[u] / 32, bp.bits) : 32;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (src[u] < 0) break;
+      const long long sampled = (long long)__reduce_add_sync(FULL, top(x[u])) * len[u];  // 32 times the sum
+      bool over = sampled > 40ll * bp.fit_score;
+      if (!over && sampled > 26ll * bp.fit_score) {
+        int y[4], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y[q] = code_at(codes, off[u] + (4 * lane + q) * len[u] / 128, bp.bits);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sum += top(y[q]);
+        over = (long long)__reduce_add_sync(FULL, sum) * len[u] > 120ll * bp.fit_score;
+      }
+      if (lane == src[u]) pass = over;
+    }
+  }
+  return pass;
+}
+
+// Flag of a pair (pair_key); s32_flag as k_bin_bound left it.  All lanes of
+// the warp call it.
+__device__ __forceinline__ int pair_flag(const BinParams& bp, const int8_t* s_top, const uint8_t* codes, const PairDesc& d,
+                                         bool listed, long p, const uint8_t* s32_flag) {
+  const int flag = listed && bound_candidate(bp, d) ? s32_flag[p] : 0;
+  if (!bp.by_letters) return flag;
+  const bool cand = listed && flag == 0 && min(d.a_len, d.b_len) > bp.fit_len;
+  return letters_pass(bp, s_top, codes, d, cand) ? 3 : flag;
+}
+
 // Sums of the pairs of one class.
 struct ClassSums {
   unsigned long long cells;
@@ -1115,23 +1179,26 @@ __device__ __forceinline__ void reject_pair(int state, long p, DevStatus* st, in
   brange[p] = 0;
 }
 
-static __global__ void k_bin_count(BinParams bp, const PairDesc* __restrict__ pairs, int n, int* hist,
-                                   const uint8_t* s32_flag, int* keys, ClassSums* sums, DevStatus* st, int* score, int* arange,
-                                   int* brange) {
+static __global__ void k_bin_count(BinParams bp, const uint8_t* __restrict__ codes,
+                                   const PairDesc* __restrict__ pairs, int n, int* hist, const uint8_t* s32_flag,
+                                   int* keys, ClassSums* sums, DevStatus* st, int* score, int* arange, int* brange) {
   __shared__ ClassSums s_sum[NCLASS_MAX];
+  __shared__ int8_t s_top[32];
   for (int k = threadIdx.x; k < NCLASS_MAX; k += blockDim.x) s_sum[k] = ClassSums{0, 0, 0};
+  if (threadIdx.x < 32) s_top[threadIdx.x] = bp.top[threadIdx.x];
   __syncthreads();
-  for (long p = (long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long)gridDim.x * blockDim.x) {
-    const PairDesc d = pairs[p];
+  const int lane = threadIdx.x & 31;
+  for (long base = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < n; base += (long)gridDim.x * blockDim.x) {
+    const long p = base + lane;
+    const PairDesc d = p < n ? pairs[p] : PairDesc{0, 0, 0, 0};
     const int state = pair_state(d, bp.n_codes, bp.max_a, bp.max_b);
+    const int flag = pair_flag(bp, s_top, codes, d, p < n && state == PAIR_OK, p, s32_flag);
+    if (p >= n) continue;
     if (state != PAIR_OK) {
       reject_pair(state, p, st, score, arange, brange);
       keys[p] = -1;
       continue;
     }
-    // Candidates (both sequences longer than s16_max_len) got their flag
-    // from k_bin_bound.
-    const int flag = bound_candidate(bp, d) ? s32_flag[p] : 0;
     const unsigned act = __activemask();
     const int key = tally_pair(bp, d, flag, s_sum, act);
     keys[p] = key;
@@ -1220,7 +1287,8 @@ static __global__ void k_bin_scan(BinParams bp, const int* hist, int* offs, cons
 // (bitonic).  Four launches and their 110,000-key histogram took 85 us for
 // 64 pairs, this 9.  s32_flag as in k_bin_count.
 constexpr int kSmallBin = 4096;
-static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const PairDesc* __restrict__ pairs, int n,
+static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const uint8_t* __restrict__ codes,
+                                                           const PairDesc* __restrict__ pairs, int n,
                                                            const uint8_t* s32_flag, unsigned long long* total,
                                                            ClassSums* sums, int* class_range, ClassAllot* allot,
                                                            DevStatus* st, int* list, int* score, int* arange,
@@ -1228,7 +1296,9 @@ static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const P
   __shared__ unsigned long long s_key[kSmallBin];  // key << 32 | pair; rejected pairs and padding last
   __shared__ ClassSums s_sum[NCLASS_MAX];
   const int tid = threadIdx.x;
+  __shared__ int8_t s_top[32];
   if (tid < NCLASS_MAX) s_sum[tid] = ClassSums{0, 0, 0};
+  if (tid < 32) s_top[tid] = bp.top[tid];
   __syncthreads();
   unsigned long long local = 0;
   for (int p = tid; p < n; p += 1024) {
@@ -1244,13 +1314,14 @@ static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const P
   while (m < n) m <<= 1;
   for (int p = tid; p < m; p += 1024) {
     unsigned long long e = ~0ull;
+    // m is a multiple of 32: whole warps take part.
+    const PairDesc d = p < n ? pairs[p] : PairDesc{0, 0, 0, 0};
+    const int state = pair_state(d, bp.n_codes, bp.max_a, bp.max_b);
+    const int flag = pair_flag(bp, s_top, codes, d, p < n && state == PAIR_OK, p, s32_flag);
     if (p < n) {
-      const PairDesc d = pairs[p];
-      const int state = pair_state(d, bp.n_codes, bp.max_a, bp.max_b);
       if (state != PAIR_OK) {
         reject_pair(state, p, st, score, arange, brange);
       } else {
-        const int flag = bound_candidate(bp, d) ? s32_flag[p] : 0;
         const int key = tally_pair(bp, d, flag, s_sum, __activemask());
         e = ((unsigned long long)key << 32) | (unsigned)p;
       }
