@@ -1153,7 +1153,6 @@ int reset_ctl(ipuma_engine* e, cudaStream_t s) {
 // pageable copies cost a small call 30 us).
 int check_status(ipuma_engine* e, cudaStream_t s, int nblk = 1) {
   nblk = std::max(1, std::min(nblk, kMaxChunks));
-  if (!e->h_ctl) CUDA_TRY(cudaHostAlloc(&e->h_ctl, sizeof(int) * CTL_CLEAR * kMaxChunks, cudaHostAllocPortable));
   for (int k = 0; k < nblk; ++k)
     CUDA_TRY(cudaMemcpyAsync(e->h_ctl + (size_t)k * CTL_CLEAR, e->d_ctl.as<int>() + (size_t)k * CTL_INTS,
                              sizeof(int) * CTL_CLEAR, cudaMemcpyDeviceToHost, s));
@@ -1882,6 +1881,8 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   e->smem_optin = (int)prop.sharedMemPerBlockOptin;
   CUDA_TRY(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   for (auto& ev : e->ev) CUDA_TRY(cudaEventCreate(&ev));
+  // (Pinning memory takes longer than a small call: not in an engine's first.)
+  CUDA_TRY(cudaHostAlloc(&e->h_ctl, sizeof(int) * CTL_CLEAR * kMaxChunks, cudaHostAllocPortable));
   // Class streams and their fork/join events (created here: no stream or
   // event is created while a stream is being captured).
   CUDA_TRY(cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming));
