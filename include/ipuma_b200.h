@@ -274,8 +274,9 @@ void ipuma_gpu_destroy(ipuma_engine* e);
  *                 couple round robin (forward pass, then the reverse pass
  *                 for start coordinates), so a long pair finishes up to that
  *                 many times sooner; the cost model sends a pair there when
- *                 its one-warp latency exceeds half of the batch's modelled
- *                 time and a team finishes it sooner
+ *                 its one-warp latency exceeds the batch's modelled time (by
+ *                 0.25 ms in a batch that fills the GPU) and a team finishes
+ *                 it sooner
  *   "chunks"      ipuma_gpu_compare(_packed) only: 0 = split large batches into up
  *                 to 8 chunks whose uploads overlap the alignment of the
  *                 previous chunks (default), 1 = upload everything first,

@@ -164,20 +164,27 @@ constexpr unsigned kCoarseClasses = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3
 // twice the columns per lane over a wavefront half as deep, so the per-step
 // work of a lane covers twice the cells.  Their profiles take twice the
 // shared memory per warp, so they replace the 16-lane classes of the same
-// widths only with the four-row profile of 2-bit codes (measured on B200:
-// 1M DNA 3383 -> 3546 GCUPS; 200k protein with 25-row profiles 2960 -> 2855,
-// from half the resident warps).
+// widths only with the four-row profile of 2-bit codes and affine gaps
+// (linear gaps: kSepLin8).  B200, |A| 50-250, 16 -> 8 lanes, 600,000 pairs
+// 8.04 -> 7.77 ms, with start coordinates 13.46 -> 13.15; 150,000 pairs with
+// start coordinates lose, 3.43 -> 3.75.  (200,000 proteins with 25-row
+// profiles lost 4 %, from half the resident warps.)
 // {16-lane class, 8-lane class of the same width}: 64, 80, 96, 112, 128 columns.
 constexpr int kNarrowPairs[5][2] = {{0, 16}, {10, 17}, {7, 18}, {11, 19}, {1, 20}};
 constexpr unsigned kFineClasses = (1u << 7) | (1u << 8) | (1u << 9) | (1u << 10) | (1u << 11) | (1u << 12) |
                                   (1u << 13) | (1u << 14) | (1u << 15);
 constexpr int kWarpsPerBlock = 4;
-// 8-lane groups of linear-gap strips (kMixLin8) from this many pairs: an
+// 8-lane groups of linear-gap strips (kSepLin8) from this many pairs: an
 // item holds eight pairs instead of four, which leaves warps without work
 // in smaller batches (10,000 pairs of 150 x 150-300 on B200: 329 us with 8
 // lanes, 250 with 16; 69,000 of 100-200 x 100-200: 1.07 against 0.91 ms).
 constexpr int kEightLaneMinPairs = 150000;
-// Batches below this size may use the latency classes.
+// Batches below this size may use the latency classes.  They shorten the tail
+// of affine nucleic acids (B200, 4-bit reads of |A| 50-250 without -> with:
+// 3,000 pairs 356 -> 297 us, 12,000 372 -> 357, 19,000 451 -> 440; with start
+// coordinates 478 -> 408, 557 -> 538, 773 -> 748; 30,000 590 -> 578 and 1,016 ->
+// 969) and change nothing from 60,000 pairs on, nor for proteins or linear
+// gaps of any size.  The line keeps most of that.
 constexpr int kLatClassMaxPairs = 20000;
 // One step (row) of a warp item of k columns a lane: `full` ps when the GPU
 // is full, less when the batch's items leave schedulers with one warp --
@@ -996,13 +1003,11 @@ int run_batched(ipuma_engine* e, const RunBufs& rb, cudaStream_t s, const uint8_
   const long thrThreads = thread_threads<16>(e);
   bp.thr_cls = kClsThread;
   bp.thr_on = e->thread_class && bits == 8;
-  bp.thr_k = kClasses[kClsThread].width;
   bp.thr_max_rows = kThrMaxRows;
   bp.thr_cap_scale = kThrLatencyShare / (2.0f * (float)thrThreads);
   bp.total_cells = reinterpret_cast<const unsigned long long*>(ctl + CTL_CELLS) + CELLS_TOTAL;
   // Concurrent launches, except when every launch is timed alone.
   const bool conc = !e->time_launches && e->concurrent != 0;
-  bp.enabled = enabled;
   for (int c = 0; c < kNumClasses; ++c)
     if (((enabled >> c) & 1u) && by_cost_class(c)) bp.by_cost |= 1u << c;
   bp.team_cls = ((enabled >> kClsTeam) & 1u) ? kClsTeam : -1;
@@ -1277,13 +1282,15 @@ int validate_algo(const ipuma_algo_config* a) {
 // size, occupancy), so they are measured: a synthetic batch of related pairs
 // per class at one strip of 1024 rows and at eight strips of 128 rows, every
 // pair forced through that class, gives two equations for the two unknowns.
+// (The batches hold byte codes: the 8-lane kernels of kSepLin8 go by the rates
+// of the 16-lane ones of the same widths.)
 // Results are kept per process (by GPU, alphabet and gaps) and optionally in
 // a cache file of "key<TAB>slot_ps...<TAB>strip_ps..." lines.
 // ---------------------------------------------------------------------------
 
 // The s32 class is not tuned (it is chosen by the overflow rules, not by
-// cost); for the GPU shares of concurrent launches it is modelled as the
-// widest s16x2 class with one pair per lane group instead of two.
+// cost); its pairs' latency is modelled as the widest s16x2 class's with one
+// pair per lane group instead of two.
 void set_s32_rates(ipuma_engine* e) {
   e->slot_ps[kClsS32] = 2.f * e->slot_ps[kClsWidest];
   e->strip_ps[kClsS32] = 2.f * e->strip_ps[kClsWidest];
@@ -1894,6 +1901,7 @@ int ipuma_gpu_create(const ipuma_sw_config* sw, const ipuma_algo_config* algo, i
   CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prLow, &prHigh));
   for (int c = 0; c < 2 * kRunStreams; ++c) {
     const int slot = c % kRunStreams;
+    if (slot == kSlotRun) continue;  // the run's own stream
     CUDA_TRY(cudaStreamCreateWithPriority(&e->cls_stream[c], cudaStreamNonBlocking,
                                           slot == kSlotMix || slot == kSlotAlt ? prLow : prHigh));
     CUDA_TRY(cudaEventCreateWithFlags(&e->join_ev[c], cudaEventDisableTiming));

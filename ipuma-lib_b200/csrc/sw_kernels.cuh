@@ -23,9 +23,10 @@
 //                     (long pairs whose latency would end the launch).
 //   k_bin_*           the cost-binning pre-pass that orders the work list:
 //                     k_bin_total (batch cells), k_bin_bound (main-diagonal
-//                     bounds of the long pairs, a warp per pair), k_bin_count
+//                     bounds of the long pairs, one at a time per warp),
+//                     k_bin_count
 //                     (class and bucket of every pair), k_bin_scan (list
-//                     offsets and class shares), k_bin_scatter (the list);
+//                     offsets and class ranges), k_bin_scatter (the list);
 //                     k_bin_small does all of it for a few thousand pairs.
 #pragma once
 #include "sw_device.cuh"
@@ -163,7 +164,7 @@ __device__ __forceinline__ void align_pairs(const SwConst& sc, uint8_t* s_prof,
     return;
   }
   if constexpr (MODE != 1) {
-  // With start coordinates both passes run through one copy of sw_pass: two
+  // With start coordinates both passes run through one copy of the pass: two
   // inlined copies alternating in the instruction cache slowed both down.
   // (A forward-only launch runs only the copy above.)  The reverse pass
   // stops early once every pair reached its forward score (PassStop).
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(256, T::LINEAR ? 2 : 1)
     // Pass 0: forward.  Pass 1 (with start coordinates): the same pass over
     // the reversed reads from each pair's end cell (as align_pairs, without
     // the early stop), whose first strict maximum gives the start.  One
-    // copy of sw_pass serves both.
+    // copy of tag_pass serves both.
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
       Best out[NP];
@@ -840,7 +841,6 @@ struct BinParams {
   // stay below thr_cap_scale * (cells of the whole batch): that bounds its
   // latency to a fraction of the batch's time (thr_cap_scale = fraction /
   // pair slots the class keeps resident).
-  unsigned int enabled;    // bit c: class c may be chosen by cost (and is launched)
   // Full-occupancy grid and strip scratch (int2) per block of each class,
   // where its launch's scratch starts (a region per stream), and the scratch
   // available.
@@ -850,7 +850,6 @@ struct BinParams {
   long long scr_cap;
   int thr_cls;             // class index
   int thr_on;              // 0: the class is never chosen (unless forced)
-  int thr_k;               // columns per strip
   int thr_max_rows, thr_fit;   // rows it accepts, and the longest min(|A|,|B|)
   float thr_cap_scale;
   const unsigned long long* total_cells;  // written by k_bin_total
@@ -1284,8 +1283,8 @@ static __global__ void k_bin_scan(BinParams bp, const int* hist, int* offs, cons
 
 // The whole pre-pass of a batch of at most kSmallBin pairs in one block:
 // batch cells, keys, class sums and the list, sorted by key in shared memory
-// (bitonic).  Four launches and their 110,000-key histogram took 85 us for
-// 64 pairs, this 9.  s32_flag as in k_bin_count.
+// (bitonic).  Four launches and their histogram (NCLASS_MAX * NBUCKET keys)
+// took 85 us for 64 pairs, this 9.  s32_flag as in k_bin_count.
 constexpr int kSmallBin = 4096;
 static __global__ void __launch_bounds__(1024) k_bin_small(BinParams bp, const uint8_t* __restrict__ codes,
                                                            const PairDesc* __restrict__ pairs, int n,

@@ -41,9 +41,10 @@
 // 0.60 (8 lanes of 30), affine 0.98; 10,000 protein pairs of 512 x 520 0.81
 // -> 0.66; 20,000 of 224 x 350 0.57 -> 0.44.  ALU instructions per column
 // and warp 8.0 -> 3.9 (linear), 6.6 (affine).  What bounds it now: the ALU
-// pipe (87 % busy) for affine DNA; linear gaps issue 0.74 instructions a
-// cycle with the ALU and FMA pipes near 75 and 50 %, which more resident
-// warps did not raise (20 or 24 per SM: within 5 %).
+// pipe, 77 % busy over a launch of affine DNA (three blocks an SM) and 70 %
+// of proteins (two); linear gaps issue 0.67 to 0.72 instructions a cycle with
+// the ALU pipe at 68 to 71 %, which more resident warps did not raise (20 or
+// 24 per SM: within 5 %).
 #pragma once
 #include "sw_device.cuh"
 
