@@ -43,14 +43,19 @@ REPO = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(REPO, "ipuma-lib_b200", "python"))
 sys.path.insert(0, os.path.join(REPO, "oracle"))
 
-LANE_OPS_PER_CELL = 7  # E: 2, F: 2, H: 2, running max: 1 (int lane-ops)
+# Operations of the ALU pipe per cell that the recurrence cannot do without
+# (one per pair of a 16-bit instruction): the unpacked substitution score, and
+# H and the running maximum (linear gaps) or F, Y, E, H (affine; the running
+# maximum's share left out).  Additions issue on the FMA pipe beside it.
+ALU_OPS_PER_CELL = {"linear": 3, "affine": 5}
+INT_PEAK_ALU_SHARE = 6 / 7  # ALU instructions in the mix ipuma_measure_int_peak times (its 7th is an addition)
 METRIC = "bit-exact GCUPS (forward pass, score + end coordinates)"
 
 # DRAM bytes (read + write) per forward-pass cell of the dominant launch,
-# from one ncu capture of that kernel on the same workload
-# (profiles/k_batched_s16x2_L16_K15_dna_1m.md: a launch reads the codes of
-# its own pairs, so its traffic scales with its cells).
-TRAFFIC_PER_CELL = {"dna_batched": 0.00622}
+# from one ncu capture of that kernel on reads of the same lengths
+# (profiles/k_batched_LaneLin_L8_K30_dna.md: a launch reads the codes of its
+# own pairs, so its traffic scales with its cells).
+TRAFFIC_PER_CELL = {"dna_batched": 0.00603}
 
 
 def parse(argv=None):
@@ -385,13 +390,14 @@ class DeviceBatch:
         self.step()
         st = self.eng.stats()
         self.eng.set_option("time_launches", 0)
-        timed = [(ib.KERNEL_NAMES.get(st.timed_kind[k], str(st.timed_kind[k])), st.timed_ms[k],
-                  st.timed_cells[k]) for k in range(st.n_timed)]
+        eight = self.bits == 2 and self.wl.gap_init == 0 and self.wl.n >= 150_000
+        timed = [(ib.kernel_name(st.timed_kind[k], eight), st.timed_ms[k], st.timed_cells[k])
+                 for k in range(st.n_timed)]
         self.eng.set_option("trace", 1)
         self.step()
         st = self.eng.stats()
         self.eng.set_option("trace", 0)
-        trace = [{"kernel": ib.KERNEL_NAMES.get(st.trace_kind[k], str(st.trace_kind[k])),
+        trace = [{"kernel": ib.kernel_name(st.trace_kind[k], eight),
                   "start_ms": round(st.trace_start_ms[k], 3), "end_ms": round(st.trace_end_ms[k], 3),
                   "gcells": round(st.trace_cells[k] / 1e9, 3)} for k in range(st.n_trace)]
         return timed, trace
@@ -737,12 +743,14 @@ def main(argv=None):
     rl = None
     if dom:
         name, dms, dcells = dom
-        achieved = dcells * LANE_OPS_PER_CELL / (dms * 1e-3) / 1e9
+        ops = ALU_OPS_PER_CELL["linear" if wl.gap_init == 0 else "affine"]
+        achieved = dcells * ops / (dms * 1e-3) / 1e9
+        alu_peak = int_peak * INT_PEAK_ALU_SHARE
         tpc = TRAFFIC_PER_CELL.get(args.workload)
         rl = {"bound": "int_issue", "kernel": name, "achieved": achieved,
-              "peak": int_peak / 1e9, "unit": "G int lane-ops/s", "frac": achieved * 1e9 / int_peak,
-              "per_unit": "%d lane-ops per cell; %d cells in this launch" % (LANE_OPS_PER_CELL, dcells),
-              "launch_ms": dms, "peak_source": "ipuma_measure_int_peak (s16x2 DPX mix, this GPU)",
+              "peak": alu_peak / 1e9, "unit": "G ALU lane-ops/s", "frac": achieved * 1e9 / alu_peak,
+              "per_unit": "%d ALU lane-ops per cell; %d cells in this launch" % (ops, dcells),
+              "launch_ms": dms, "peak_source": "ipuma_measure_int_peak (s16x2 DPX mix, this GPU) x 6/7",
               "traffic": (dcells * tpc) if tpc else None,
               "traffic_unit": "bytes per launch (ncu dram__bytes_read+write per cell x launch cells)"}
     algo_bytes = algorithmic_bytes(wl)

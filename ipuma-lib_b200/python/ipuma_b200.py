@@ -45,21 +45,28 @@ EXPORTS = [
     "ipuma_gpu_compare_packed", "ipuma_pack_codes", "ipuma_gpu_compare_device_packed",
 ]
 
-KERNEL_NAMES = {0: "k_batched<s32,L32,K16>", 1: "k_batched<s16x2,L16,K4>",
-                2: "k_batched<s16x2,L16,K8>", 3: "k_batched<s16x2,L16,K12>",
-                4: "k_batched<s16x2,L16,K16>", 5: "k_batched<s16x2,L32,K12>",
-                6: "k_batched<s16x2,L32,K16>", 7: "k_batched<s32,L32,K16> rerun",
-                8: "k_plain<K>", 9: "k_exact", 10: "k_thread<s16x2,K16>",
-                11: "k_batched<s16x2,L16,K6>", 12: "k_batched<s16x2,L16,K10>",
-                13: "k_batched<s16x2,L16,K14>", 14: "k_batched<s16x2,L16,K5>",
-                15: "k_batched<s16x2,L16,K7>", 16: "k_batched<s16x2,L16,K9>",
-                17: "k_batched<s16x2,L16,K11>", 18: "k_batched<s16x2,L16,K13>",
-                19: "k_batched<s16x2,L16,K15>", 20: "k_hybrid<b16x2->s32,L32,K16>",
-                21: "k_plain16<K>", 22: "k_batched<s16x2,L8,K8>",
-                23: "k_batched<s16x2,L8,K10>", 24: "k_batched<s16x2,L8,K12>",
-                25: "k_batched<s16x2,L8,K14>", 26: "k_batched<s16x2,L8,K16>",
-                27: "k_strips<s16x2,L32,K16> team", 28: "k_batched<s16x2,L32,K8>",
-                29: "k_batched<s16x2,L32,K4>"}
+# Kernels of the ipuma_stats kinds.  The 16-bit strips by width are classes of
+# k_mix; in 2-bit batches of 150,000 pairs and more with linear gaps those of
+# 16 lanes are k_batched launches of 8 lanes with twice the columns.
+KERNEL_NAMES = {0: "k_batched<s32,L32,K16>", 7: "k_batched<s32,L32,K16> rerun", 8: "k_plain<K>", 9: "k_exact",
+                10: "k_thread<s16x2,K16>", 20: "k_batched<b16x2,L32,K16> big or hybrid", 21: "k_plain16<K>",
+                27: "k_strips<L32,K16> team"}
+KERNEL_NAMES.update({kind: "k_mix strips L%d,K%d" % (lanes, k) for kind, lanes, k in
+                     [(1, 16, 4), (2, 16, 8), (3, 16, 12), (4, 16, 16), (5, 32, 12), (6, 32, 16), (11, 16, 6),
+                      (12, 16, 10), (13, 16, 14), (14, 16, 5), (15, 16, 7), (16, 16, 9), (17, 16, 11), (18, 16, 13),
+                      (19, 16, 15), (22, 8, 8), (23, 8, 10), (24, 8, 12), (25, 8, 14), (26, 8, 16), (28, 32, 8),
+                      (29, 32, 4)]})
+KERNEL_NAMES[6] += " (k_batched for the long class)"
+
+
+def kernel_name(kind: int, eight_lanes: bool = False) -> str:
+    """Kernel of a launch; eight_lanes: of a batch whose 16-lane strips run as 8 lanes."""
+    name = KERNEL_NAMES.get(kind, str(kind))
+    if eight_lanes and "L16,K" in name:
+        return "k_batched<LaneLin,L8,K%d>" % (2 * int(name.rsplit("K", 1)[1]))
+    return name
+
+
 MAX_TIMED = 24  # IPUMA_MAX_TIMED
 
 
