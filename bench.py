@@ -52,9 +52,8 @@ INT_PEAK_ALU_SHARE = 6 / 7  # ALU instructions in the mix ipuma_measure_int_peak
 METRIC = "bit-exact GCUPS (forward pass, score + end coordinates)"
 
 # DRAM bytes (read + write) per forward-pass cell of the dominant launch,
-# from one ncu capture of that kernel on reads of the same lengths
-# (profiles/k_batched_LaneLin_L8_K30_dna.md: a launch reads the codes of its
-# own pairs, so its traffic scales with its cells).
+# from one ncu capture of that kernel on reads of the same lengths (a launch
+# reads the codes of its own pairs, so its traffic scales with its cells).
 TRAFFIC_PER_CELL = {"dna_batched": 0.00603}
 
 
